@@ -254,7 +254,7 @@ def kernel_split(kern, fused: bool, stream_bytes: int, n_v: int, n_t: int, persi
     decode's time in the second slot: the group kernel, persistent 3, or the
     fused kernel, persistent 2)."""
     if fused:  # one kernel reads the stream and writes both outputs
-        name = "group_kernel" if persistent == 3 else "flow_kernel"
+        name = {3: "group_kernel", 4: "team_kernel"}.get(persistent, "flow_kernel")
         return ("scan_kernel", name), 1, stream_bytes + 12 * (n_v + n_t)
     # connectivity reads the stream and writes the indices (12 B per
     # triangle); the vertex kernel writes the positions (12 B per vertex)

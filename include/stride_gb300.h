@@ -61,8 +61,8 @@ typedef struct {
     int32_t pred_k[3];
     uint32_t kernels;    /* kernel launches one decode makes: 2 with the
                             one-kernel shapes (scan, which also fills any
-                            per-code dequantisation tables; then the fused
-                            or the group kernel: persistent 2 or 3), 3 with
+                            per-code dequantisation tables; then the fused,
+                            group or team kernel: persistent 2, 3 or 4), 3 with
                             the two-kernel shapes (persistent 0 or 1), 0 for
                             an empty stream                                   */
     float g_min[3];      /* header g_min, g_range: a position's normalised   */
@@ -81,7 +81,7 @@ typedef struct {
                                 (1, 2) or two (4) parser/assembler warp pairs
                                 of 32 meshlets each; the vertex kernel's CTA is
                                 always three warps (one per axis)            */
-    int32_t persistent;      /* 2 (default) = one persistent kernel for both
+    int32_t persistent;      /* 2 = one persistent kernel for both
                                 phases: CTAs of two pairs take connectivity
                                 groups, then vertex work in the order groups
                                 finish (warps_per_cta must be 4);
@@ -89,6 +89,11 @@ typedef struct {
                                 32 meshlets through every phase, lane per
                                 meshlet (warps_per_cta 1 or 2; stage_bytes
                                 and code_bytes unused);
+                                4 = team kernel, the default of up to 9,728
+                                meshlets: a CTA of ten warps decodes 4, 8 or
+                                16 meshlets (warps_per_cta 1, 2 or 4) from
+                                bytes to positions (stage_bytes, code_bytes
+                                and ctas_per_sm unused);
                                 1 = connectivity kernel, then a persistent
                                 work-stealing vertex grid; 0 = connectivity
                                 kernel, then one vertex CTA per group        */
@@ -151,7 +156,8 @@ int stride_decode(stride_handle* h, void* stream, uint32_t* d_idx, float* d_pos,
  * copy them to h_idx / h_pos (host, n_t*3 uint32 and n_v*3 float32) and
  * synchronise.  Returns the decode status.  The triangle copy starts when
  * the connectivity kernel ends, beside the vertex kernel (a fused launch
- * shape is replaced by the persistent two-kernel one for this call); from
+ * shape, and the team kernel above 4,096 meshlets, is replaced by the
+ * persistent two-kernel one for this call); from
  * about 3 million triangles the connectivity runs in four parts and each
  * part's triangles are copied as soon as it ends, and after a
  * stride_reload of such a stream (uploaded in the same parts) each part
@@ -209,9 +215,10 @@ int stride_cull_meshlets(const float* d_bounds, uint32_t n, const float* planes,
 int stride_decode_timed(stride_handle* h, void* stream, uint32_t* d_idx, float* d_pos, float* kernel_ms);
 
 /* Launch shape for this handle's decodes.  Until it is set the shape
- * follows the mesh's size: the two kernels (persistent 1) for 128 to 1,023
- * groups of 32 meshlets, the fused kernel (persistent 2) otherwise; a
- * reload keeps a shape that was set. */
+ * follows the mesh's size: the team kernel (persistent 4) up to 9,728
+ * meshlets, the two kernels (persistent 1) up to 1,023 groups of 32
+ * meshlets, the fused kernel (persistent 2) above; a reload keeps a shape
+ * that was set. */
 int stride_set_config(stride_handle* h, const stride_launch_cfg* cfg);
 
 /* No counterpart in the reference.  SM clocks each device wait of this

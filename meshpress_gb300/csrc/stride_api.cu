@@ -136,13 +136,13 @@ using namespace stride;
 namespace stride {
 
 unsigned long long plan_luts(MeshParams* p, uint32_t n, uint32_t* meshes, uint32_t max_meshes, uint32_t* n_lut,
-                             uint32_t* lut_max) {
+                             uint32_t* lut_max, bool alone) {
     unsigned long long total = 0;
     uint32_t k = 0, mx = 0;
     for (uint32_t i = 0; i < n; i++) {
         p[i].has_lut = 0;
         p[i].lut_off = 0;
-        const unsigned long long e = lut_entries(p[i]);
+        const unsigned long long e = lut_entries(p[i], alone);
         if (!e || k >= max_meshes || k >= 65535u) continue;  // bounds the table blocks of the scan launch
         p[i].has_lut = 1;
         p[i].lut_off = total;
@@ -253,6 +253,11 @@ int decode_to_host(HostLink& L, const DecodeArgs& a, LaunchCfg cfg, void* stream
         return cuda_fail(err, what);
     };
     if (cfg.persistent == 2) cfg.persistent = 1;
+    if (cfg.persistent == 4 && a.total_meshlets > kHostTeam) {
+        LaunchCfg two = cfg;
+        two.persistent = 1;
+        if (check_config(two, a.wide_codes) == STRIDE_OK) cfg = two;
+    }
     const size_t ib = 12 * n_t, pb = 12 * n_v;
     const bool parts = cfg.persistent < 2 && host_parts(n_t, a.total_meshlets);
     if (parts) {
@@ -365,7 +370,7 @@ static int ensure_capacity(stride_handle* h, size_t len, MeshParams& p) {
     const uint32_t n_meshlets = p.n_meshlets;
     const uint64_t n_v = p.n_v;
     cudaError_t e;
-    const unsigned long long lut = plan_luts(&p, 1, nullptr, 1, &h->n_lut, &h->lut_max);
+    const unsigned long long lut = plan_luts(&p, 1, nullptr, 1, &h->n_lut, &h->lut_max, true);
     if (!h->d_lut_mesh) {
         const uint32_t zero = 0u;
         if ((e = cudaMalloc(&h->d_lut_mesh, sizeof(uint32_t))) != cudaSuccess ||
@@ -591,6 +596,9 @@ static DecodeArgs handle_args(stride_handle* h, uint32_t* d_idx, float* d_pos, i
     a.lut_meshes = h->d_lut_mesh;
     a.n_lut_meshes = h->n_lut;
     a.lut_max = h->lut_max;
+    a.hint_bytes = h->len;
+    a.hint_v = h->params.n_v;
+    a.hint_t = h->params.n_t;
     return a;
 }
 

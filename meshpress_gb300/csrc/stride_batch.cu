@@ -123,6 +123,9 @@ static DecodeArgs batch_args(const stride_batch* b, uint32_t* d_idx, float* d_po
     a.lut_meshes = b->d_lut_meshes;
     a.n_lut_meshes = b->n_lut;
     a.lut_max = b->lut_max;
+    a.hint_bytes = b->arena_bytes;
+    a.hint_v = b->total_v;
+    a.hint_t = b->total_t;
     return a;
 }
 
@@ -431,6 +434,12 @@ int stride_batch_autotune(stride_batch* b, void* stream, uint32_t* d_idx, float*
         c.warps_per_cta = w;
         c.persistent = 3;
         c.ctas_per_sm = 0;
+        cands.push_back(c);
+    }
+    for (int w : {1, 2, 4}) {  // the team kernel sizes itself
+        LaunchCfg c;
+        c.warps_per_cta = w;
+        c.persistent = 4;
         cands.push_back(c);
     }
     cudaEvent_t e0, e1;

@@ -59,16 +59,22 @@ struct MeshParams {
 // Dequantisation tables: a mesh with at least as many duplicated vertices as
 // half its code space (all axes together) gets one float per code and axis,
 // evaluated once per decode by extra blocks of the scan launch; axis d's table follows those of
-// the axes before it.  Only for codes of up to kLutMaxBits bits.
+// the axes before it.  Only for codes of up to kLutMaxBits bits.  A mesh
+// decoded alone (`alone`) also gets tables of up to kLutAlone floats whatever
+// its size: the GPU is idle then, and a code whose float-float result is too
+// close to a rounding boundary (every vertex at coordinate 0, say) costs a
+// float64 evaluation per vertex where the table pays it once per code, in
+// parallel (33^2 heightfield: 7 us of the decode).
 constexpr uint32_t kLutMaxBits = 16;
+constexpr unsigned long long kLutAlone = 16384;
 
-inline unsigned long long lut_entries(const MeshParams& p) {
+inline unsigned long long lut_entries(const MeshParams& p, bool alone = false) {
     unsigned long long e = 0;
     for (int d = 0; d < 3; d++) {
         if (p.g_bits[d] > kLutMaxBits) return 0;
         e += 1ull << p.g_bits[d];
     }
-    return e <= 2ull * p.n_v ? e : 0;
+    return e <= 2ull * p.n_v || (alone && e <= kLutAlone) ? e : 0;
 }
 
 // Per-meshlet record: the scan kernel writes the first part, the
@@ -108,6 +114,7 @@ struct LaunchCfg {
     int warps_per_cta = 4;
     int persistent = 2;  // 0: one vertex CTA per group, 1: persistent vertex grid, 2: one fused kernel,
                          // 3: group kernel (one warp per group, every phase; warps_per_cta 1 or 2)
+                         // 4: team kernel (warps_per_cta 1, 2, 4: 4, 8, 16 meshlets per CTA of ten warps)
     int ctas_per_sm = 0;
     uint32_t stage_bytes = 16 * 1024;  // per-warp payload staging (vertex kernel: half)
     uint32_t code_bytes = 12 * 1024;   // per-warp integer code plane (vertex kernel)
@@ -141,13 +148,16 @@ struct DecodeArgs {
     // shape): whole 256-meshlet windows, i.e. multiples of eight; the
     // defaults take every group
     uint32_t conn_g0 = 0u, conn_g1 = 0xFFFFFFFFu;
+    // totals of what is decoded, from which the team kernel sizes its shared
+    // memory (estimates: any value decodes)
+    unsigned long long hint_bytes = 0ull, hint_v = 0ull, hint_t = 0ull;
 };
 
 // Host: assigns table offsets (has_lut, lut_off) to the meshes that get
-// tables; returns the floats needed, fills `meshes` (at most max_meshes
+// tables (`alone`: see lut_entries); returns the floats needed, fills `meshes` (at most max_meshes
 // indices) and the largest per-mesh size.
 unsigned long long plan_luts(MeshParams* p, uint32_t n, uint32_t* meshes, uint32_t max_meshes, uint32_t* n_lut,
-                             uint32_t* lut_max);
+                             uint32_t* lut_max, bool alone = false);
 
 inline uint32_t scan_blocks(uint32_t total_meshlets) {
     return (total_meshlets + kScanThreads - 1) / kScanThreads;
@@ -212,6 +222,12 @@ void last_launch(uint32_t* smem_bytes, uint32_t* grid);
 // shared memory per CTA.
 cudaError_t launch_group(const DecodeArgs& a, const LaunchCfg& cfg, void* stream);
 size_t group_smem_bytes(const LaunchCfg& cfg);
+
+// The team kernel (stride_team.cu): launch for `a` on `stream`, as the scan's
+// programmatic dependent when `after_scan`.
+cudaError_t launch_team(const DecodeArgs& a, const LaunchCfg& cfg, cudaStream_t stream, bool after_scan);
+
+inline uint32_t team_meshlets(const LaunchCfg& cfg) { return 4u * static_cast<uint32_t>(cfg.warps_per_cta); }
 
 // STRIDE_OK when `cfg` is a launchable shape.
 int check_config(const LaunchCfg& cfg, bool wide);

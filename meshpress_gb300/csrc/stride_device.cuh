@@ -343,9 +343,9 @@ __device__ __forceinline__ uint32_t group_at(uint32_t f, uint32_t n_groups) {
     return kPer * w + l;
 }
 
-__device__ __forceinline__ void load_group_lane(const DecodeArgs& a, uint32_t g, int lane, GroupLane& L) {
-    const uint32_t slot = g * 32u + lane;
-    L.valid = slot < a.total_meshlets;
+// The meshlet of a slot (of none when !in).
+__device__ __forceinline__ void load_slot_lane(const DecodeArgs& a, uint32_t slot, bool in, GroupLane& L) {
+    L.valid = in && slot < a.total_meshlets;
     L.m = L.valid ? __ldcg(&a.descs[slot].slot_meshlet) : slot;
     if (L.valid) {
         const uint4* src = reinterpret_cast<const uint4*>(a.descs + L.m);
@@ -354,7 +354,8 @@ __device__ __forceinline__ void load_group_lane(const DecodeArgs& a, uint32_t g,
         dst[1] = __ldcg(src + 1);
         dst[2] = __ldcg(src + 2);
         dst[3] = __ldcg(src + 3);
-        const BlockPrefix& bp = a.blk_prefix[L.m / kScanThreads];
+        // a slot's meshlet lies in the slot's own window
+        const BlockPrefix& bp = a.blk_prefix[slot / kScanThreads];
         L.v_base = bp.v + L.d.v_pref;
         L.t_base = bp.t + L.d.t_pref;
         L.wp_base = bp.wp + L.d.wp_pref;
@@ -365,6 +366,11 @@ __device__ __forceinline__ void load_group_lane(const DecodeArgs& a, uint32_t g,
     L.mi = (L.valid && a.meshlet_mesh) ? __ldcg(a.meshlet_mesh + L.m) : 0u;
     L.P = a.meshes + L.mi;
     L.blob_off = L.valid ? L.P->blob_off : 0ull;
+}
+
+// Lane's meshlet of a group of 32 slots.
+__device__ __forceinline__ void load_group_lane(const DecodeArgs& a, uint32_t g, int lane, GroupLane& L) {
+    load_slot_lane(a, g * 32u + lane, true, L);
 }
 
 // The meshlet's output ranges lie inside its mesh's (header n_v_total, n_t)
@@ -708,6 +714,53 @@ __device__ __forceinline__ uint4 mtf_mask_row(uint32_t p) {
     m.z = __funnelshift_lc(0xFFFFFFFFu, 0u, static_cast<uint32_t>(max(b - 64, 0)));
     m.w = __funnelshift_lc(0xFFFFFFFFu, 0u, static_cast<uint32_t>(max(b - 96, 0)));
     return m;
+}
+
+// A meshlet's offset table entries and header, checked; 0 or an error code.
+__device__ __forceinline__ int scan_meshlet(const uint8_t* __restrict__ arena, const MeshParams& P, uint32_t lm, MeshletDesc& d) {
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(arena + P.blob_off);
+    const uint32_t nbits = static_cast<uint32_t>(P.nbits);
+    const uint32_t tbit = kHeaderBytes * 8u;
+    const uint32_t off = peek32<false>(w, tbit + 32u * lm);
+    const uint32_t next = (lm + 1u < P.n_meshlets) ? peek32<false>(w, tbit + 32u * (lm + 1u)) : nbits;
+    // decode_dup reads meshlets back to back from the end of the table, so
+    // the table must start there and increase (paradelta_v5_dup.py:496-507)
+    if ((lm == 0u && off != P.body_bit) || off < P.body_bit || next > nbits || off > nbits - 48u ||
+        next < off + 48u)
+        return kErrOffset;
+    const uint32_t h0 = peek32<false>(w, off);
+    const uint32_t n_local = h0 >> 16;
+    const uint32_t n_tris = h0 & 0xFFFFu;
+    const uint32_t n_strips = peek32<false>(w, off + 32u) >> 16;
+    if (n_local > static_cast<uint32_t>(kMaxLocal) || n_tris > static_cast<uint32_t>(kMaxTris))
+        return kErrUnsupported;
+    if (n_strips > n_tris) return kErrCorrupt;  // every strip emits >= 1 triangle
+    d.start_bit = off;
+    d.end_bit = next;
+    d.counts0 = n_local | (n_tris << 16);
+    d.n_strips = n_strips;
+    return 0;
+}
+
+// Host: lets `kernel` use `smem` bytes of dynamic shared memory on the
+// current device (once per device and size; `configured` is the caller's).
+template <class K>
+cudaError_t opt_in_smem(K kernel, size_t smem, size_t* configured) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    dev = dev < 0 || dev >= 64 ? 0 : dev;
+    if (configured[dev] < smem) {
+        cudaError_t e =
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        if (e != cudaSuccess) return e;
+        // the whole unified L1 as shared memory: both kernels read global
+        // data through L2 only, and the default split leaves room for one
+        // CTA fewer per SM than the shared-memory size allows
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        if (e != cudaSuccess) return e;
+        configured[dev] = smem;
+    }
+    return cudaSuccess;
 }
 
 }  // namespace

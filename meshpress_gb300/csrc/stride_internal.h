@@ -34,6 +34,13 @@ const char* status_message(int code);
 constexpr int kHostParts = 4;
 constexpr uint64_t kHostPartTris = 3ull << 20;
 
+// Meshlets up to which such a decode keeps the team kernel, which ends before
+// the two kernels' triangles are out; above, their copy beside the vertex
+// kernel gains more (a call with pinned buffers, 14-bit heightfields of 45 /
+// 1,295 / 2,631 / 4,090 / 5,221 meshlets: two kernels 161 / 203 / 187 / 208 /
+// 234 us, team 85 / 121 / 165 / 204 / 268).
+constexpr uint32_t kHostTeam = 4096;
+
 // The end of a part's windows: the last window's block prefix and sums
 // (their sum is the next part's first rows).
 struct PartEnd {

@@ -94,31 +94,6 @@ __device__ __forceinline__ void claim_bar(uint32_t pair) {
 // ---------------------------------------------------------------------------
 // 1. scan kernel
 // ---------------------------------------------------------------------------
-__device__ int scan_meshlet(const uint8_t* __restrict__ arena, const MeshParams& P, uint32_t lm, MeshletDesc& d) {
-    const uint32_t* w = reinterpret_cast<const uint32_t*>(arena + P.blob_off);
-    const uint32_t nbits = static_cast<uint32_t>(P.nbits);
-    const uint32_t tbit = kHeaderBytes * 8u;
-    const uint32_t off = peek32<false>(w, tbit + 32u * lm);
-    const uint32_t next = (lm + 1u < P.n_meshlets) ? peek32<false>(w, tbit + 32u * (lm + 1u)) : nbits;
-    // decode_dup reads meshlets back to back from the end of the table, so
-    // the table must start there and increase (paradelta_v5_dup.py:496-507)
-    if ((lm == 0u && off != P.body_bit) || off < P.body_bit || next > nbits || off > nbits - 48u ||
-        next < off + 48u)
-        return kErrOffset;
-    const uint32_t h0 = peek32<false>(w, off);
-    const uint32_t n_local = h0 >> 16;
-    const uint32_t n_tris = h0 & 0xFFFFu;
-    const uint32_t n_strips = peek32<false>(w, off + 32u) >> 16;
-    if (n_local > static_cast<uint32_t>(kMaxLocal) || n_tris > static_cast<uint32_t>(kMaxTris))
-        return kErrUnsupported;
-    if (n_strips > n_tris) return kErrCorrupt;  // every strip emits >= 1 triangle
-    d.start_bit = off;
-    d.end_bit = next;
-    d.counts0 = n_local | (n_tris << 16);
-    d.n_strips = n_strips;
-    return 0;
-}
-
 // Exclusive scan over the block; returns the thread's prefix and the total.
 __device__ __forceinline__ unsigned long long block_scan(unsigned long long x, unsigned long long* wsum,
                                                          unsigned long long& total) {
@@ -1053,25 +1028,6 @@ __global__ void __launch_bounds__(128, kMinBlocks) flow_kernel(DecodeArgs a, uin
 // ---------------------------------------------------------------------------
 // launch plumbing
 // ---------------------------------------------------------------------------
-template <class K>
-cudaError_t opt_in_smem(K kernel, size_t smem, size_t* configured) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    dev = dev < 0 || dev >= 64 ? 0 : dev;
-    if (configured[dev] < smem) {
-        cudaError_t e =
-            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-        if (e != cudaSuccess) return e;
-        // the whole unified L1 as shared memory: both kernels read global
-        // data through L2 only, and the default split leaves room for one
-        // CTA fewer per SM than the shared-memory size allows
-        e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-        if (e != cudaSuccess) return e;
-        configured[dev] = smem;
-    }
-    return cudaSuccess;
-}
-
 // Resident CTAs per SM of one kernel instantiation, cached per device and
 // shared-memory size (the occupancy query costs microseconds per launch).
 struct OccCache {
@@ -1250,6 +1206,7 @@ __global__ void side_table_kernel(const MeshletDesc* __restrict__ descs, uint32_
 
 int check_config(const LaunchCfg& cfg, bool wide) {
     if (cfg.warps_per_cta != 1 && cfg.warps_per_cta != 2 && cfg.warps_per_cta != 4) return STRIDE_ERR_ARG;
+    if (cfg.persistent == 4) return STRIDE_OK;  // sizes itself; a meshlet that does not fit is read in place
     if (cfg.persistent < 0 || cfg.persistent > 3 || (cfg.persistent == 2 && cfg.warps_per_cta != 4) ||
         (cfg.persistent == 3 && cfg.warps_per_cta > 2))
         return STRIDE_ERR_ARG;
@@ -1261,22 +1218,35 @@ int check_config(const LaunchCfg& cfg, bool wide) {
     return STRIDE_OK;
 }
 
-// Groups from which the default launch shape is the two-kernel one, below
-// kFlowFiveGroups.  Measured on one GB300 (step, L2 flushed, every output
-// bit-identical), fused against two kernels: 513^2 heightfield (83 groups)
-// 0.111 / 0.115 ms, level-8 icosphere (210) 0.137 / 0.121, 1025^2 (331)
-// 0.147 / 0.125, 1449^2 (666) 0.177 / 0.173, 2049^2 (1,347) 0.222 / 0.278,
-// 2897^2 (2,700) 0.407 / 0.475.  Between these bounds the vertex kernel's
-// three-warp CTAs (no idle warp, two meshlets per L2 round trip in the
-// output pass) outrun the fused kernel's vertex phase; above them the
-// fused kernel's overlap of the two phases wins, below them its single
-// launch.
-constexpr uint32_t kTwoKernelGroups = 128u;
+// Meshlets up to which the default launch shape is the team kernel, and with
+// 4, 8 and 16 meshlets per CTA: as many CTAs as the 152 SMs hold at once (two
+// per SM; four meshlets while there is one CTA per SM), and 16 for up to two
+// such waves.  Step in us, L2 flushed, 12-bit heightfields, every output
+// bit-identical; before: the fused kernel up to 128 groups, then the two
+// kernels:
+//   meshlets            10   158   650  1295  2631  4090  5221  7503  9229  10584
+//   before              99   110   114   112   112   116   119   118   122    124
+//   4 per CTA           38    37    39    63    95   128
+//   8 per CTA           38    40    40    46    71    79   108   136   151    177
+//   16 per CTA          50    50    48    50    58    60   100   106   110    146
+// (14-bit spheres of 103 and 1,738 meshlets: 220 -> 56, 196 -> 58 us; 20-bit
+// heightfield of 5,221: 245 -> 108 us.)
+constexpr uint32_t kTeam4 = 700u, kTeam8 = 2432u, kTeamMost = 9728u;
 
 LaunchCfg default_config(uint32_t total_meshlets) {
     LaunchCfg cfg;
+    if (total_meshlets <= kTeamMost) {
+        cfg.persistent = 4;
+        cfg.warps_per_cta = total_meshlets <= kTeam4 ? 1 : (total_meshlets <= kTeam8 ? 2 : 4);
+        return cfg;
+    }
     const uint32_t groups = (total_meshlets + 31u) / 32u;
-    cfg.persistent = (groups >= kTwoKernelGroups && groups < kFlowFiveGroups) ? 1 : 2;
+    // Above: the two kernels below kFlowFiveGroups, where the fused kernel's
+    // completion list runs short of finished groups and its vertex phase
+    // waits (1449^2, 666 groups: 0.177 against 0.173 ms), then the fused
+    // kernel, whose overlap of the two phases wins (2049^2, 1,347 groups:
+    // 0.222 against 0.278).
+    cfg.persistent = groups < kFlowFiveGroups ? 1 : 2;
     return cfg;
 }
 
@@ -1306,13 +1276,17 @@ int enqueue_decode(const DecodeArgs& a, const LaunchCfg& cfg, void* stream, void
     record(ev, 1, s);
     if (a.total_meshlets != 0) {
         cudaError_t e;
-        if (cfg.persistent == 3) {  // one warp per group: no connectivity/vertex split
+        // without an event between them, the team and the fused kernel are the
+        // scan's programmatic dependents
+        const bool after_scan = ev == nullptr || ev[1] == nullptr;
+        if (cfg.persistent == 4) {  // a CTA of ten warps per 4, 8 or 16 meshlets
+            e = launch_team(a, cfg, s, after_scan);
+            record(ev, 2, s);
+        } else if (cfg.persistent == 3) {  // one warp per group: no connectivity/vertex split
             e = launch_group(a, cfg, s);
             record(ev, 2, s);
         } else if (cfg.persistent == 2) {  // one kernel: the connectivity/vertex split is not timed
-            // without timing events between them, the fused kernel is the
-            // scan's programmatic dependent
-            e = launch_flow_any(a, cfg, s, ev == nullptr);
+            e = launch_flow_any(a, cfg, s, after_scan);
             record(ev, 2, s);
         } else {
             switch (cfg.warps_per_cta) {

@@ -499,6 +499,9 @@ bool dispatch(stride_server* s, int slot_i) {
         a.lut_meshes = reinterpret_cast<const uint32_t*>(sc + sp.lut_list);
         a.n_lut_meshes = n_lut;
         a.lut_max = lut_max;
+        a.hint_v = tv;
+        a.hint_t = tt;
+        for (const Request* r : take) a.hint_bytes += r->len;
         a.wide_codes = false;
         for (const MeshParams& p : params)
             a.wide_codes = a.wide_codes || p.g_bits[0] > 16 || p.g_bits[1] > 16 || p.g_bits[2] > 16;

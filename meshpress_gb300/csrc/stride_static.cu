@@ -91,7 +91,7 @@ StaticLayout plan(size_t len, const MeshParams& p) {
     L.walk = o;
     o += up256(4ull * walk_scratch_words(p.n_v, p.n_meshlets));
     L.lut = o;
-    o += up256(4ull * lut_entries(p));
+    o += up256(4ull * lut_entries(p, true));
     L.status = o;
     o += up256(sizeof(Status));
     L.total = o;
@@ -109,7 +109,7 @@ extern "C" int stride_decode_static(const uint8_t* data, size_t len, void* strea
     int rc = parse_header(data, len, &p, why, sizeof(why));
     if (rc) return fail(rc, "%s", why);
     uint32_t n_lut = 0, lut_max = 0;
-    plan_luts(&p, 1, nullptr, 1, &n_lut, &lut_max);
+    plan_luts(&p, 1, nullptr, 1, &n_lut, &lut_max, true);
     const StaticLayout L = plan(len, p);
     if (L.total > kStaticScratchBytes)
         return fail(STRIDE_ERR_NOMEM,
@@ -150,6 +150,9 @@ extern "C" int stride_decode_static(const uint8_t* data, size_t len, void* strea
     a.lut_meshes = reinterpret_cast<const uint32_t*>(base + L.lut_list);
     a.n_lut_meshes = n_lut;
     a.lut_max = lut_max;
+    a.hint_bytes = len;
+    a.hint_v = p.n_v;
+    a.hint_t = p.n_t;
     // always the fused shape: one set of kernels, loaded by the first call
     // (a shape used for the first time later would load its kernels then)
     LaunchCfg cfg;

@@ -1,0 +1,1301 @@
+// Team kernel (launch shape 4): a CTA of ten warps decodes M consecutive
+// meshlets (M = 4, 8 or 16) from their bytes to positions, in shared memory.
+//
+// What bounds a decode is the length of one meshlet's serial chains: token
+// widths depend on flag bits, the FIFO on every earlier token, codewords on
+// the ones before them, IRLP on earlier codes.  The team keeps on those
+// chains only what is serial, one lane per meshlet, and spreads the rest over
+// whole warps:
+//
+//  1. stage    a warp per meshlet: its bytes into shared memory, in bit order.
+//  2. parse    a warp, lane per meshlet: token boundaries.  Six tokens of
+//              seven are raw, so a step takes up to three raw tokens and the
+//              FIFO token after them.
+//     FIFO     a warp, lane per meshlet, a chunk of steps behind: the
+//              move-to-front FIFO, once per step; ids of the FIFO tokens.
+//     assemble eight warps, a warp per meshlet, a chunk behind the FIFO: steps
+//              to token records (lane per step), then windows of 32 tokens
+//              (lane per token): strip state by ballots (a strip-body
+//              triangle is the previous two ids and the id two before the
+//              last edge-code-0 token), triangles, first occurrences, walk.
+//  3. walk     lane per (meshlet, axis): a decoder warp finds the substreams
+//              and reads residuals, a predictor warp behind it runs IRLP.
+//  4. emit     a warp per meshlet, lane per vertex: exact positions.
+//
+// Loops that carry a chain are unrolled, free of branches and of the same
+// length in every lane where they can be: a taken branch costs a lone warp
+// about 20 cycles, a diverged one twice that.  Groups are independent: no
+// work queue, no waits between CTAs; several CTAs per SM overlap one
+// another's phases.
+//
+// The scan (output placement, tables, the offset table's checks) runs beside
+// the first half: connectivity needs only the stream, so the kernel is
+// launched as the scan's programmatic dependent, reads the meshlet headers
+// itself and waits for the scan before it writes anything.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "stride_common.cuh"
+#include "stride_device.cuh"
+#include "stride_gb300.h"
+
+namespace stride {
+namespace {
+
+constexpr uint32_t kTeamAsm = 8u;  // assembler warps, beside the parser and the FIFO warp
+constexpr uint32_t kTeamThreads = 32u * (kTeamAsm + 2u);
+// Warps w, w + 4 and w + 8 share one of the SM's four schedulers, whose
+// integer ALU the parser and the FIFO warp keep busy by themselves: they are
+// warps 2 and 3, with one assembler each beside them (and none up to M = 4),
+// the other six three to a scheduler.
+constexpr uint32_t kTeamParser = 2u, kTeamFifo = 3u;
+__device__ __forceinline__ uint32_t team_asm_index(uint32_t warp) {  // 0 1 4 5 8 9 6 7 -> 0..7
+    return warp < 2u ? warp : (warp < 6u ? warp - 2u : (warp < 8u ? warp : warp - 4u));
+}
+constexpr uint32_t kTeamSteps = 16u;  // parser steps between hand-overs
+constexpr uint32_t kTeamRes = 16u;    // residuals between hand-overs from decoder to predictor warps
+constexpr uint32_t kTeamTokens = 768u;  // most tokens of a meshlet: n_tris + 2 n_strips
+// Token records: bits 0..8 the nine bits after the flag (a raw token's id on
+// top, or a FIFO index in bits 4..8, replaced by the field of the id it
+// names), bit 9 raw, bit 10 the edge code of a strip-body token, bit 11 the
+// first token of a strip.
+constexpr uint32_t kTokRaw = 1u << 9, kTokEdge = 1u << 10, kTokHead = 1u << 11;
+// A corrupt lane's cursor runs on past its meshlet until its loop ends: at
+// most 768 steps of 32 bits, or 256 codewords of 32 bits and a window.
+constexpr uint32_t kTeamSlack = 5120u;
+
+// Shared memory of a round: staged bytes, walks, then the token records and
+// the assembly's words (each id's last token, the triangles), whose place the
+// code planes take when the walk starts.  Laid out by what the round's
+// meshlets need.
+__host__ __device__ inline uint32_t team_bytes(uint32_t bits, uint32_t walk, uint32_t tok, uint32_t asm_words,
+                                               uint32_t plane) {
+    const uint32_t uni = tok + asm_words > plane ? tok + asm_words : plane;
+    const uint32_t rest = 4u * (walk + uni);
+    return bits + (rest > kTeamSlack ? rest : kTeamSlack);
+}
+// A meshlet's words in each.
+__host__ __device__ inline uint32_t team_walk_words(uint32_t n_local) {  // entries, then the vertex list
+    return (n_local + ((n_local + 3u) >> 2)) | 1u;
+}
+__host__ __device__ inline uint32_t team_tok_words(uint32_t n_tok) { return ((n_tok + 6u) >> 1) | 1u; }
+__host__ __device__ inline uint32_t team_asm_words(uint32_t n_tris) { return 256u + ((n_tris + 3u) & ~3u); }
+__host__ __device__ inline uint32_t team_axis_words(uint32_t n_local, uint32_t code_size) {
+    return ((n_local * code_size + 3u) >> 2) | 1u;
+}
+
+// Decoder warps for M meshlets (a lane per meshlet and axis), each with a
+// predictor warp behind it.
+template <uint32_t M>
+__host__ __device__ constexpr uint32_t team_dec_warps() {
+    return (3u * M + 31u) / 32u;
+}
+
+// Barriers of two warps; ids are immediates (see pair_bar).
+__device__ __forceinline__ void team_all_bar() {  // every warp, from its own loop
+    asm volatile("bar.sync 4, %0;" ::"n"(kTeamThreads) : "memory");
+}
+template <int kId>
+__device__ __forceinline__ void team_bar() {
+    asm volatile("bar.sync %0, 64;" ::"n"(kId) : "memory");
+}
+__device__ __forceinline__ void team_dec_bar(uint32_t k) {  // warp-uniform
+    if (k == 0u) {
+        team_bar<1>();
+    } else if (k == 1u) {
+        team_bar<2>();
+    } else {
+        team_bar<3>();
+    }
+}
+
+// A lane's next bits in registers: hi | mid | lo hold `cnt` (65..96) bits, the
+// next one the MSB of hi; nxt is the word after them.  Consuming bits is
+// three shifts, and neither the refill nor its load is on the chain from one
+// token or codeword to the next (branch-free: a taken branch costs a lone
+// warp about 20 cycles).
+template <bool kShared>
+struct BitBuf {
+    const uint32_t* w;
+    uint32_t hi, mid, lo, nxt, cnt, wi;  // wi: index of nxt
+    uint32_t end_word;                   // global reads stop here (a staged lane's overrun stays in shared memory)
+
+    __device__ __forceinline__ uint32_t load(uint32_t i) const {
+        return (kShared || i < end_word) ? ldw<kShared>(w, i) : 0u;
+    }
+    // at bit q of w
+    __device__ __forceinline__ void seek(uint32_t q) {
+        const uint32_t i = q >> 5, o = q & 31u;
+        const uint32_t a = load(i), b = load(i + 1u), c = load(i + 2u);
+        wi = i + 3u;
+        nxt = load(wi);
+        hi = __funnelshift_l(b, a, o);
+        mid = __funnelshift_l(c, b, o);
+        lo = c << o;
+        cnt = 96u - o;
+    }
+    __device__ __forceinline__ uint32_t at() const { return 32u * wi - cnt; }
+    // n <= 32
+    __device__ __forceinline__ void skip(uint32_t n) {
+        hi = __funnelshift_lc(mid, hi, n);
+        mid = __funnelshift_lc(lo, mid, n);
+        lo = __funnelshift_lc(0u, lo, n);
+        cnt -= n;
+        const bool refill = cnt <= 64u;  // lo is used up, mid holds cnt - 32 bits
+        const uint32_t t = __funnelshift_rc(nxt, 0u, cnt - 32u);
+        mid |= refill ? t : 0u;
+        lo = refill ? nxt << ((64u - cnt) & 31u) : lo;
+        cnt += refill ? 32u : 0u;
+        wi += refill ? 1u : 0u;
+        nxt = load(wi);
+    }
+};
+
+// a * b + c on the multiplier, which leaves the integer ALU to the rest.
+__device__ __forceinline__ uint32_t mad_u32(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t d;
+    asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
+
+// 32 bits at bit `pos` of the words at shared address `base`.
+__device__ __forceinline__ uint32_t peek_shared(uint32_t base, uint32_t pos) {
+    const uint32_t a = mad_u32(pos >> 5, 4u, base);
+    uint32_t hi, lo;
+    asm("ld.shared.u32 %0, [%1];" : "=r"(hi) : "r"(a));
+    asm("ld.shared.u32 %0, [%1+4];" : "=r"(lo) : "r"(a));
+    return __funnelshift_l(lo, hi, pos & 31u);
+}
+
+// A parser step: what it read (32 bits from its first token's edge code or
+// flag) and, for the FIFO warp and the assembler, bits 0..1 the raw tokens,
+// bit 2 a FIFO token after them, bit 3 strip-body tokens (each with its edge
+// code before the flag), bit 4 the strip's first tokens; the FIFO warp adds
+// the FIFO token's id in bits 8..15 and the step's first token in bits
+// 16..25.  A strip header is a step without tokens.
+constexpr uint32_t kStepFifo = 1u << 2, kStepBody = 1u << 3, kStepHead = 1u << 4;
+
+struct TeamParse {
+    uint32_t pos;         // bit of w
+    uint32_t t = 0u;      // tokens read
+    uint32_t left = 0u;   // tokens left in the strip
+    uint32_t roots = 0u;  // of which roots
+    uint32_t strips;      // strips to read
+    uint32_t head = 0u;   // kStepHead after a header
+};
+
+// All ones when x is negative.
+__device__ __forceinline__ uint32_t sign_mask(uint32_t x) { return static_cast<uint32_t>(static_cast<int32_t>(x) >> 31); }
+
+// kTeamSteps parser steps of a lane (x and meta: its slots, M apart).  A
+// strip of length len takes max(len, 1) + 2 tokens, so a valid meshlet's
+// strips end with its n_tris + 2 n_strips tokens; a corrupt one's cursor
+// runs on until the count is reached and its strips do not come out (checked
+// by the caller).  All a step may take is laid out before its flag bits are
+// known (tokens at 0, L, 2 L).  Conditions are masks: what the compiler made
+// branches of cost a lane that took them 40 cycles (170 cycles a step on one
+// warp against 128 without any taken).
+template <bool kShared, uint32_t M>
+__device__ __forceinline__ void team_parse(TeamParse& T, const uint32_t* __restrict__ w, uint32_t n_tok, uint32_t ib,
+                                           uint32_t limit, uint32_t* __restrict__ x_out, uint8_t* __restrict__ meta_out) {
+    const uint32_t most = ib <= 8u ? 3u : 2u;  // three tokens of 1 + 1 + ib bits in a window
+    const uint32_t p1 = 2u << ib;
+    const uint32_t ws = kShared ? smem_addr(w) : 0u;
+#pragma unroll 4
+    for (uint32_t i = 0; i < kTeamSteps; i++) {
+        uint32_t x;
+        if constexpr (kShared) {
+            x = peek_shared(ws, T.pos);
+        } else {
+            x = peek32<false>(w, T.pos);
+        }
+        const uint32_t on = sign_mask(T.t - n_tok);
+        const uint32_t hdr = sign_mask(T.left - 1u);    // strip header (paradelta_v5_dup.py:519)
+        const uint32_t body = sign_mask(T.roots - 1u);
+        const uint32_t L = ib + 1u - body, pl = p1 + (p1 & body);  // 2^L
+        const uint32_t lim = min((T.left & body) | T.roots, most);  // none for a header
+        const uint32_t x0 = x * (1u - body), x1 = x0 * pl, x2 = x1 * pl;  // flags on top (shifts on the multiplier)
+        const uint32_t s0 = sign_mask(x0), s1 = s0 & sign_mask(x1), s2 = s1 & sign_mask(x2);
+        const uint32_t r = min(0u - (s0 + s1 + s2), lim);
+        const uint32_t f = sign_mask(r - lim);  // then the next token is a FIFO token
+        const uint32_t k = (r - f) & on;
+        const uint32_t used = r * L + (f & (6u - body)) + (hdr & 16u);
+        x_out[i * M] = x;
+        meta_out[i * M] = static_cast<uint8_t>((r | (f & kStepFifo) | (body & kStepBody) | T.head) & on);
+        T.pos += used & on;
+        if constexpr (!kShared) T.pos = min(T.pos, limit);  // reads stay inside the stream (a staged lane's, the stage)
+        const uint32_t open = hdr & on;
+        const uint32_t len = max(x >> 16, 1u) + 2u;
+        T.t += k;
+        T.strips += open;  // minus one
+        T.left = ((T.left - k) & ~open) | (len & open);
+        T.roots = (T.roots - (k & ~body)) | (open & 3u);
+        T.head = open & kStepHead;
+    }
+}
+
+// The FIFO over kTeamSteps steps of a lane.  Raw ids are taken as new to the
+// FIFO (an encoder writes an index for an id it still holds; the assembly
+// checks it).
+template <uint32_t M>
+__device__ __forceinline__ void team_fifo(MtfFifo& fifo, uint32_t& t, const uint32_t* __restrict__ xs,
+                                          const uint8_t* __restrict__ meta, uint32_t* __restrict__ out, uint32_t ib,
+                                          const uint4* __restrict__ masks, uint32_t& past) {
+    const uint32_t ish = 32u - ib, p1 = 2u << ib;
+#pragma unroll 4
+    for (uint32_t i = 0; i < kTeamSteps; i++) {
+        const uint32_t x = xs[i * M], me = meta[i * M];
+        const uint32_t body = (me >> 3) & 1u, r = me & 3u, f = 0u - ((me >> 2) & 1u);
+        const uint32_t L = ib + 1u + body, pl = p1 << body;
+        const uint32_t y = x << (1u + body);  // the first token's id on top
+        const uint32_t y1 = y * pl, y2 = y1 * pl;
+        // push the first r ids: depths 0..15 move r deeper
+        const uint32_t ids = __byte_perm(__byte_perm(y2 >> ish, y1 >> ish, 0x0400u), y >> ish, 0x4210u) & 0xFFFFFF00u;
+        const uint32_t sh = 8u * r;
+        fifo.f3 = __funnelshift_l(fifo.f2, fifo.f3, sh);
+        fifo.f2 = __funnelshift_l(fifo.f1, fifo.f2, sh);
+        fifo.f1 = __funnelshift_l(fifo.f0, fifo.f1, sh);
+        fifo.f0 = __funnelshift_l(ids, fifo.f0, sh);
+        fifo.len = min(fifo.len + r, 16u);
+        // the FIFO token: its entry moves to the front
+        const uint32_t fi = (y << (r * L)) >> 27;
+        const uint32_t sd = fifo.len - 1u - fi;
+        past |= sd & f;  // negative: past the entries
+        const uint32_t d = sd & 15u;
+        const uint32_t h = 0u - (d >> 3);
+        const uint32_t a0 = fifo.f0 ^ ((fifo.f0 ^ fifo.f2) & h), a1 = fifo.f1 ^ ((fifo.f1 ^ fifo.f3) & h);
+        const uint32_t v = __byte_perm(a0, a1, d & 7u) & 0xFFu;
+        fifo.mtf_masked(v, masks[(d & f) | (16u & ~f)]);  // row 16 changes nothing
+        out[i * M] = me | (v << 8) | (t << 16);
+        t += r - f;
+    }
+}
+
+// A token's local id: the top bits of its field (idsh = 9 - the id width).
+__device__ __forceinline__ uint32_t tok_id(uint32_t rec, uint32_t idsh) { return (rec & 0x1FFu) >> idsh; }
+
+// All of a lane's records with the exact FIFO (a raw id is searched for and
+// moved from where it is, as in conn_parse); whether every FIFO index named
+// an entry.
+__device__ __noinline__ bool team_fifo_exact(uint16_t* row, uint32_t n, uint32_t idsh, const uint4* masks) {
+    MtfFifo fifo;
+    fifo.f0 = fifo.f1 = fifo.f2 = fifo.f3 = 0xFFFFFFFFu;
+    int32_t smin = 0;
+    for (uint32_t i = 0; i < n; i++) {
+        const uint32_t rec = row[i];
+        const bool raw = (rec & kTokRaw) != 0u;
+        const int32_t sd = static_cast<int32_t>(fifo.len) - 1 - static_cast<int32_t>((rec >> 4) & 31u);
+        smin = min(smin, raw ? 0 : sd);
+        const uint32_t s = static_cast<uint32_t>(sd) & 15u;
+        const uint32_t v = raw ? (tok_id(rec, idsh) & 0xFFu) : fifo.at(s);
+        const uint32_t at = raw ? fifo.find(v) : 16u;
+        const bool fresh = raw & (at == 16u);
+        fifo.mtf_masked(v, masks[raw ? (fresh ? min(fifo.len, 15u) : at) : s]);
+        fifo.len += (fresh & (fifo.len < 16u)) ? 1u : 0u;
+        if (!raw) row[i] = static_cast<uint16_t>((rec & ~0x1FFu) | ((v << idsh) & 0x1FFu));
+    }
+    return smin >= 0;
+}
+
+// A round's meshlet as every warp sees it, in shared memory.
+struct TeamFacts {
+    MeshParams P;
+    unsigned long long src16;           // arena offset of its bytes (16-byte aligned)
+    unsigned long long v_base, t_base;  // its first output rows (from the scan)
+    uint32_t placed;                    // ... which lie inside its mesh's
+    uint32_t m;                         // meshlet, or none when not in the round
+    uint32_t mi;                        // its mesh
+    uint32_t n_local, n_tris, n_tok, n_strips;
+    uint32_t start_bit, end_bit, ssz;   // ssz: bytes staged
+    uint32_t bit_off, walk_off, tok_off, asm_off, plane_off;  // bytes, then words
+    uint32_t axis_words;                // one axis' code plane
+    uint32_t idsh;                      // 9 - id width (_idx_bits_for, paradelta_codec.py:124-125)
+    // found on the way
+    uint32_t anchor;                    // the stream bit after the connectivity
+    uint32_t walk;                      // n_kind0 | n_walk << 16
+    uint32_t bad;                       // invalid connectivity: reported, the later phases skip it
+    uint32_t wbad;                      // invalid walk
+    uint32_t slow[3];                   // the axis is decoded by team_walk_slow
+};
+
+// One meshlet's assembly: a warp's state between windows of 32 tokens.
+struct TeamAsm {
+    uint32_t heads = 0u;    // heads of the window before
+    uint32_t last0 = 2u;    // the last token that reset p0 (edge code 0 or a strip's third root)
+    uint32_t tcnt = 0u, wcnt = 0u, kind0 = 0u, n_raw = 0u;
+    uint32_t t = 0u;        // records written
+    uint32_t t0 = 0u;       // the next window
+    uint32_t tp_prev = 0u;  // lane's token of the window before: its id's token before it, + 1
+    bool out = false;       // an id outside the meshlet (lane's)
+    bool redo = false;      // needs the exact FIFO
+};
+
+// A meshlet's token records from a chunk of steps, a lane per step (xs and
+// steps: its slots, M apart).  FIFO tokens get the field of their id, or keep
+// their index when `exact` (the exact FIFO resolves them).
+template <uint32_t M>
+__device__ __forceinline__ void team_records(TeamAsm& S, const TeamFacts& F, bool exact, uint16_t* __restrict__ row,
+                                             const uint32_t* __restrict__ xs, const uint32_t* __restrict__ steps,
+                                             int lane) {
+    const bool has = static_cast<uint32_t>(lane) < kTeamSteps;
+    const uint32_t x = has ? xs[lane * M] : 0u, st = has ? steps[lane * M] : 0u;
+    const bool body = (st & kStepBody) != 0u;
+    const uint32_t L = 9u - F.idsh + (body ? 2u : 1u), s = body ? 21u : 22u;
+    const uint32_t r = st & 3u, f = (st >> 2) & 1u, t = st >> 16;
+    if (r + f > 0u) row[t] = static_cast<uint16_t>((x >> s) | ((st & kStepHead) ? kTokHead : 0u));
+    if (r + f > 1u) row[t + 1u] = static_cast<uint16_t>((x << L) >> s);
+    if (r + f > 2u) row[t + 2u] = static_cast<uint16_t>((x << (2u * L)) >> s);
+    if (f && !exact) {
+        const uint32_t rec = ((x << (r * L)) >> s) & ~0x1FFu;
+        row[t + r] = static_cast<uint16_t>(rec | ((((st >> 8) & 0xFFu) << F.idsh) & 0x1FFu) |
+                                           (r == 0u && (st & kStepHead) ? kTokHead : 0u));
+    }
+    S.t = __shfl_sync(kFull, t + r + f, kTeamSteps - 1);
+    __syncwarp();
+}
+
+// Tokens [t0, t0 + 32) of a meshlet.  `row` has two readable entries before
+// it.  The walk goes out as entries in walk order and, as bytes, the vertices
+// of the parallelogram entries from the front of `vlist` and of the roots
+// from its end.  `exact`: by the exact
+// FIFO, raw ids need no check.
+__device__ __forceinline__ void team_window(TeamAsm& S, const TeamFacts& F, bool exact, uint32_t t0,
+                                            const uint16_t* __restrict__ row, uint32_t* __restrict__ walk,
+                                            uint8_t* __restrict__ vlist, uint32_t* __restrict__ last,
+                                            uint32_t* __restrict__ tri, int lane) {
+    const uint32_t me = 1u << lane, lt = me - 1u, le = lt | me;
+    const uint32_t n_tok = F.n_tok, n_local = F.n_local, idsh = F.idsh;
+    const uint32_t t = t0 + lane;
+    const bool in = t < n_tok;
+    const uint32_t rec = in ? row[t] : 0u;
+    const bool raw = (rec & kTokRaw) != 0u;
+    const uint32_t lm = __ballot_sync(kFull, in);
+    const uint32_t rm = __ballot_sync(kFull, raw);
+    const uint32_t hm = __ballot_sync(kFull, (rec & kTokHead) != 0u);
+    const uint32_t em = __ballot_sync(kFull, (rec & kTokEdge) != 0u);
+    const uint32_t id = tok_id(rec, idsh), v = id & 0xFFu;
+    const uint32_t v1 = tok_id(row[static_cast<int>(t) - 1], idsh) & 0xFFu;
+    const uint32_t v2 = tok_id(row[static_cast<int>(t) - 2], idsh) & 0xFFu;
+    // the id's token before this one, and the raw tokens up to it
+    const uint32_t same = __match_any_sync(kFull, in ? v : 256u + lane);
+    const uint32_t lw = last[v];  // (token + 1) << 16 | raw tokens up to it, 0: none
+    const uint32_t pm = same & lt;
+    const uint32_t pl = 31u - __clz(pm);
+    const bool seen = (pm | lw) != 0u;
+    const uint32_t raws = S.n_raw + __popc(rm & le);
+    const uint32_t raws_to = pm ? S.n_raw + __popc(rm & ((2u << (pl & 31u)) - 1u)) : lw & 0xFFFFu;
+    const uint32_t tp1 = in & seen ? (pm ? t0 + pl + 1u : lw >> 16) : 0u;
+    const bool isnew = raw & !seen;  // first occurrences are raw
+    __syncwarp();
+    if (in && (same & ~le) == 0u) last[v] = ((t + 1u) << 16) | raws;
+    const uint32_t nm = __ballot_sync(kFull, isnew);
+    const uint32_t r2 = ((hm << 2) | (S.heads >> 30)) & lm;  // third roots
+    const uint32_t rootm = hm | (hm << 1) | (S.heads >> 31) | r2;
+    const uint32_t bodym = lm & ~rootm;
+    const uint32_t emit = bodym | r2;
+    const uint32_t zm = r2 | (bodym & ~em);  // tokens that reset p0
+    const bool body = (bodym & me) != 0u;
+    S.out = S.out | (in & (id >= n_local));
+    // p0 before this token: the id two before the last reset
+    const uint32_t m = zm & lt;
+    const uint32_t l0 = m ? t0 + 31u - __clz(m) : S.last0;
+    const uint32_t p0p = tok_id(row[static_cast<int>(l0) - 2], idsh) & 0xFFu;
+    // edge code 0 -> (p1, p2 | p0), 1 -> (p0, p2 | p1) (:530-535)
+    const bool ec = body & ((em & me) != 0u);
+    const uint32_t p0 = ec ? p0p : v2;
+    const uint32_t cref = ec ? v2 : p0p;
+    const uint32_t ts = S.tcnt + __popc(emit & lt);
+    if ((emit & me) && ts < F.n_tris) tri[ts] = p0 | (v1 << 8) | (v << 16);
+    const uint32_t wi = S.wcnt + __popc(nm & lt);
+    if (isnew && wi < n_local) {
+        walk[wi] = body ? (v | (p0 << 8) | (v1 << 16) | (cref << 24)) : v * 0x01010101u;
+        const uint32_t rk = S.kind0 + __popc(nm & rootm & lt);  // roots before this entry
+        vlist[body ? wi - rk : n_local - 1u - rk] = static_cast<uint8_t>(v);
+    }
+    // The raw ids must be new to the FIFO.  Sixteen raw tokens since the id's
+    // token pushed it out; with fewer, sixteen distinct ids did: tokens since
+    // whose own predecessor lies before it.  (Counted as far back as the
+    // window before this one: a lower bound.)
+    if (!exact) {
+        for (uint32_t mb = __ballot_sync(kFull, raw & seen & (raws - raws_to <= 16u)); mb; mb &= mb - 1u) {
+            const uint32_t b = 31u - __clz(mb & (0u - mb));
+            const uint32_t from = __shfl_sync(kFull, tp1, b);  // that token + 1
+            const uint32_t now = __ballot_sync(kFull, in & (t >= from) & (tp1 < from)) & ((1u << b) - 1u);
+            const uint32_t before = __ballot_sync(kFull, t >= from + 32u && S.tp_prev < from);
+            S.redo = S.redo | (__popc(now) + __popc(before) < 16);
+        }
+        S.tp_prev = tp1;
+    }
+    S.kind0 += __popc(nm & rootm);
+    S.wcnt += __popc(nm);
+    S.tcnt += __popc(emit);
+    S.n_raw += __popc(rm);
+    S.last0 = zm ? t0 + 31u - __clz(zm) : S.last0;
+    S.heads = hm;
+    __syncwarp();
+}
+
+// A meshlet's first n triangles out to its index rows (out = idx + 3 *
+// t_base, ph = t_base & 3): whole quads as 48 bytes from a 16-byte boundary,
+// then the up to three triangles before the first and after the last.
+__device__ __forceinline__ void team_triangles(uint32_t* __restrict__ out, const uint32_t* __restrict__ tri, uint32_t ph,
+                                               uint32_t n, uint32_t vloc, int lane) {
+    auto id = [&](uint32_t p, uint32_t k) { return vloc + ((p >> (8u * k)) & 0xFFu); };
+    const uint32_t h = min((4u - ph) & 3u, n);   // head: [0, h)
+    const uint32_t q = h + ((n - h) & ~3u);      // whole quads: [h, q)
+    for (uint32_t l = h + 4u * lane; l < q; l += 128u) {
+        const uint32_t x = tri[l], y = tri[l + 1u], z = tri[l + 2u], w = tri[l + 3u];
+        uint4* o = reinterpret_cast<uint4*>(out + 3u * l);
+        o[0] = make_uint4(id(x, 0), id(x, 1), id(x, 2), id(y, 0));
+        o[1] = make_uint4(id(y, 1), id(y, 2), id(z, 0), id(z, 1));
+        o[2] = make_uint4(id(z, 2), id(w, 0), id(w, 1), id(w, 2));
+    }
+    const uint32_t odd = h + (n - q);
+    if (static_cast<uint32_t>(lane) < odd) {
+        const uint32_t l = static_cast<uint32_t>(lane) < h ? lane : q + (lane - h);
+        const uint32_t p = tri[l];
+        out[3u * l] = id(p, 0);
+        out[3u * l + 1u] = id(p, 1);
+        out[3u * l + 2u] = id(p, 2);
+    }
+}
+
+// Skip n codewords of one substream from bit `pos` of w (their lengths are
+// not stored), n its own in every lane of the warp (0: none).  Unary
+// (Rice(0)) codewords end at a one bit each: when every lane's are, whole
+// windows by their count of one bits, then the last one by halving.  Others
+// eight at a time; a lane that met one longer than the window takes its eight
+// again by the general reader.  False for a malformed one.
+__device__ __forceinline__ bool team_skip(const uint32_t* __restrict__ w, uint32_t& pos, uint32_t tk, uint32_t n,
+                                          uint32_t limit) {
+    const uint32_t most = __reduce_max_sync(kFull, n);
+    if (most == 0u) return true;
+    bool ok = true;
+    BitBuf<true> b;
+    b.w = w;
+    b.end_word = 0u;
+    b.seek(pos);
+    if (__all_sync(kFull, tk == 0u || n == 0u)) {
+        uint32_t c;
+        while ((c = __popc(b.hi)) < n) {
+            b.skip(32u);
+            n -= c;
+            if (b.at() > limit) break;  // only a corrupt stream runs past its meshlet
+        }
+        __syncwarp();
+        uint32_t y = b.hi, at = 0u, need = n;
+#pragma unroll
+        for (uint32_t wd = 16u; wd >= 1u; wd >>= 1) {
+            const uint32_t t = __popc(y >> (32u - wd));  // ones in the top wd bits
+            const bool more = t < need;
+            need -= more ? t : 0u;
+            y = more ? (y << wd) : y;
+            at += more ? wd : 0u;
+        }
+        b.skip(n ? at + 1u : 0u);
+    } else {
+        const uint32_t k1 = (tk & 0x3Fu) + 1u, em = (tk & 0x80u) ? 2u : 1u;
+        for (uint32_t i0 = 0; i0 < most; i0 += 8u) {
+            uint32_t from = b.at();
+            bool longc = false;
+#pragma unroll
+            for (uint32_t i = 0; i < 8u; i++) {
+                const bool on = i0 + i < n;
+                const uint32_t len = __clz(b.hi) * em + k1;
+                longc = longc | (on & (len > 32u));
+                b.skip(on ? min(len, 32u) : 0u);
+            }
+            if (longc) {
+                const uint32_t m = min(8u, n - i0);
+                int32_t r;
+                for (uint32_t i = 0; i < m; i++) ok = residual<true>(w, 0u, from, tk, limit, r) & ok;
+                b.seek(from);
+            }
+            if (b.at() > limit) b.seek(limit), ok = false;
+            __syncwarp();
+        }
+    }
+    pos = b.at();
+    return ok & (pos <= limit);
+}
+
+// One (meshlet, axis) of the residual decoder: a lane of a decoder warp.
+struct TeamAxis {
+    uint32_t pos0;         // the first substream's bit, after the (tag, k) pairs
+    uint32_t cp, cdd;      // parallelogram and delta cursors (bits of w)
+    uint32_t tp, td;       // their (tag, k)
+    uint32_t tk[6];
+    uint32_t n_para, n_delta;
+    int32_t anc;
+    bool bad, slow;
+};
+
+// Anchor codes and (tag, k) pairs (paradelta_v5_dup.py:544-557); `act`: the
+// lane has a meshlet.
+template <bool kShared>
+__device__ __forceinline__ void team_axis_open(TeamAxis& X, const MeshParams* __restrict__ P, uint32_t d, bool act,
+                                               uint32_t anchor_bit, uint32_t end, uint32_t wk,
+                                               const uint32_t* __restrict__ w, uint32_t rbase) {
+    uint32_t pos = anchor_bit + rbase;
+    X.bad = !act;
+    X.slow = !kShared;
+    X.anc = 0;
+#pragma unroll
+    for (int i = 0; i < 6; i++) X.tk[i] = 0u;
+    if (act) {
+#pragma unroll
+        for (uint32_t e = 0; e < 3u; e++) {
+            const uint32_t gb = P->g_bits[e];
+            const int32_t v = gb ? static_cast<int32_t>(peek32<kShared>(w, pos) >> (32u - gb)) : 0;
+            X.anc = e == d ? v : X.anc;
+            pos += gb;
+        }
+#pragma unroll
+        for (int i = 0; i < 6; i++) {
+            const uint32_t t = peek32<kShared>(w, pos) >> 16;
+            pos += 16u;
+            const uint32_t k = t & 0xFFu;
+            X.bad = X.bad || k > static_cast<uint32_t>(kMaxResidK);
+            X.tk[i] = ((t >> 8) == 1u ? 0u : 0x80u) | (k & 0x3Fu);
+        }
+        X.bad = X.bad || pos > end + rbase;
+    }
+    const uint32_t n_kind0 = wk & 0xFFFFu;
+    X.n_delta = n_kind0 ? n_kind0 - 1u : 0u;  // the anchor has no delta
+    X.n_para = (wk >> 16) - n_kind0;
+    X.pos0 = X.cp = X.cdd = pos;
+    X.td = d == 0u ? X.tk[0] : (d == 1u ? X.tk[1] : X.tk[2]);
+    X.tp = d == 0u ? X.tk[3] : (d == 1u ? X.tk[4] : X.tk[5]);
+}
+
+// Eight codewords of a parallelogram substream as residuals into the code
+// plane at their vertices, the first n of the eight bytes at `list`.  A lane that
+// met one longer than the window takes its eight again by the general
+// reader.  A residual that does not fit the plane sets `slow`; false for a
+// malformed codeword.
+// kDown: the list runs backwards; kStore false: only skipped.
+template <bool kWide, bool kDown>
+__device__ __forceinline__ bool team_decode(BitBuf<true>& b, uint32_t tk, uint32_t limit,
+                                            const uint8_t* __restrict__ list, int n, bool store, uint32_t plane,
+                                            bool& slow) {
+    constexpr uint32_t kSize = sizeof(PlaneT<kWide>);
+    const uint32_t k = tk & 0x3Fu, k1 = k + 1u;
+    const bool eg = (tk & 0x80u) != 0u;
+    const uint32_t em = eg ? 2u : 1u, zmul = eg ? 0u : 1u << k, pow = 1u << k;
+    uint32_t l0 = 0u, l1 = 0u;
+    if constexpr (!kDown) {
+        l0 = reinterpret_cast<const uint32_t*>(list)[0];
+        l1 = reinterpret_cast<const uint32_t*>(list)[1];
+    }
+    uint32_t from = b.at(), u[8];
+    bool longc = false, ok = true;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const uint32_t z = __clz(b.hi);
+        const uint32_t len = z * em + k1;
+        longc = longc | ((i < n) & (len > 32u));
+        // the value bits with the terminator as their leading one: 2^nb + value
+        u[i] = z * zmul + ((b.hi >> ((32u - len) & 31u)) - pow);
+        b.skip(i < n ? min(len, 32u) : 0u);
+    }
+    if (longc) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            if (i < n) {
+                int32_t r;
+                ok = residual<true>(b.w, 0u, from, tk, limit, r) & ok;
+                u[i] = (static_cast<uint32_t>(r) << 1) ^ static_cast<uint32_t>(r >> 31);
+            }
+        }
+        b.seek(from);
+    }
+    uint32_t big = 0u;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const bool on = store & (i < n);
+        const uint32_t v = kDown ? (on ? list[-i] : 0u) : __byte_perm(i < 4 ? l0 : l1, 0u, 0x4440u | (i & 3));
+        const uint32_t at = mad_u32(v, kSize, plane);
+        if (on) {
+            const int32_t r = unzigzag(u[i]);
+            if constexpr (kWide) {
+                asm volatile("st.shared.u32 [%0], %1;" ::"r"(at), "r"(r) : "memory");
+            } else {
+                asm volatile("st.shared.u16 [%0], %1;" ::"r"(at), "h"(static_cast<short>(r)) : "memory");
+                big |= u[i];
+            }
+        }
+    }
+    slow = slow | (big > 0xFFFFu);  // outside 16 bits
+    if (b.at() > limit) {
+        b.seek(limit);
+        ok = false;
+    }
+    return ok;
+}
+
+// IRLP of walk entries [h, h + 8) below n_walk (paradelta_v5_dup.py:91-104,
+// 581-600): a vertex's residual is in its place of the code plane.  The
+// plane's addresses are formed for all eight entries first, with multiply-adds
+// (the integer ALU, which issues every other cycle, has the byte extractions),
+// so that only loads, arithmetic and the store are between one code and the
+// next: 86 cycles an entry on one warp against 143 with the addresses where
+// they are used.
+template <bool kWide>
+__device__ __forceinline__ void team_predict(uint32_t plane, const uint32_t* __restrict__ walk, uint32_t h,
+                                             uint32_t n_walk, int32_t n0, int32_t n1, int32_t n2, int32_t K,
+                                             int32_t half, int32_t& prev, uint32_t& codes) {
+    constexpr uint32_t kSize = sizeof(PlaneT<kWide>);
+    uint32_t av[8], aa[8], ab[8], ac[8];
+    bool para[8];
+#pragma unroll
+    for (uint32_t i = 0; i < 8u; i++) {
+        const uint32_t e = h + i < n_walk ? walk[h + i] : 0u;
+        av[i] = mad_u32(__byte_perm(e, 0u, 0x4440u), kSize, plane);
+        aa[i] = mad_u32(__byte_perm(e, 0u, 0x4441u), kSize, plane);
+        ab[i] = mad_u32(__byte_perm(e, 0u, 0x4442u), kSize, plane);
+        ac[i] = mad_u32(e >> 24, kSize, plane);
+        para[i] = av[i] != aa[i];  // roots are stored as (v, v, v, v)
+    }
+#pragma unroll
+    for (uint32_t i = 0; i < 8u; i++) {
+        const bool act = h + i < n_walk;
+        int32_t r, ca, cb, cc;
+        if constexpr (kWide) {
+            asm volatile("ld.shared.s32 %0, [%1];" : "=r"(r) : "r"(av[i]) : "memory");
+            asm volatile("ld.shared.s32 %0, [%1];" : "=r"(ca) : "r"(aa[i]) : "memory");
+            asm volatile("ld.shared.s32 %0, [%1];" : "=r"(cb) : "r"(ab[i]) : "memory");
+            asm volatile("ld.shared.s32 %0, [%1];" : "=r"(cc) : "r"(ac[i]) : "memory");
+        } else {
+            asm volatile("ld.shared.s16 %0, [%1];" : "=r"(r) : "r"(av[i]) : "memory");
+            asm volatile("ld.shared.u16 %0, [%1];" : "=r"(ca) : "r"(aa[i]) : "memory");
+            asm volatile("ld.shared.u16 %0, [%1];" : "=r"(cb) : "r"(ab[i]) : "memory");
+            asm volatile("ld.shared.u16 %0, [%1];" : "=r"(cc) : "r"(ac[i]) : "memory");
+            if (i == 0u) r = h == 0u ? r & 0xFFFF : r;  // the first entry is the anchor, a code
+        }
+        const int32_t code = (para[i] ? (n0 * ca + n1 * cb + n2 * cc + half) >> K : prev) + r;
+        if (act) {
+            if constexpr (kWide) {
+                asm volatile("st.shared.u32 [%0], %1;" ::"r"(av[i]), "r"(code) : "memory");
+            } else {
+                asm volatile("st.shared.u16 [%0], %1;" ::"r"(av[i]), "h"(static_cast<short>(code)) : "memory");
+            }
+            codes |= static_cast<uint32_t>(code);
+        }
+        prev = code;
+    }
+}
+
+// The whole axis by the general reader, one lane: substream starts,
+// residuals and IRLP together.  For residuals wider than the plane and
+// meshlets read in place.
+template <bool kShared, bool kWide>
+__device__ __noinline__ bool team_walk_slow(TeamAxis& X, const MeshParams* P, uint32_t d, const uint32_t* w,
+                                            uint32_t limit, const uint32_t* walk, uint32_t n_walk,
+                                            PlaneT<kWide>* plane) {
+    uint32_t pos = X.pos0;
+    X.cdd = pos;
+    for (uint32_t e = 0; e < 3u + d; e++) {
+        if (e == d && e < 3u) X.cdd = pos;
+        if (!skip_codes<kShared>(w, 0u, pos, X.tk[e], e < 3u ? X.n_delta : X.n_para, limit)) return false;
+    }
+    X.cp = pos;
+    uint32_t cp = pos, cdd = X.cdd;
+    const int32_t n0 = P->pred_n[3 * d], n1 = P->pred_n[3 * d + 1], n2 = P->pred_n[3 * d + 2];
+    const int32_t K = P->pred_k[d], half = P->pred_half[d];
+    const uint32_t cmax = P->code_max[d];
+    int32_t prev = X.anc;
+    bool ok = true;
+    for (uint32_t i = 0; i < n_walk; i++) {
+        const uint32_t e = walk[i], v = e & 0xFFu, ra = (e >> 8) & 0xFFu;
+        const bool para = ra != v;
+        int32_t code = prev;  // the anchor's
+        if (i) {
+            int32_t r;
+            uint32_t p = para ? cp : cdd;
+            ok = residual<kShared>(w, 0u, p, para ? X.tp : X.td, limit, r) & ok;
+            cp = para ? p : cp;
+            cdd = para ? cdd : p;
+            const int32_t ca = static_cast<int32_t>(plane[ra]), cb = static_cast<int32_t>(plane[(e >> 16) & 0xFFu]),
+                          cc = static_cast<int32_t>(plane[e >> 24]);
+            code = (para ? (n0 * ca + n1 * cb + n2 * cc + half) >> K : prev) + r;
+        }
+        ok = ok & (static_cast<uint32_t>(code) <= cmax);
+        plane[v] = static_cast<PlaneT<kWide>>(code);
+        prev = code;
+    }
+    X.pos0 = cp;  // where the axis' parallelogram codewords end
+    return ok;
+}
+
+// Positions (and codes) of one meshlet: lane per vertex.
+template <bool kWide>
+__device__ __forceinline__ void team_emit(const DecodeArgs& a, const MeshParams* __restrict__ P, uint32_t nv,
+                                          unsigned long long vb, const PlaneT<kWide>* __restrict__ plane,
+                                          uint32_t stride, int lane) {
+    float* __restrict__ dst = a.pos + 3ull * vb;
+    if (P->has_lut) {
+        const uint32_t g0 = P->g_bits[0], g1 = P->g_bits[1];
+        const float* __restrict__ l0 = a.lut + P->lut_off;
+        const float* __restrict__ l1 = l0 + (1u << g0);
+        const float* __restrict__ l2 = l1 + (1u << g1);
+        // codes lie inside the tables: an invalid meshlet is not written
+#pragma unroll 4
+        for (uint32_t v = lane; v < nv; v += 32u) {
+            const float x = __ldcg(l0 + plane[v]), y = __ldcg(l1 + plane[v + stride]),
+                        z = __ldcg(l2 + plane[v + 2u * stride]);
+            dst[3u * v] = x;
+            dst[3u * v + 1u] = y;
+            dst[3u * v + 2u] = z;
+        }
+    } else {
+#pragma unroll
+        for (uint32_t d = 0; d < 3u; d++) {
+            stride_dequant_axis c;
+            c.a_hi = P->dq[d].a_hi;
+            c.a_lo = P->dq[d].a_lo;
+            c.b_hi = P->dq[d].b_hi;
+            c.b_lo = P->dq[d].b_lo;
+            c.err = P->dq[d].err;
+            const bool zero_bits = P->dq[d].zero_bits != 0;
+            for (uint32_t v = lane; v < nv; v += 32u) {
+                const uint32_t q = static_cast<uint32_t>(plane[v + d * stride]);
+                float y;
+                const bool fast = stride_dequant_fast(&c, q, &y) != 0;
+                if (!fast || zero_bits) y = dequant_slow(P, d, q);
+                dst[3u * v + d] = y;
+            }
+        }
+    }
+    if (a.codes) {
+        int32_t* cd = a.codes + 3ull * vb;
+        for (uint32_t v = lane; v < nv; v += 32u) {
+            cd[3u * v] = static_cast<int32_t>(plane[v]);
+            cd[3u * v + 1u] = static_cast<int32_t>(plane[v + stride]);
+            cd[3u * v + 2u] = static_cast<int32_t>(plane[v + 2u * stride]);
+        }
+    }
+}
+
+template <uint32_t M>
+struct TeamShared {
+    uint4 masks[17];
+    TeamFacts f[M];
+    // parser steps of three chunks (being written; with the FIFO; with the assemblers)
+    uint32_t x[3][kTeamSteps * M];
+    uint32_t step[3][kTeamSteps * M];
+    uint8_t meta[3][kTeamSteps * M];
+    uint32_t more[2];  // the parser has tokens left after its last chunk
+    uint32_t rmask;   // meshlets of the round
+    uint32_t walk_base, uni_base;  // bytes
+    uint32_t staged;
+    uint32_t redo;    // decode the connectivity again, with the exact FIFO
+};
+
+// The meshlets of a round from their bytes to positions.
+template <uint32_t M, bool kShared, bool kWide>
+__device__ __forceinline__ void team_round(const DecodeArgs& a, TeamShared<M>& s, uint8_t* bits, uint32_t warp,
+                                           int lane) {
+    const uint32_t rmask = s.rmask;
+    uint32_t* walks = reinterpret_cast<uint32_t*>(bits + s.walk_base);
+    uint32_t* uni = reinterpret_cast<uint32_t*>(bits + s.uni_base);
+    constexpr uint32_t kPer = (M + kTeamAsm - 1u) / kTeamAsm;  // meshlets of an assembler warp
+    const bool assembler = warp != kTeamParser && warp != kTeamFifo;
+    const uint32_t aw0 = team_asm_index(warp);  // an assembler's first meshlet
+    const uint32_t* bit_words = reinterpret_cast<const uint32_t*>(bits);
+    // 1. stage
+    if (assembler) {
+        for (uint32_t j = aw0; j < M; j += kTeamAsm) {
+            if (!((rmask >> j) & 1u)) continue;  // warp-uniform, here and below
+            TeamFacts& F = s.f[j];
+            const uint32_t* ps = reinterpret_cast<const uint32_t*>(a.meshes + F.mi);
+            uint32_t* pd = reinterpret_cast<uint32_t*>(&F.P);
+            for (uint32_t i = lane; i < sizeof(MeshParams) / 4u; i += 32u) pd[i] = __ldcg(ps + i);
+            if constexpr (kShared) {
+                const uint32_t n16 = F.ssz >> 4;
+                const uint4* src = reinterpret_cast<const uint4*>(a.arena + F.src16);
+                uint4* dst = reinterpret_cast<uint4*>(bits + F.bit_off);
+                for (uint32_t i = lane; i < n16; i += 32u) {
+                    uint4 q = __ldcg(src + i);
+                    q.x = bswap32(q.x);
+                    q.y = bswap32(q.y);
+                    q.z = bswap32(q.z);
+                    q.w = bswap32(q.w);
+                    dst[i] = q;
+                }
+            }
+        }
+    }
+    // bit p of the stream is bit p + rbase of w
+    auto base_of = [&](const TeamFacts& F, const uint32_t*& w) -> uint32_t {
+        w = kShared ? bit_words : reinterpret_cast<const uint32_t*>(a.arena + F.P.blob_off);
+        return kShared ? static_cast<uint32_t>((F.P.blob_off - F.src16 + F.bit_off) * 8ull) : 0u;
+    };
+    // Output rows of the warp's meshlet, once the scan has ended: inside its
+    // mesh's (header n_v_total, n_t), and the last meshlet's end exactly there
+    // (see placement_ok).
+    auto place = [&](TeamFacts& F) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        if (lane == 0) {
+            const MeshletDesc* D = a.descs + F.m;
+            const BlockPrefix* bp = a.blk_prefix + F.m / kScanThreads;
+            const bool failed = *reinterpret_cast<volatile unsigned long long*>(&a.status->err) != 0ull;
+            F.v_base = __ldcg(&bp->v) + __ldcg(&D->v_pref);
+            F.t_base = __ldcg(&bp->t) + __ldcg(&D->t_pref);
+            const unsigned long long v0 = F.P.v_offset, v1 = v0 + F.P.n_v, t0 = F.P.t_offset, t1 = t0 + F.P.n_t;
+            const unsigned long long ve = F.v_base + F.n_local, te = F.t_base + F.n_tris;
+            bool ok = F.v_base >= v0 && ve <= v1 && F.t_base >= t0 && te <= t1;
+            if (ok && F.m - F.P.meshlet_begin + 1u == F.P.n_meshlets) ok = ve == v1 && te == t1;
+            F.placed = ok && !failed ? 1u : 0u;
+        }
+        __syncwarp();
+    };
+    bool placed = false;
+    for (uint32_t pass = 0; pass < 2u; pass++) {  // the second one with the exact FIFO, rarely
+        const bool exact = pass != 0u;
+        if (threadIdx.x == 0) s.redo = 0u;
+        if (threadIdx.x < M) {
+            TeamFacts& F = s.f[threadIdx.x];
+            F.bad = F.wbad = F.slow[0] = F.slow[1] = F.slow[2] = 0u;
+        }
+        __syncthreads();
+        // 2. connectivity, in step: chunk c with the parser, c - 1 with the
+        // FIFO warp, c - 2 with the assemblers
+        if (!assembler) {
+            const bool act = (rmask >> lane) & 1u;
+            TeamFacts& F = s.f[act ? lane : 0];
+            const uint32_t* w;
+            const uint32_t rbase = base_of(F, w);
+            const uint32_t n_tok = act ? F.n_tok : 0u;
+            const uint32_t ib = 9u - F.idsh;
+            uint16_t* row = reinterpret_cast<uint16_t*>(uni + F.tok_off) + 2;
+            const uint32_t sl = act ? lane : 0u;  // an idle lane repeats the first one's steps
+            TeamParse T;
+            MtfFifo fifo;
+            uint32_t t = 0u;
+            uint32_t past = 0u;  // negative: a FIFO index named no entry
+            T.strips = F.n_strips;
+            T.pos = act ? F.start_bit + 48u + rbase : 0u;
+            fifo.f0 = fifo.f1 = fifo.f2 = fifo.f3 = 0xFFFFFFFFu;
+            if (warp == kTeamParser && act) {
+                row[-2] = row[-1] = 0;
+            }
+            bool more = true;
+            for (uint32_t c = 0;; c++) {
+                if (warp == kTeamParser) {
+                    const uint32_t b = c % 3u;
+                    if (act) team_parse<kShared, M>(T, w, n_tok, ib, F.end_bit + rbase + 1u, s.x[b] + lane, s.meta[b] + lane);
+                    __syncwarp();
+                    const bool m = __any_sync(kFull, T.t < n_tok);
+                    if (lane == 0) s.more[c & 1u] = m ? 1u : 0u;
+                } else if (c > 0u) {
+                    const uint32_t b = (c - 1u) % 3u;
+                    if (act) team_fifo<M>(fifo, t, s.x[b] + sl, s.meta[b] + sl, s.step[b] + sl, ib, s.masks, past);
+                }
+                __syncwarp();
+                team_all_bar();
+                if (!more) break;  // this was the chunk after the parser's last
+                more = s.more[c & 1u] != 0u;
+            }
+            if (act && warp == kTeamParser) {
+                const uint32_t pos = T.pos - rbase;  // the stream bit after the last token
+                F.anchor = pos;
+                // every strip read, inside the meshlet
+                if (T.t != n_tok || T.strips != 0u || T.left != 0u || pos > F.end_bit) atomicOr(&F.bad, 1u);
+            }
+            if (exact) team_all_bar();  // the records are there
+            if (act && warp == kTeamFifo) {
+                if (exact ? !team_fifo_exact(row, n_tok, F.idsh, s.masks) : sign_mask(past) != 0u) atomicOr(&F.bad, 1u);
+            }
+            __syncwarp();
+            if (exact) team_all_bar();
+        } else {
+            TeamAsm S[kPer];
+#pragma unroll
+            for (uint32_t q = 0; q < kPer; q++) {
+                const uint32_t j = aw0 + q * kTeamAsm;
+                if (j >= M || !((rmask >> j) & 1u)) continue;
+                uint4* last = reinterpret_cast<uint4*>(uni + s.f[j].asm_off);
+                last[lane] = last[lane + 32] = make_uint4(0u, 0u, 0u, 0u);
+            }
+            __syncwarp();
+            // the windows that the records fill (or end)
+            auto windows = [&](TeamAsm& A, const TeamFacts& F) {
+                uint32_t* walk = walks + F.walk_off;
+                uint32_t* last = uni + F.asm_off;
+                const uint32_t have = A.t >= F.n_tok ? F.n_tok + 31u : A.t;
+                for (; A.t0 + 32u <= have; A.t0 += 32u)
+                    team_window(A, F, exact, A.t0, reinterpret_cast<const uint16_t*>(uni + F.tok_off) + 2, walk,
+                                reinterpret_cast<uint8_t*>(walk + F.n_local), last, last + 256, lane);
+            };
+            auto chunk = [&](uint32_t c) {
+#pragma unroll
+                for (uint32_t q = 0; q < kPer; q++) {
+                    const uint32_t j = aw0 + q * kTeamAsm;
+                    if (j >= M || !((rmask >> j) & 1u)) continue;
+                    const TeamFacts& F = s.f[j];
+                    if (S[q].t >= F.n_tok) continue;
+                    team_records<M>(S[q], F, exact, reinterpret_cast<uint16_t*>(uni + F.tok_off) + 2,
+                                    s.x[c % 3u] + j, s.step[c % 3u] + j, lane);
+                    if (!exact) windows(S[q], F);
+                }
+            };
+            bool more = true;
+            uint32_t c = 0u;
+            for (;; c++) {
+                if (c > 1u) chunk(c - 2u);
+                team_all_bar();
+                if (!more) break;
+                more = s.more[c & 1u] != 0u;
+            }
+            chunk(c - 1u);  // the parser's last chunk
+            if (exact) {
+                __syncwarp();
+                team_all_bar();
+                team_all_bar();  // the FIFO warp has resolved the records
+#pragma unroll
+                for (uint32_t q = 0; q < kPer; q++) {
+                    const uint32_t j = aw0 + q * kTeamAsm;
+                    if (j < M && ((rmask >> j) & 1u)) windows(S[q], s.f[j]);
+                }
+            }
+#pragma unroll
+            for (uint32_t q = 0; q < kPer; q++) {
+                const uint32_t j = aw0 + q * kTeamAsm;
+                if (j >= M || !((rmask >> j) & 1u)) continue;
+                TeamFacts& F = s.f[j];
+                if (!placed) place(F);
+                // triangle indices are relative to the mesh's first vertex
+                if (F.placed)
+                    team_triangles(a.idx + 3ull * F.t_base, uni + F.asm_off + 256,
+                                   static_cast<uint32_t>(F.t_base) & 3u, min(S[q].tcnt, F.n_tris),
+                                   static_cast<uint32_t>(F.v_base - F.P.v_offset), lane);
+                const bool bad = __any_sync(kFull, S[q].out) || S[q].tcnt != F.n_tris || !F.placed;
+                if (lane == 0) {
+                    F.walk = S[q].kind0 | (min(S[q].wcnt, F.n_local) << 16);
+                    if (bad) atomicOr(&F.bad, 1u);
+                    if (S[q].redo && !exact) s.redo = 1u;
+                }
+            }
+        }
+        __syncthreads();
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        if (threadIdx.x < M && ((rmask >> threadIdx.x) & 1u)) a.descs[s.f[threadIdx.x].m].anchor_bit = s.f[threadIdx.x].anchor;
+        placed = true;
+        if (s.redo == 0u || exact) break;
+        __syncthreads();  // everyone has read it
+    }
+    // 3. walk: lane (axis, meshlet) of a decoder warp and of the predictor
+    // warp a chunk behind it, so that the chains of the bit cursor and of the
+    // codes run side by side.  A residual waits in its vertex's own place of
+    // the code plane, which nothing reads before the vertex is reached.
+    constexpr uint32_t kDec = team_dec_warps<M>();
+    if (warp < 2u * kDec) {
+        const uint32_t k = warp % kDec;
+        const uint32_t tid = 32u * k + lane;
+        const uint32_t d = tid / M < 3u ? tid / M : 2u, j = tid % M;
+        TeamFacts& F = s.f[j];
+        const MeshParams& P = F.P;
+        const bool on = tid < 3u * M && ((rmask >> j) & 1u) && F.bad == 0u;
+        const uint32_t nl = on ? F.n_local : 0u;
+        const uint32_t wk = on ? F.walk : 0u;
+        const uint32_t n_walk = wk >> 16;
+        // (a lane without a meshlet reads the front of each array)
+        const uint32_t* __restrict__ walk = walks + (on ? F.walk_off : 0u);
+        const uint8_t* __restrict__ vlist = reinterpret_cast<const uint8_t*>(walk + nl);
+        PlaneT<kWide>* __restrict__ plane = reinterpret_cast<PlaneT<kWide>*>(uni + (on ? F.plane_off + d * F.axis_words : 0u));
+        const uint32_t chunks = (__reduce_max_sync(kFull, n_walk) + kTeamRes - 1u) / kTeamRes;
+        const bool decoder = warp < kDec;
+        if (!decoder && n_walk < nl && on) {  // vertices the walk never reaches keep code 0
+            uint32_t* z = reinterpret_cast<uint32_t*>(plane);
+            const uint32_t nz = (nl * static_cast<uint32_t>(sizeof(PlaneT<kWide>)) + 3u) >> 2;
+            for (uint32_t i = 0; i < nz; i++) z[i] = 0u;
+        }
+        __syncwarp();
+        team_dec_bar(k);
+        if (decoder) {
+            const uint32_t* w;
+            const uint32_t rbase = base_of(F, w);
+            const uint32_t limit = on ? F.end_bit + rbase : 0u;
+            TeamAxis X;
+            team_axis_open<kShared>(X, &P, d, on, F.anchor, F.end_bit, wk, w, rbase);
+            BitBuf<true> b;
+            b.w = w;
+            b.end_word = 0u;
+            const uint32_t plane_addr = smem_addr(plane);
+            bool run = kShared && !X.bad;
+            if constexpr (kShared) {
+                // dx dy dz, the lane's own one into its roots' places; then the
+                // parallelogram substreams before its own
+                const uint32_t nd = run ? X.n_delta : 0u;
+                const uint32_t most = __reduce_max_sync(kFull, nd);
+                b.seek(run ? X.pos0 : 0u);
+#pragma unroll
+                for (uint32_t e = 0; e < 3u; e++) {
+                    X.cdd = e == d ? b.at() : X.cdd;
+#pragma unroll 1
+                    for (uint32_t i = 0; i < most; i += 8u) {
+                        run = team_decode<kWide, true>(b, X.tk[e], limit, vlist + nl - 2u - i,
+                                                       run ? static_cast<int>(nd) - static_cast<int>(i) : 0, e == d,
+                                                       plane_addr, X.slow) & run;
+                        __syncwarp();
+                    }
+                }
+                uint32_t pos = b.at();
+#pragma unroll
+                for (uint32_t e = 0; e < 2u; e++) {
+                    run = team_skip(w, pos, X.tk[3 + e], run && e < d ? X.n_para : 0u, limit) & run;
+                    __syncwarp();
+                }
+                X.cp = pos;
+                run = run && n_walk;
+                if (run) plane[vlist[nl - 1u]] = static_cast<PlaneT<kWide>>(X.anc);  // the first root is the anchor
+                X.bad = X.bad || (n_walk && !run);
+                b.seek(run ? X.cp : 0u);
+            }
+            const uint32_t np = run ? X.n_para : 0u;
+            for (uint32_t c = 0; c <= chunks; c++) {
+                if constexpr (kShared) {
+                    if (c < chunks) {
+                        const uint32_t i0 = c * kTeamRes;
+#pragma unroll 1
+                        for (uint32_t h = 0; h < kTeamRes; h += 8u) {
+                            if (!team_decode<kWide, false>(b, X.tp, limit, vlist + i0 + h,
+                                                           static_cast<int>(np) - static_cast<int>(i0 + h), true,
+                                                           plane_addr, X.slow))
+                                X.bad = true;
+                            __syncwarp();
+                        }
+                    }
+                }
+                if (c == chunks && on) F.slow[d] = X.slow ? 1u : 0u;
+                __syncwarp();
+                team_dec_bar(k);
+            }
+            uint32_t cend = run ? b.at() : X.cp;
+            team_dec_bar(k);  // the predictor has left the planes
+            if (on && X.slow) {
+                TeamAxis Y = X;  // a copy: only this path keeps it in memory
+                X.bad = !team_walk_slow<kShared, kWide>(Y, &P, d, w, limit, walk, n_walk, plane);
+                cend = Y.pos0;
+                X.cp = Y.cp;
+                X.cdd = Y.cdd;
+            }
+            if (on) {
+                // pz, the last substream, must end where the next meshlet starts (:507)
+                const bool last = F.m - P.meshlet_begin + 1u == P.n_meshlets;
+                const bool ends = (d != 2u || last) ? cend <= limit : cend == limit;
+                if (X.bad || !ends) atomicOr(&F.wbad, 1u);
+                // the side table: this axis' substream starts after the anchor
+                const uint32_t a0 = F.anchor + rbase;
+                const uint32_t rp = min(X.cp - a0, 0xFFFFu), rd = min(X.cdd - a0, 0xFFFFu);
+                uint16_t* so = a.descs[F.m].sub_offs;
+                if (d != 0u) so[d - 1u] = static_cast<uint16_t>(rd);
+                so[2u + d] = static_cast<uint16_t>(rp);
+            }
+        } else {
+            const int32_t n0 = P.pred_n[3 * d], n1 = P.pred_n[3 * d + 1], n2 = P.pred_n[3 * d + 2];
+            const int32_t K = P.pred_k[d], half = P.pred_half[d];
+            const uint32_t cmax = P.code_max[d];
+            int32_t prev = 0;
+            uint32_t codes = 0u;  // every code, or-ed
+            const uint32_t plane_addr = smem_addr(plane);
+            for (uint32_t c = 0; c <= chunks; c++) {
+                if (c > 0u) {
+                    const uint32_t i0 = (c - 1u) * kTeamRes;
+#pragma unroll 1
+                    for (uint32_t h = i0; h < i0 + kTeamRes; h += 8u)
+                        team_predict<kWide>(plane_addr, walk, h, n_walk, n0, n1, n2, K, half, prev, codes);
+                }
+                __syncwarp();
+                team_dec_bar(k);
+            }
+            // codes of a valid stream lie in [0, 2^g_bits)
+            if (on && (codes & ~cmax) != 0u && F.slow[d] == 0u) atomicOr(&F.wbad, 1u);
+            __syncwarp();
+            team_dec_bar(k);
+        }
+    }
+    __syncthreads();
+    // 4. emit
+    if (assembler) {
+        for (uint32_t j = aw0; j < M; j += kTeamAsm) {
+            const TeamFacts& F = s.f[j];
+            if (!((rmask >> j) & 1u)) continue;
+            if (F.bad | F.wbad) {
+                if (lane == 0) report(a.status, kErrCorrupt, F.m);
+                continue;
+            }
+            team_emit<kWide>(a, &F.P, F.n_local, F.v_base,
+                             reinterpret_cast<const PlaneT<kWide>*>(uni + F.plane_off),
+                             F.axis_words * 4u / static_cast<uint32_t>(sizeof(PlaneT<kWide>)), lane);
+        }
+    }
+    __syncthreads();  // the next round overwrites the shared memory
+}
+
+template <uint32_t M, bool kWide>
+__global__ void __launch_bounds__(kTeamThreads, 2) team_kernel(DecodeArgs a, uint32_t smem_bytes) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    __shared__ TeamShared<M> s;
+    if (threadIdx.x < 17u)
+        s.masks[threadIdx.x] = threadIdx.x < 16u ? mtf_mask_row(threadIdx.x) : make_uint4(0u, 0u, 0u, 0u);
+    const uint32_t warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    uint32_t todo = 0u, nb = 0u, nw = 0u, nt = 0u, na = 0u, np = 0u;
+    if (warp == 0u) {
+        bool ok = false;
+        if (static_cast<uint32_t>(lane) < M) {
+            TeamFacts& F = s.f[lane];
+            MeshletDesc D;
+            memset(&D, 0, sizeof(D));
+            F.m = blockIdx.x * M + lane;
+            F.mi = 0u;
+            F.ssz = 0u;
+            if (F.m < a.total_meshlets) {
+                F.mi = a.meshlet_mesh ? __ldcg(a.meshlet_mesh + F.m) : 0u;
+                const MeshParams& P = a.meshes[F.mi];
+                ok = scan_meshlet(a.arena, P, F.m - P.meshlet_begin, D) == 0;  // the scan reports an error
+                const unsigned long long blob = P.blob_off;
+                F.src16 = (blob + (D.start_bit >> 3)) & ~15ull;
+                const unsigned long long end16 = (blob + ((D.end_bit + 7u) >> 3) + 15ull) & ~15ull;
+                F.ssz = ok ? static_cast<uint32_t>(end16 - F.src16) : 0u;
+            }
+            F.n_local = ok ? D.counts0 & 0xFFFFu : 0u;
+            F.n_tris = ok ? D.counts0 >> 16 : 0u;
+            F.n_strips = ok ? D.n_strips : 0u;
+            F.n_tok = F.n_tris + 2u * F.n_strips;
+            F.start_bit = D.start_bit;
+            F.end_bit = D.end_bit;
+            F.idsh = 9u - max(1u, 32u - __clz(F.n_local));
+            // odd strides (in words; the staged bytes in 16-byte units): lanes
+            // work at about the same offsets of their meshlets at the same time
+            F.axis_words = team_axis_words(F.n_local, sizeof(PlaneT<kWide>));
+            nb = F.ssz + ((F.ssz & 16u) ? 0u : 16u);
+            nw = team_walk_words(F.n_local);
+            nt = team_tok_words(F.n_tok);
+            na = team_asm_words(F.n_tris);
+            np = 3u * F.axis_words;
+        }
+        todo = __ballot_sync(kFull, ok);
+    }
+    for (;;) {  // rounds of as many meshlets as fit, in slot order (nearly always one)
+        if (warp == 0u) {
+            const bool in = (todo >> lane) & 1u;
+            uint32_t cb = in ? nb : 0u, cw = in ? nw : 0u, ct = in ? nt : 0u, ca = in ? na : 0u, cp = in ? np : 0u;
+#pragma unroll
+            for (uint32_t o = 1; o < M; o <<= 1) {
+                const uint32_t t0 = __shfl_up_sync(kFull, cb, o), t1 = __shfl_up_sync(kFull, cw, o);
+                const uint32_t t2 = __shfl_up_sync(kFull, ct, o), t3 = __shfl_up_sync(kFull, ca, o);
+                const uint32_t t4 = __shfl_up_sync(kFull, cp, o);
+                if (static_cast<uint32_t>(lane) >= o) {
+                    cb += t0;
+                    cw += t1;
+                    ct += t2;
+                    ca += t3;
+                    cp += t4;
+                }
+            }
+            // (six words: alignments)
+            const bool fit = in && team_bytes(cb, cw, ct, ca, cp) + 24u <= smem_bytes;
+            uint32_t rmask = __ballot_sync(kFull, fit);
+            const bool staged = rmask != 0u;
+            // one meshlet whose bytes exceed the stage: read in place
+            if (!staged && todo) rmask = 1u << (__ffs(todo) - 1);
+            todo &= ~rmask;
+            const int end = rmask ? 31 - __clz(rmask) : 0;  // the round's last meshlet
+            const uint32_t walk_base = staged ? __shfl_sync(kFull, cb, end) : 0u;
+            const uint32_t tw = staged ? __shfl_sync(kFull, cw, end) : 0u, tt = staged ? __shfl_sync(kFull, ct, end) : 0u;
+            // the words after the walks and after the records start on 16 bytes
+            const uint32_t uni_base = staged ? (walk_base + 4u * tw + 15u) & ~15u : 0u;
+            const uint32_t asm_base = (tt + 3u) & ~3u;
+            const bool mine = (rmask >> lane) & 1u;
+            if (mine) {
+                TeamFacts& F = s.f[lane];
+                F.bit_off = staged ? cb - nb : 0u;
+                F.walk_off = staged ? cw - nw : 0u;
+                F.tok_off = staged ? ct - nt : 0u;
+                F.asm_off = staged ? asm_base + ca - na : (nt + 3u) & ~3u;
+                F.plane_off = staged ? cp - np : 0u;
+                if (!staged) {
+                    s.walk_base = 0u;
+                    s.uni_base = (4u * nw + 15u) & ~15u;
+                }
+            }
+            if (lane == 0 && staged) {
+                s.walk_base = walk_base;
+                s.uni_base = uni_base;
+            }
+            if (lane == 0) {
+                s.rmask = rmask;
+                s.staged = staged ? 1u : 0u;
+            }
+        }
+        __syncthreads();
+        if (s.rmask == 0u) {  // CTA-uniform
+            // what follows this kernel on the stream must find the scan ended
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+            return;
+        }
+        if (s.staged) {
+            team_round<M, true, kWide>(a, s, smem, warp, lane);
+        } else {
+            team_round<M, false, kWide>(a, s, smem, warp, lane);
+        }
+    }
+}
+
+// Dynamic shared memory of a team CTA: room for M meshlets 2/5 above the
+// average of what is decoded (consecutive meshlets are about equally large);
+// a group that needs more goes in rounds.  Never less than one meshlet of the
+// largest size read in place.
+uint32_t team_smem(const DecodeArgs& a, uint32_t m, bool wide) {
+    const unsigned long long n = std::max<uint32_t>(1u, a.total_meshlets);
+    auto avg = [&](unsigned long long total, unsigned long long most) {
+        return static_cast<uint32_t>(std::min<unsigned long long>(total / n + 1ull, most)) * 7u / 5u;
+    };
+    const uint32_t size = wide ? 4u : 2u;
+    const uint32_t by = (avg(a.hint_bytes, 1024u) + 63u) & ~31u;
+    const uint32_t nv = std::min(avg(a.hint_v, 256u) + 4u, 256u), nt = std::min(avg(a.hint_t, 256u) + 8u, 256u);
+    const uint32_t b = team_bytes(m * by, m * team_walk_words(nv), m * team_tok_words(nt + nt / 12u),
+                                  m * team_asm_words(nt), m * 3u * team_axis_words(nv, size)) + 32u;
+    const uint32_t least = team_bytes(0u, team_walk_words(256u), team_tok_words(kTeamTokens), team_asm_words(256u),
+                                      3u * team_axis_words(256u, size)) + 32u;
+    return (std::max(b, least) + 15u) & ~15u;
+}
+
+template <uint32_t M, bool kWide>
+cudaError_t launch_team_m(const DecodeArgs& a, cudaStream_t s, bool after_scan) {
+    static size_t configured[64] = {0};
+    const uint32_t smem = team_smem(a, M, kWide);
+    cudaError_t e = opt_in_smem(team_kernel<M, kWide>, smem, configured);
+    if (e != cudaSuccess) return e;
+    const uint32_t grid = (a.total_meshlets + M - 1u) / M;
+    if (grid == 0u) return cudaSuccess;
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3(grid);
+    lc.blockDim = dim3(kTeamThreads);
+    lc.dynamicSmemBytes = smem;
+    lc.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = attr;
+    lc.numAttrs = after_scan ? 1 : 0;
+    e = cudaLaunchKernelEx(&lc, team_kernel<M, kWide>, a, smem);
+    note_launch(smem, grid);
+    return e;
+}
+
+}  // namespace
+
+cudaError_t launch_team(const DecodeArgs& a, const LaunchCfg& cfg, cudaStream_t s, bool after_scan) {
+    const bool w = a.wide_codes;
+    switch (team_meshlets(cfg)) {
+        case 4: return w ? launch_team_m<4, true>(a, s, after_scan) : launch_team_m<4, false>(a, s, after_scan);
+        case 8: return w ? launch_team_m<8, true>(a, s, after_scan) : launch_team_m<8, false>(a, s, after_scan);
+        default: return w ? launch_team_m<16, true>(a, s, after_scan) : launch_team_m<16, false>(a, s, after_scan);
+    }
+}
+
+}  // namespace stride
