@@ -152,6 +152,12 @@ int stride_info(const stride_handle* h, stride_info_t* info);
 int stride_decode(stride_handle* h, void* stream, uint32_t* d_idx, float* d_pos,
                   int32_t* d_codes);
 
+/* Normalised positions, the reference decode()'s (utils/paradelta_v5_cuda.py:
+ * 686-712), from the integer codes of a stride_decode of this handle:
+ * float32(g_min + q / (2^g_bits - 1) * g_range) evaluated in float64, n_v x 3
+ * floats.  Asynchronous on `stream`. */
+int stride_normalise_codes(const stride_handle* h, void* stream, const int32_t* d_codes, float* d_norm);
+
 /* Decode with host buffers: enqueue decode into handle-owned device outputs,
  * copy them to h_idx / h_pos (host, n_t*3 uint32 and n_v*3 float32) and
  * synchronise.  Returns the decode status.  The triangle copy starts when

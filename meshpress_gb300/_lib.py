@@ -99,6 +99,7 @@ SIGNATURES = [
     ("stride_reload", _I, [_P, _P, _SZ, _P]),
     ("stride_info", _I, [_P, ctypes.POINTER(StrideInfo)]),
     ("stride_decode", _I, [_P, _P, _P, _P, _P]),
+    ("stride_normalise_codes", _I, [_P, _P, _P, _P]),
     ("stride_decode_host", _I, [_P, _P, _P, _P]),
     ("stride_status", _I, [_P, _I, ctypes.POINTER(_U32)]),
     ("stride_decode_timed", _I, [_P, _P, _P, _P, _P]),

@@ -706,6 +706,19 @@ int stride_meshlet_bounds(stride_handle* h, void* stream, const float* d_pos, fl
     return r2 ? fail(r2, "meshlet bounds launch failed") : STRIDE_OK;
 }
 
+int stride_normalise_codes(const stride_handle* h, void* stream, const int32_t* d_codes, float* d_norm) {
+    if (!h || ((!d_codes || !d_norm) && h->params.n_v)) return fail(STRIDE_ERR_ARG, "null argument");
+    if ((reinterpret_cast<uintptr_t>(d_codes) & 3u) || (reinterpret_cast<uintptr_t>(d_norm) & 3u))
+        return fail(STRIDE_ERR_ARG, "codes and positions must be 4-byte aligned");
+    NormAxes c;
+    // placed by the identity: a centre of -0 leaves every value, a -0 too, as it is
+    for (int d = 0; d < 3; d++)
+        stride_dequant_setup(&c.d[d], -0.0f, 1.0f, static_cast<float>(h->params.dq[d].gmin),
+                             static_cast<float>(h->params.dq[d].grange), h->params.g_bits[d]);
+    const int rc = enqueue_normalise(d_codes, 3ull * h->params.n_v, c, d_norm, stream);
+    return rc ? fail(rc, "normalise launch failed") : STRIDE_OK;
+}
+
 int stride_cull_meshlets(const float* d_bounds, uint32_t n, const float* planes, void* stream, uint32_t* d_visible,
                          uint32_t* d_count) {
     if (!planes || !d_count || (n && (!d_bounds || !d_visible))) return fail(STRIDE_ERR_ARG, "null argument");

@@ -198,6 +198,12 @@ LaunchCfg default_config(uint32_t total_meshlets);
 struct Planes {
     float p[24];  // six planes (a, b, c, d): inside where a x + b y + c z + d >= 0
 };
+// Float32 of g_min + q / mx * g_range (float64, step by step) of n integer
+// codes, code i on axis i % 3.
+struct NormAxes {
+    stride_dequant_axis d[3];
+};
+int enqueue_normalise(const int32_t* codes, unsigned long long n, const NormAxes& axes, float* out, void* stream);
 int enqueue_meshlet_ranges(const MeshletDesc* descs, const BlockPrefix* bp, uint32_t n, unsigned long long* v_first,
                            unsigned long long* t_first, void* stream);
 int enqueue_meshlet_bounds(const MeshletDesc* descs, const BlockPrefix* bp, uint32_t n, const float* pos,

@@ -1408,6 +1408,32 @@ __global__ void meshlet_bounds_kernel(const MeshletDesc* __restrict__ descs, con
     if (lane < 6) bounds[6ull * m + lane] = lane < 3 ? lo[lane] : hi[lane - 3];
 }
 
+// Normalised positions from integer codes: value i is axis i % 3 of vertex
+// i / 3, as the float-float evaluation of stride_dequant.h (constants of an
+// identity placement).  Four values a thread, 16-byte loads and stores where
+// both arrays allow them; bound by memory (24 bytes a vertex).
+__device__ __forceinline__ float normalised_value(const NormAxes& c, unsigned long long i, int32_t q) {
+    const uint32_t d = static_cast<uint32_t>(i % 3ull);
+    const stride_dequant_axis* p = &c.d[d];
+    float y;
+    if (!p->zero_bits && stride_dequant_fast(p, static_cast<uint32_t>(q), &y)) return y;
+    return stride_dequant_exact(p, static_cast<uint32_t>(q));
+}
+
+__global__ void __launch_bounds__(256) normalise_kernel(const int32_t* __restrict__ codes, unsigned long long n,
+                                                        const __grid_constant__ NormAxes c, bool vec,
+                                                        float* __restrict__ out) {
+    const unsigned long long i0 = 4ull * (blockIdx.x * static_cast<unsigned long long>(blockDim.x) + threadIdx.x);
+    if (vec && i0 + 4ull <= n) {
+        const int4 q = __ldcg(reinterpret_cast<const int4*>(codes + i0));
+        *reinterpret_cast<float4*>(out + i0) =
+            make_float4(normalised_value(c, i0, q.x), normalised_value(c, i0 + 1ull, q.y),
+                        normalised_value(c, i0 + 2ull, q.z), normalised_value(c, i0 + 3ull, q.w));
+    } else {
+        for (unsigned long long i = i0; i < n && i < i0 + 4ull; i++) out[i] = normalised_value(c, i, __ldcg(codes + i));
+    }
+}
+
 // A box is culled when it lies wholly on the outer side of one plane: its
 // corner furthest along the plane normal (the p-vertex) has
 // a x + b y + c z + d < 0.  Evaluated left to right without contraction.
@@ -1447,6 +1473,16 @@ int enqueue_meshlet_bounds(const MeshletDesc* descs, const BlockPrefix* bp, uint
                            float* bounds, void* stream) {
     if (n == 0u) return STRIDE_OK;
     meshlet_bounds_kernel<<<(n + 7u) / 8u, 256, 0, static_cast<cudaStream_t>(stream)>>>(descs, bp, n, pos, bounds);
+    return cudaGetLastError() == cudaSuccess ? STRIDE_OK : STRIDE_ERR_CUDA;
+}
+
+int enqueue_normalise(const int32_t* codes, unsigned long long n, const NormAxes& axes, float* out, void* stream) {
+    if (n == 0ull) return STRIDE_OK;
+    const unsigned long long blocks = (n + 1023ull) / 1024ull;
+    if (blocks > 0x7FFFFFFFull) return STRIDE_ERR_UNSUPPORTED;
+    const bool vec = ((reinterpret_cast<uintptr_t>(codes) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0u;
+    normalise_kernel<<<static_cast<uint32_t>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(codes, n, axes, vec,
+                                                                                                    out);
     return cudaGetLastError() == cudaSuccess ? STRIDE_OK : STRIDE_ERR_CUDA;
 }
 

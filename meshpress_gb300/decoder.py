@@ -200,19 +200,17 @@ class ParaDeltaV5GpuDecoder:
             return verts, tris
         torch = _torch()
         tris, verts = self._outputs()
-        codes = torch.empty((self.n_v_total, 3), dtype=torch.int32, device=verts.device)
-        self.decode_into(tris, verts, codes=codes, stream=stream, check=check)
         s = stream if stream is not None else torch.cuda.current_stream()
-        with torch.cuda.stream(s):
-            vn = torch.empty((self.n_v_total, 3), dtype=torch.float64, device=verts.device)
-            for d in range(3):
-                gmin, grange, bits = float(self.info.g_min[d]), float(self.info.g_range[d]), int(self.g_bits[d])
-                if bits == 0:
-                    vn[:, d] = gmin
-                else:
-                    # one operation per step, in decode_dup's order, each rounded in float64
-                    vn[:, d] = (codes[:, d].double() / float((1 << bits) - 1)) * grange + gmin
-            self.d_verts_norm = vn.float()
+        with torch.cuda.stream(s):  # the codes live on the stream that uses them
+            codes = torch.empty((self.n_v_total, 3), dtype=torch.int32, device=verts.device)
+            vn = torch.empty((self.n_v_total, 3), dtype=torch.float32, device=verts.device)
+            self.decode_into(tris, verts, codes=codes, stream=s, check=False)
+            rc = self._lib.stride_normalise_codes(self._h, ctypes.c_void_p(_stream_handle(s)),
+                                                  ctypes.c_void_p(codes.data_ptr()), ctypes.c_void_p(vn.data_ptr()))
+            _lib.check(rc, "stride_normalise_codes")
+        if check:
+            self.check()
+        self.d_verts_norm = vn
         return self.d_verts_norm, tris.view(torch.int32)
 
     def decode_to_host(self, out=None, *, stream=None):
