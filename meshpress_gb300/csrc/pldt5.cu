@@ -6,9 +6,10 @@
 // Split as in the reference: the host parses the global header and the
 // boundary table (parse_globals_v5, :515-577) and reads every meshlet's
 // four-field header from the offset table (the reference's sizes kernel and
-// cumulative sums, :640-660); the device decodes the meshlets, one thread
-// each, into float64 normalised rows, and a second kernel turns the rows
-// into float32 world positions.
+// cumulative sums, :640-660); the device decodes the meshlets: the team kernel
+// from their bytes to float32 world positions in one launch, or, for streams
+// with a meshlet too large for it, the general kernel, one thread per meshlet,
+// into float64 normalised rows, which a second kernel turns into positions.
 //
 // Rows: the boundary vertices, then every meshlet's interior vertices in
 // meshlet order.  A meshlet's triangles go to its rows of the index output
@@ -26,6 +27,7 @@
 #include "stride_device.cuh"
 #include "stride_gb300.h"
 #include "stride_internal.h"
+#include "stride_team.cuh"
 
 namespace stride {
 namespace {
@@ -50,8 +52,16 @@ struct P5Args {
     uint32_t* walk;            // first-reach order per interior row: v | a << 8 | b << 16 | c << 24
     uint32_t* idx;             // output triangles (n_t x 3)
     double w0, w1, w2, delta;
+    double scale, center[3];   // to world positions
+    float* pos;                // output (n_rows x 3)
     Status* status;
 };
+
+// row -> f32(row * scale + center)
+__device__ __forceinline__ float p5_world(const P5Args& a, double x, uint32_t d) {
+    const double c = d == 0u ? a.center[0] : (d == 1u ? a.center[1] : a.center[2]);
+    return __double2float_rn(__dadd_rn(__dmul_rn(x, a.scale), c));
+}
 
 __device__ __forceinline__ void p5_report(Status* st, int code, uint32_t m) {
     const unsigned long long v = (static_cast<unsigned long long>(static_cast<unsigned>(code)) << 32) | m;
@@ -193,6 +203,7 @@ __device__ __forceinline__ unsigned long long p5_codeword(P5Bits& r, bool eg, in
 constexpr int kP5Threads = 64;     // meshlets (lanes) per block
 constexpr int kP5RefCache = 128;   // a lane's first boundary references kept in shared memory
 
+// The general kernel, for streams that the team kernel does not take (p5_plan).
 // One lane per meshlet, 32 meshlets per warp, every phase a loop that the
 // whole warp runs to its longest lane's count (no branch per token: the
 // lanes stay together), as in the DPR4 kernels:
@@ -448,14 +459,711 @@ __global__ void __launch_bounds__(kP5Threads) p5_decode_kernel(P5Args a) {
     }
 }
 
-// rows -> f32(row * scale + center)
-__global__ void p5_world_kernel(const double* __restrict__ rows, unsigned long long n, double scale, double c0,
-                                double c1, double c2, float* __restrict__ pos) {
+// ---- team kernel ------------------------------------------------------------
+// A CTA takes up to M consecutive meshlets from their bytes to world positions
+// in shared memory, as in stride_team.cu (whose parser, FIFO and assembly it
+// shares): only what is serial stays on one lane per meshlet.
+//
+//  1. stage    a warp per meshlet: its bytes into shared memory, in bit order;
+//              the parser warp then reads the boundary references.
+//  2. connect  parser, FIFO and eight assembler warps, a chunk behind one
+//              another; beside them the predictor warps sum the boundary rows
+//              (the roots' prediction).
+//  3. walk     a decoder lane per meshlet reads the three residual substreams
+//              one after the other; two warps behind it scale the residuals
+//              into their vertices' places; a predictor lane per (meshlet,
+//              axis) follows on the last axis, in float64 and the reference's
+//              operation order; three warps behind it put out float32 world
+//              positions.
+//
+// What bounds it are the chains: 2.5K cycles to stage, 4.5K for the references,
+// 31K for 280 tokens, 21K for the first two substreams of 120 residuals, 39K
+// for 120 float64 predictions (a 33 x 33 terrain).  The general kernel, whose
+// one lane has all of it, tokens one by one, takes ten times as long: 361 x 361
+// terrain, 1,295 meshlets, 715 us against 90.
+//
+// The host knows every meshlet's size, so each one has the same room, that of
+// the stream's largest.
+struct P5Team {
+    uint32_t bits;                  // staged bytes of a meshlet (odd in units of 16)
+    uint32_t axis;                  // doubles of an axis (odd)
+    uint32_t walk, tok, asm_w, tab;  // words: walk, token records, assembly, row table
+};
+
+constexpr int32_t kP5Zigzag = 1 << 30;  // in place of a minimum (16 bits): zigzag values
+constexpr uint32_t kP5Res = 16u;  // residuals between hand-overs from the decoder to the predictor warps
+constexpr uint32_t kP5MaxStage = 16384u;  // most staged bytes of a meshlet
+
+template <uint32_t M>
+__host__ __device__ constexpr uint32_t p5_pred_warps() {
+    return (3u * M + 31u) / 32u;
+}
+template <uint32_t M>
+__host__ __device__ constexpr uint32_t p5_team_threads() {
+    return 32u * (kTeamAsm + 2u + p5_pred_warps<M>());
+}
+// Shared memory: staged bytes, then (also where a corrupt lane's reads end)
+// walks and row tables, then the token records (read up to 31 past the last)
+// and the assembly, whose place the planes take when the walk starts.
+__host__ __device__ inline uint32_t p5_tables(const P5Team& t, uint32_t m) {  // bytes before that
+    return (m * (t.bits + 4u * (t.walk + t.tab)) + 15u) & ~15u;
+}
+__host__ __device__ inline uint32_t p5_records(const P5Team& t, uint32_t m) {  // their words
+    return (m * t.tok + 3u) & ~3u;
+}
+inline uint32_t p5_team_bytes(const P5Team& t, uint32_t m) {
+    const uint32_t both = std::max(24u * m * t.axis, 4u * (p5_records(t, m) + m * t.asm_w));
+    return (std::max(p5_tables(t, m) + both, m * t.bits + kTeamSlack) + 15u) & ~15u;
+}
+
+struct P5Facts : TeamSize {
+    unsigned long long row0, tri0;
+    uint32_t m, n_bnd, n_int, n_strips;
+    uint32_t at, end;    // bits of the staged words: after the header, the meshlet's end
+    uint32_t conn;       // where the connectivity starts
+    uint32_t anchor;     // ... and ends
+    uint32_t n_walk;
+    uint32_t bad;
+    int32_t mn[3];       // a fixed-width substream's minimum, or kP5Zigzag
+};
+
+template <uint32_t M>
+struct P5Shared {
+    uint4 masks[17];
+    P5Facts f[M];
+    // parser steps of three chunks (being written; with the FIFO; with the assemblers)
+    union {
+        struct {
+            uint32_t x[3][kTeamSteps * M];
+            uint32_t step[3][kTeamSteps * M];
+        };
+        unsigned long long res[2][kP5Res * M];  // in the walk: codeword values of two chunks
+    };
+    uint8_t meta[3][kTeamSteps * M];
+    double mean[3 * M];  // the roots' prediction, by (axis, meshlet)
+    uint32_t more[2];  // the parser has tokens left after its last chunk
+    uint32_t rmask;    // meshlets to decode
+    uint32_t redo;     // decode the connectivity again, with the exact FIFO
+};
+
+// One codeword from bit `pos` of staged words, of any length below `limit`
+// (the general reader, for the codewords longer than a window).
+__device__ __noinline__ bool p5_long(const uint32_t* w, uint32_t& pos, uint32_t tag, uint32_t k, uint32_t limit,
+                                     unsigned long long& u) {
+    uint32_t q = 0u;
+    if (tag != 0u) {
+        for (;;) {
+            if (pos >= limit) return false;
+            const uint32_t x = peek32<true>(w, pos);
+            const uint32_t z = static_cast<uint32_t>(__clz(x));
+            q += z;
+            pos += z;
+            if (x) break;
+        }
+        pos++;
+        if (tag == 2u && q > 32u) return false;  // (see P5Bits::eg)
+    }
+    auto take = [&](uint32_t n) -> uint32_t {
+        if (n == 0u) return 0u;
+        const uint32_t v = peek32<true>(w, pos) >> (32u - n);
+        pos += n;
+        return v;
+    };
+    unsigned long long head = q;
+    if (tag == 2u) {
+        if (pos + q > limit) return false;
+        head = ((1ull << q) - 1ull) + take(q);
+    }
+    if (pos + k > limit) return false;
+    const uint32_t low = take(k);
+    u = (head << k) + low;
+    return true;
+}
+
+// Four codewords of a substream (tag 0: fixed width k) from bit `pos` of the
+// words at shared address `base`, the first n of them, as values into u.
+// `far` when one is longer than 32 bits or starts beyond the window, or a fixed
+// width is above 30: its lane then takes them again by the general reader.
+// Bound by the chain from one codeword to the next: a 96-bit window read once
+// for four leaves on it the leading zeros, a multiply-add and a funnel shift
+// (45 cycles a codeword on one warp; with a window refilled at each one, 100).
+__device__ __forceinline__ bool p5_four(uint32_t base, uint32_t& pos, uint32_t tag, uint32_t k, int n, uint32_t (&u)[4]) {
+    const uint32_t em = tag, k1 = tag ? k + 1u : k, pow = tag ? 1u << (k & 31u) : 0u;
+    const uint32_t zmul = tag == 1u ? pow : 0u, most = tag ? 32u : 30u;
+    const uint32_t a = mad_u32(pos >> 5, 4u, base), o = pos & 31u;
+    uint32_t w0, w1, w2, w3;
+    asm("ld.shared.u32 %0, [%1];" : "=r"(w0) : "r"(a));
+    asm("ld.shared.u32 %0, [%1+4];" : "=r"(w1) : "r"(a));
+    asm("ld.shared.u32 %0, [%1+8];" : "=r"(w2) : "r"(a));
+    asm("ld.shared.u32 %0, [%1+12];" : "=r"(w3) : "r"(a));
+    uint32_t hi = __funnelshift_l(w1, w0, o), mid = __funnelshift_l(w2, w1, o), lo = __funnelshift_l(w3, w2, o);
+    uint32_t used = 0u, longest = 0u, before = 0u;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const uint32_t len = __clz(hi) * em + k1;
+        // with the terminator as the value bits' leading one: 2^nb + value
+        u[i] = __clz(hi) * zmul + (__funnelshift_rc(hi, 0u, 32u - len) - pow);
+        const uint32_t take = i < n ? len : 0u;
+        longest = max(longest, take);
+        before = used;
+        used += take;
+        hi = __funnelshift_lc(mid, hi, take);
+        mid = __funnelshift_lc(lo, mid, take);
+        lo = __funnelshift_lc(0u, lo, take);
+    }
+    pos += used;
+    return (longest > most) | (before > 64u);
+}
+
+// A double from 32 bits by integer instructions: a float64 instruction takes a
+// warp 64 cycles, a conversion 100.
+__device__ __forceinline__ double p5_double(uint32_t q) {
+    const uint32_t neg = sign_mask(q), u = (q ^ neg) - neg;
+    const uint32_t z = __clz(u), m = __funnelshift_lc(0u, u, z);  // leading one on top
+    const uint32_t top = u ? (neg & 0x80000000u) + ((1053u - z) << 20) + (m >> 11) : 0u;
+    return __hiloint2double(static_cast<int>(top), static_cast<int>(m << 21));
+}
+
+__device__ __forceinline__ double ld_shared_f64(uint32_t a) {
+    double x;
+    asm volatile("ld.shared.f64 %0, [%1];" : "=d"(x) : "r"(a) : "memory");
+    return x;
+}
+
+// Predictions of parallelogram entries of the walk, [h, h + 8) below n_walk, in
+// the reference's order and without contraction (encoder/paradelta_v5.py:
+// 426-445); a vertex's scaled residual is in its place of the plane, where the
+// roots' rows are already.  Bound by the chain of float64 instructions, 64
+// cycles each whatever their lanes: three an entry with the canonical weights
+// 1, 1, -1 (kUnit: their products are exact), six with others.  Addresses are
+// formed for all eight first, and no select is on the chain (one on a float64
+// result costs it 50 cycles; rows through shared memory, 35): 256 cycles an
+// entry on one warp, 342 with the last row kept in registers and the roots here.
+template <bool kUnit>
+__device__ __forceinline__ void p5_predict(uint32_t plane, const uint32_t* __restrict__ walk, uint32_t h, uint32_t n_walk,
+                                           double w0, double w1, double w2) {
+    uint32_t av[8], aa[8], ab[8], ac[8];
+    double r[8];
+#pragma unroll
+    for (uint32_t i = 0; i < 8u; i++) {
+        const uint32_t e = h + i < n_walk ? walk[h + i] : 0u;
+        av[i] = mad_u32(__byte_perm(e, 0u, 0x4440u), 8u, plane);
+        aa[i] = mad_u32(__byte_perm(e, 0u, 0x4441u), 8u, plane);
+        ab[i] = mad_u32(__byte_perm(e, 0u, 0x4442u), 8u, plane);
+        ac[i] = mad_u32(e >> 24, 8u, plane);
+        r[i] = ld_shared_f64(av[i]);
+    }
+#pragma unroll
+    for (uint32_t i = 0; i < 8u; i++) {
+        const double a = ld_shared_f64(aa[i]), b = ld_shared_f64(ab[i]), c = ld_shared_f64(ac[i]);
+        const double p = kUnit ? __dadd_rn(__dadd_rn(a, b), -c)
+                               : __dadd_rn(__dadd_rn(__dmul_rn(w0, a), __dmul_rn(w1, b)), __dmul_rn(w2, c));
+        const double x = __dadd_rn(p, r[i]);
+        // roots, and entries past the end, are (v, v, v, v)
+        asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %0, %2;\n@p st.shared.f64 [%0], %1;\n}" ::"r"(av[i]), "d"(x), "r"(aa[i])
+                     : "memory");
+    }
+}
+
+template <uint32_t M>
+__global__ void __launch_bounds__(p5_team_threads<M>(), 2) p5_team_kernel(P5Args a, P5Team L) {
+    constexpr uint32_t kThreads = p5_team_threads<M>(), kPred = p5_pred_warps<M>();
+    constexpr uint32_t kPer = (M + kTeamAsm - 1u) / kTeamAsm;  // meshlets of an assembler warp
+    extern __shared__ __align__(128) uint8_t smem[];
+    __shared__ P5Shared<M> s;
+    const uint32_t warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    const bool predictor = warp >= kTeamAsm + 2u;
+    const bool assembler = warp != kTeamParser && warp != kTeamFifo && !predictor;
+    const uint32_t aw0 = team_asm_index(warp);  // an assembler's first meshlet
+    const uint32_t n_here = min(M, a.n_meshlets - blockIdx.x * M);
+    const uint32_t* words = reinterpret_cast<const uint32_t*>(smem);
+    uint32_t* walks = reinterpret_cast<uint32_t*>(smem + M * L.bits);
+    uint32_t* tabs = walks + M * L.walk;
+    double* planes = reinterpret_cast<double*>(smem + p5_tables(L, M));
+    uint32_t* toks = reinterpret_cast<uint32_t*>(planes);
+    uint32_t* asms = toks + p5_records(L, M);
+    // 1. stage; facts of the meshlets
+    if (threadIdx.x < 17u) s.masks[threadIdx.x] = threadIdx.x < 16u ? mtf_mask_row(threadIdx.x) : make_uint4(0u, 0u, 0u, 0u);
+    if (assembler) {
+        for (uint32_t j = aw0; j < n_here; j += kTeamAsm) {
+            const uint32_t m = blockIdx.x * M + j;
+            const uint32_t s0 = __ldcg(a.start + m), s1 = __ldcg(a.start + m + 1u);
+            const uint32_t from = (s0 >> 3) & ~15u;  // the first byte staged
+            const uint32_t n16 = (((s1 - 8u * from) + 127u) >> 7);
+            const uint4* src = reinterpret_cast<const uint4*>(a.blob + from);
+            uint4* dst = reinterpret_cast<uint4*>(smem + j * L.bits);
+            for (uint32_t i = lane; i < n16; i += 32u) {
+                uint4 q = __ldcg(src + i);
+                q.x = bswap32(q.x);
+                q.y = bswap32(q.y);
+                q.z = bswap32(q.z);
+                q.w = bswap32(q.w);
+                dst[i] = q;
+            }
+            // the header (:350-353), inside the stream as the host has checked, may end past the meshlet
+            const uint32_t* g = reinterpret_cast<const uint32_t*>(a.blob) + (s0 >> 5);
+            const uint32_t x = bswap32(__ldcg(g)), y = bswap32(__ldcg(g + 1)), z = bswap32(__ldcg(g + 2));
+            const uint32_t h0 = __funnelshift_l(y, x, s0 & 31u), h1 = __funnelshift_l(z, y, s0 & 31u);
+            P5Facts& F = s.f[j];
+            const unsigned long long row0 = __ldcg(a.row_base + m), tri0 = __ldcg(a.tri_base + m);
+            const uint32_t n_bnd = h0 >> 16, n_int = h0 & 0xFFFFu;
+            if (lane == 0) {
+                F.m = m;
+                F.n_bnd = n_bnd;
+                F.n_int = n_int;
+                F.n_local = n_bnd + n_int;
+                F.n_tris = h1 >> 16;
+                F.n_strips = h1 & 0xFFFFu;
+                F.n_tok = F.n_tris + 2u * F.n_strips;
+                F.idsh = 9u - max(1u, 32u - __clz(F.n_local));
+                F.row0 = row0;
+                F.tri0 = tri0;
+                F.end = s1 - 8u * from + 8u * j * L.bits;
+                F.at = s0 + 64u - 8u * from + 8u * j * L.bits;
+            }
+            // rows of the interior vertices
+            for (uint32_t i = lane; i < n_int; i += 32u) tabs[j * L.tab + n_bnd + i] = static_cast<uint32_t>(row0) + i;
+        }
+    }
+    __syncthreads();
+    // boundary references: the first in 32 bits, then Rice codewords of the
+    // differences less one (:354-361); rows of the boundary table
+    if (warp == kTeamParser) {
+        const bool act = static_cast<uint32_t>(lane) < n_here;
+        P5Facts& F = s.f[act ? lane : 0];
+        const uint32_t n = act ? F.n_bnd : 0u;
+        uint32_t* tab = tabs + (act ? lane : 0) * L.tab;
+        bool bad = act && (F.n_strips > F.n_tris || F.at > F.end);  // every strip emits a triangle
+        const uint32_t limit = act ? F.end : 0u;
+        const uint32_t base = smem_addr(words);
+        uint32_t pos = act ? min(F.at, F.end) : 0u;
+        unsigned long long prev = peek_shared(base, pos);
+        pos += n > 0u ? 32u : 0u;
+        uint32_t k = n > 1u ? peek_shared(base, pos) >> 24 : 0u;
+        pos += n > 1u ? 8u : 0u;
+        bad = bad || k > static_cast<uint32_t>(kP5MaxK) || pos > limit;
+        if (n > 0u && !bad) {
+            tab[0] = static_cast<uint32_t>(prev);
+            bad = prev >= a.n_boundary;
+        }
+        k = bad ? 0u : k;
+        const uint32_t most = __reduce_max_sync(kFull, bad ? 0u : n);
+#pragma unroll 1
+        for (uint32_t i0 = 1u; i0 < most; i0 += 8u) {
+            const int left = bad ? 0 : static_cast<int>(n) - static_cast<int>(i0);
+            uint32_t u[8], at = pos;
+            bool far = false;
+#pragma unroll
+            for (int h = 0; h < 8; h += 4)
+                far = p5_four(base, pos, 1u, k, left - h, *reinterpret_cast<uint32_t(*)[4]>(u + h)) | far;
+            if (far) {
+                for (int i = 0; i < 8; i++) {
+                    if (i >= left || bad) continue;
+                    unsigned long long v = 0ull;
+                    if (!p5_long(words, at, 1u, k, limit, v) || v >= a.n_boundary) bad = true;
+                    u[i] = static_cast<uint32_t>(v);
+                }
+                pos = at;
+            }
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                prev += i < left ? u[i] + 1ull : 0ull;
+                if (i < left) tab[i0 + i] = static_cast<uint32_t>(prev);
+            }
+            bad = bad || (left > 0 && (pos > limit || prev >= a.n_boundary));
+            pos = min(pos, limit);
+            __syncwarp();
+        }
+        if (act) F.conn = pos;
+        if (bad) p5_report(a.status, kErrCorrupt, F.m);
+        const uint32_t mask = __ballot_sync(kFull, act && !bad);
+        if (lane == 0) s.rmask = mask;
+    } else {
+        // meanwhile the others: this CTA's share of the boundary rows' positions
+        const uint32_t t = threadIdx.x < 32u * kTeamParser ? threadIdx.x : threadIdx.x - 32u;
+        const unsigned long long all = static_cast<unsigned long long>(gridDim.x) * (kThreads - 32u);
+        for (unsigned long long e = static_cast<unsigned long long>(blockIdx.x) * (kThreads - 32u) + t;
+             e < 3ull * a.n_boundary; e += all)
+            a.pos[e] = p5_world(a, __ldcg(a.rows + e), static_cast<uint32_t>(e % 3ull));
+    }
+    __syncthreads();
+    const uint32_t rmask = s.rmask;
+    // a predictor's (meshlet, axis)
+    const uint32_t pid = (warp - kTeamAsm - 2u) * 32u + lane;
+    const uint32_t pj = pid % M, pd = pid / M < 3u ? pid / M : 2u;
+    const bool pon = predictor && pid < 3u * M && ((rmask >> pj) & 1u);
+    double* pplane = planes + (pon ? (pj * 3u + pd) * L.axis : 0u);
+    // 2. connectivity, in step: chunk c with the parser, c - 1 with the FIFO
+    // warp, c - 2 with the assemblers
+    for (uint32_t pass = 0; pass < 2u; pass++) {  // the second one with the exact FIFO, rarely
+        const bool exact = pass != 0u;
+        if (threadIdx.x == 0) s.redo = 0u;
+        if (threadIdx.x < M) s.f[threadIdx.x].bad = 0u;
+        __syncthreads();
+        if (predictor) {
+            // the roots' prediction: the mean of the boundary rows, summed in
+            // order (:362-365)
+            const uint32_t n = pon && !exact ? s.f[pj].n_bnd : 0u;
+            const uint32_t most = __reduce_max_sync(kFull, n);
+            const uint32_t* tab = tabs + (pon ? pj : 0u) * L.tab;
+            double mean = 0.0;
+            uint32_t at = 0u;
+            auto sum = [&](uint32_t upto) {
+                for (; at < upto; at += 8u) {
+                    double r[8];
+#pragma unroll
+                    for (uint32_t i = 0; i < 8u; i++) r[i] = at + i < n ? __ldcg(a.rows + 3ull * tab[at + i] + pd) : 0.0;
+                    if (at == 0u) mean = n ? -0.0 : 0.0;  // the first sum is the first row
+#pragma unroll
+                    for (uint32_t i = 0; i < 8u; i++)
+                        if (at + i < n) mean = __dadd_rn(mean, r[i]);
+                }
+            };
+            bool more = true;
+            for (uint32_t c = 0;; c++) {
+                sum(min(at + 16u, most));
+                team_all_bar<kThreads>();
+                if (!more) break;
+                more = s.more[c & 1u] != 0u;
+            }
+            sum(most);
+            if (n) mean = __ddiv_rn(mean, static_cast<double>(n));
+            if (pon && !exact) s.mean[pid] = mean;
+            if (exact) {
+                team_all_bar<kThreads>();
+                team_all_bar<kThreads>();
+            }
+        } else if (!assembler) {
+            const bool act = (rmask >> lane) & 1u;
+            P5Facts& F = s.f[act ? lane : 0];
+            const uint32_t n_tok = act ? F.n_tok : 0u;
+            const uint32_t sl = act ? lane : 0u;  // an idle lane repeats the first one's steps
+            const uint32_t ib = act ? 9u - F.idsh : 1u;
+            uint16_t* row = reinterpret_cast<uint16_t*>(toks + sl * L.tok) + 2;
+            TeamParse T;
+            MtfFifo fifo;
+            uint32_t t = 0u;
+            uint32_t past = 0u;  // negative: a FIFO index named no entry
+            T.strips = F.n_strips;
+            T.pos = act ? F.conn : 0u;
+            fifo.f0 = fifo.f1 = fifo.f2 = fifo.f3 = 0xFFFFFFFFu;
+            if (warp == kTeamParser && act) row[-2] = row[-1] = 0;
+            bool more = true;
+            for (uint32_t c = 0;; c++) {
+                if (warp == kTeamParser) {
+                    const uint32_t b = c % 3u;
+                    if (act) team_parse<true, M>(T, words, n_tok, ib, 0u, s.x[b] + lane, s.meta[b] + lane);
+                    __syncwarp();
+                    const bool m = __any_sync(kFull, T.t < n_tok);
+                    if (lane == 0) s.more[c & 1u] = m ? 1u : 0u;
+                } else if (c > 0u) {
+                    const uint32_t b = (c - 1u) % 3u;
+                    if (act) team_fifo<M>(fifo, t, s.x[b] + sl, s.meta[b] + sl, s.step[b] + sl, ib, s.masks, past);
+                }
+                __syncwarp();
+                team_all_bar<kThreads>();
+                if (!more) break;  // this was the chunk after the parser's last
+                more = s.more[c & 1u] != 0u;
+            }
+            if (act && warp == kTeamParser) {
+                F.anchor = T.pos;
+                // every strip read, inside the meshlet
+                if (T.t != n_tok || T.strips != 0u || T.left != 0u || T.pos > F.end) atomicOr(&F.bad, 1u);
+            }
+            if (exact) team_all_bar<kThreads>();  // the records are there
+            if (act && warp == kTeamFifo) {
+                if (exact ? !team_fifo_exact(row, n_tok, F.idsh, s.masks) : sign_mask(past) != 0u) atomicOr(&F.bad, 1u);
+            }
+            __syncwarp();
+            if (exact) team_all_bar<kThreads>();
+        } else {
+            TeamAsm S[kPer];
+            auto mine = [&](uint32_t q) { return aw0 + q * kTeamAsm < M && ((rmask >> (aw0 + q * kTeamAsm)) & 1u); };
+            // the windows that the records fill (or end)
+            auto windows = [&](TeamAsm& A, uint32_t j) {
+                const P5Facts& F = s.f[j];
+                uint32_t* last = asms + j * L.asm_w;
+                const uint32_t have = A.t >= F.n_tok ? F.n_tok + 31u : A.t;
+                for (; A.t0 + 32u <= have; A.t0 += 32u)
+                    team_window<false>(A, F, F.n_bnd, exact, A.t0, reinterpret_cast<const uint16_t*>(toks + j * L.tok) + 2,
+                                       walks + j * L.walk, nullptr, last, last + 256, lane);
+            };
+            auto chunk = [&](uint32_t c) {
+#pragma unroll
+                for (uint32_t q = 0; q < kPer; q++) {
+                    const uint32_t j = aw0 + q * kTeamAsm;
+                    if (!mine(q) || S[q].t >= s.f[j].n_tok) continue;  // warp-uniform, here and below
+                    team_records<M>(S[q], s.f[j], exact, reinterpret_cast<uint16_t*>(toks + j * L.tok) + 2,
+                                    s.x[c % 3u] + j, s.step[c % 3u] + j, lane);
+                    if (!exact) windows(S[q], j);
+                }
+            };
+#pragma unroll
+            for (uint32_t q = 0; q < kPer; q++) {
+                const uint32_t j = aw0 + q * kTeamAsm;
+                if (!mine(q)) continue;
+                uint4* last = reinterpret_cast<uint4*>(asms + j * L.asm_w);
+                last[lane] = last[lane + 32] = make_uint4(0u, 0u, 0u, 0u);
+            }
+            __syncwarp();
+            bool more = true;
+            uint32_t c = 0u;
+            for (;; c++) {
+                if (c > 1u) chunk(c - 2u);
+                team_all_bar<kThreads>();
+                if (!more) break;
+                more = s.more[c & 1u] != 0u;
+            }
+            chunk(c - 1u);  // the parser's last chunk
+            if (exact) {
+                __syncwarp();
+                team_all_bar<kThreads>();
+                team_all_bar<kThreads>();  // the FIFO warp has resolved the records
+#pragma unroll
+                for (uint32_t q = 0; q < kPer; q++)
+                    if (mine(q)) windows(S[q], aw0 + q * kTeamAsm);
+            }
+#pragma unroll
+            for (uint32_t q = 0; q < kPer; q++) {
+                const uint32_t j = aw0 + q * kTeamAsm;
+                if (!mine(q)) continue;
+                P5Facts& F = s.f[j];
+                const uint32_t* tab = tabs + j * L.tab;
+                // ids of a valid meshlet lie in the table; an invalid one's are cut to it
+                const uint32_t vmax = F.n_local ? F.n_local - 1u : 0u;
+                uint32_t* out = a.idx + 3ull * F.tri0;
+                const uint32_t ph = (0u - static_cast<uint32_t>(reinterpret_cast<uintptr_t>(out) >> 2)) & 3u;
+                team_triangles(out, asms + j * L.asm_w + 256, ph, min(S[q].tcnt, F.n_tris),
+                               [&](uint32_t v) { return tab[min(v, vmax)]; }, lane);
+                const bool bad = __any_sync(kFull, S[q].out) || S[q].tcnt != F.n_tris;
+                if (lane == 0) {
+                    F.n_walk = min(S[q].wcnt, F.n_int);
+                    if (bad || S[q].wcnt > F.n_int) atomicOr(&F.bad, 1u);
+                    if (S[q].redo && !exact) s.redo = 1u;
+                }
+            }
+        }
+        __syncthreads();
+        if (s.redo == 0u || exact) break;
+        __syncthreads();  // everyone has read it
+    }
+    // 3. walk, in step: chunk g with the decoder, g - 1 with the warps that
+    // put its residuals, scaled, and the roots' rows into the plane, and of
+    // the last axis g - 2 with the predictors and g - 3 with the warps that put
+    // positions out (on schedulers that the predictors do not use).
+    constexpr uint32_t kScalers = 2u, kEmitters = 3u;
+    const uint32_t scaler = warp == 1u ? 0u : (warp == 4u ? 1u : kScalers);
+    const uint32_t emitter = warp == 5u ? 0u : (warp == 8u || warp == 9u ? warp - 7u : kEmitters);
+    const bool lon = static_cast<uint32_t>(lane) < M && ((rmask >> lane) & 1u) && s.f[lane].bad == 0u;
+    const uint32_t on_mask = __ballot_sync(kFull, lon);
+    if (warp == 0u || scaler < kScalers || predictor || emitter < kEmitters) {
+        constexpr uint32_t kBar = 32u * (1u + kScalers + kPred + kEmitters);
+        auto bar = [&]() { asm volatile("bar.sync 1, %0;" ::"n"(kBar) : "memory"); };
+        const uint32_t chunks = (__reduce_max_sync(kFull, lon ? s.f[lane].n_int : 0u) + kP5Res - 1u) / kP5Res;
+        const uint32_t steps = 3u * chunks + 3u;
+        if (predictor) {
+            const bool on = pon && ((on_mask >> pj) & 1u);
+            const P5Facts& F = s.f[on ? pj : 0u];
+            const uint32_t n_walk = on ? F.n_walk : 0u;
+            if (on && n_walk < F.n_int)  // vertices that the walk never reaches keep row 0
+                for (uint32_t i = 0; i < F.n_int; i++) pplane[F.n_bnd + i] = 0.0;
+            __syncwarp();
+            bar();
+            const uint32_t* walk = walks + (on ? pj : 0u) * L.walk;
+            const uint32_t plane_addr = smem_addr(pplane);
+            const bool unit = a.w0 == 1.0 && a.w1 == 1.0 && a.w2 == -1.0;
+            for (uint32_t g = 0; g < steps; g++) {
+                if (g >= 2u * chunks + 2u && g < 3u * chunks + 2u) {
+                    const uint32_t h0 = (g - 2u - 2u * chunks) * kP5Res;
+#pragma unroll 1
+                    for (uint32_t h = h0; h < h0 + kP5Res; h += 8u) {
+                        if (unit) {
+                            p5_predict<true>(plane_addr, walk, h, n_walk, a.w0, a.w1, a.w2);
+                        } else {
+                            p5_predict<false>(plane_addr, walk, h, n_walk, a.w0, a.w1, a.w2);
+                        }
+                    }
+                }
+                __syncwarp();
+                bar();
+            }
+        } else if (scaler < kScalers) {
+            bar();
+            uint32_t d = 0u, c = 0u;
+            for (uint32_t g = 0; g < steps; g++) {
+                if (g > 0u && g <= 3u * chunks) {
+                    constexpr uint32_t kIts = M * kP5Res / 64u;
+                    double* slot[kIts];
+                    double x[kIts], mean[kIts];
+                    long long r[kIts];
+                    bool in[kIts], wide = false;
+#pragma unroll
+                    for (uint32_t q = 0; q < kIts; q++) {
+                        const uint32_t it = 64u * q + 32u * scaler + lane, j = it % M, i = c * kP5Res + it / M;
+                        in[q] = ((on_mask >> j) & 1u) && i < s.f[j].n_walk;
+                        const int32_t mn = s.f[j].mn[d];
+                        const unsigned long long u = s.res[(g - 1u) & 1u][it];
+                        r[q] = mn == kP5Zigzag ? unzig(u) : mn + static_cast<long long>(u);
+                        const uint32_t e = walks[j * L.walk + (in[q] ? i : 0u)], v = e & 0xFFu;
+                        // roots are (v, v, v, v); a residual that is added to nothing is added to -0
+                        mean[q] = v == ((e >> 8) & 0xFFu) ? s.mean[d * M + j] : -0.0;
+                        slot[q] = planes + (3u * j + d) * L.axis + v;
+                        x[q] = p5_double(static_cast<uint32_t>(r[q]));
+                        wide = wide | (r[q] != static_cast<int32_t>(r[q]));
+                    }
+                    if (__any_sync(kFull, wide)) {
+#pragma unroll
+                        for (uint32_t q = 0; q < kIts; q++) x[q] = static_cast<double>(r[q]);
+                    }
+#pragma unroll
+                    for (uint32_t q = 0; q < kIts; q++) {
+                        x[q] = __dadd_rn(mean[q], __dmul_rn(x[q], a.delta));
+                        if (in[q]) *slot[q] = x[q];
+                    }
+                    c++;
+                    if (c == chunks) c = 0u, d++;
+                }
+                __syncwarp();
+                bar();
+            }
+        } else if (warp == 0u) {
+            // (lanes from M on repeat the first M)
+            const uint32_t j = lane % M;
+            const bool on = (on_mask >> j) & 1u;
+            P5Facts& F = s.f[on ? j : 0u];
+            const uint32_t n = on ? F.n_int : 0u;
+            const uint32_t limit = on ? F.end : 0u;
+            const uint32_t base = smem_addr(words);
+            uint32_t pos = on ? F.anchor : 0u;
+            bool bad = false;
+            bar();
+            uint32_t g = 0u;
+#pragma unroll 1
+            for (uint32_t d = 0; d < 3u; d++) {
+                // tag, then fixed width (tag 0: minimum and width) or Rice /
+                // Exp-Golomb (tags 1, 2: k) (:403-424)
+                uint32_t tag = 1u, k = 0u;
+                if (n) {
+                    const uint32_t x = peek_shared(base, pos), y = peek_shared(base, pos + 24u);
+                    tag = x >> 24;
+                    k = tag ? (x >> 16) & 0xFFu : y >> 24;
+                    F.mn[d] = tag ? kP5Zigzag : static_cast<int32_t>(x << 8) >> 16;
+                    pos += tag ? 16u : 32u;
+                    bad = bad || tag > 2u || k > static_cast<uint32_t>(tag ? kP5MaxK : kP5MaxWidth);
+                    tag = bad ? 1u : tag;
+                    k = bad ? 0u : k;
+                }
+                __syncwarp();
+#pragma unroll 1
+                for (uint32_t c = 0; c < chunks; c++, g++) {
+                    unsigned long long* res = s.res[g & 1u] + j;
+                    const int left = bad ? 0 : static_cast<int>(n) - static_cast<int>(c * kP5Res);
+                    uint32_t at = pos;
+                    bool far = false;
+#pragma unroll
+                    for (uint32_t h = 0; h < kP5Res; h += 4u) {
+                        uint32_t u[4];
+                        far = p5_four(base, pos, tag, k, left - static_cast<int>(h), u) | far;
+                        pos = min(pos, limit + 128u);  // inside what a corrupt lane may read
+#pragma unroll
+                        for (uint32_t i = 0; i < 4u; i++) res[(h + i) * M] = u[i];
+                    }
+                    if (far) {
+                        for (int i = 0; i < static_cast<int>(kP5Res); i++) {
+                            unsigned long long v = 0ull;
+                            if (i < left && !bad) bad = !p5_long(words, at, tag, k, limit, v);
+                            res[i * M] = v;
+                        }
+                        pos = at;
+                    }
+                    bad = bad || pos > limit;
+                    pos = min(pos, limit);
+                    __syncwarp();
+                    bar();
+                }
+            }
+            // meshlets lie back to back, as the CPU decoder reads them
+            const bool last = F.m + 1u == a.n_meshlets;
+            if (on && (bad || (!last && pos != limit))) F.bad = 1u;
+            bar();
+            bar();
+            bar();
+        } else {
+            // f32(row * scale + center)
+            bar();
+            // first, the boundary rows into the planes
+            for (uint32_t j = 0; j < n_here; j++) {
+                if (!((on_mask >> j) & 1u)) continue;
+                const uint32_t n3 = 3u * s.f[j].n_bnd;
+                for (uint32_t e = 32u * emitter + lane; e < n3; e += 32u * kEmitters) {
+                    const uint32_t i = e / 3u, d = e - 3u * i;
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(planes + (3u * j + d) * L.axis + i)),
+                                 "l"(a.rows + 3ull * tabs[j * L.tab + i] + d)
+                                 : "memory");
+                }
+            }
+            cp_async_commit();
+            for (uint32_t g = 0; g < steps; g++) {
+                if (g == 2u * chunks + 1u) cp_async_wait_all();
+                if (g >= 2u * chunks + 3u) {
+                    const uint32_t c = g - 3u - 2u * chunks;
+#pragma unroll 2
+                    for (uint32_t it = 32u * emitter + lane; it < 3u * M * kP5Res; it += 32u * kEmitters) {
+                        const uint32_t d = it % 3u, j = it / (3u * kP5Res), i = c * kP5Res + it / 3u % kP5Res;
+                        const P5Facts& F = s.f[j];
+                        if (!((on_mask >> j) & 1u) || i >= F.n_walk) continue;
+                        const uint32_t v = walks[j * L.walk + i] & 0xFFu;
+                        a.pos[3ull * (F.row0 + (v - F.n_bnd)) + d] = p5_world(a, planes[(3u * j + d) * L.axis + v], d);
+                    }
+                }
+                __syncwarp();
+                bar();
+            }
+        }
+    }
+    __syncthreads();
+    // invalid meshlets, and those with vertices that the walk never reaches
+    if (assembler) {
+        for (uint32_t j = aw0; j < n_here; j += kTeamAsm) {
+            if (!((rmask >> j) & 1u)) continue;
+            const P5Facts& F = s.f[j];
+            if (F.bad) {
+                if (lane == 0) p5_report(a.status, kErrCorrupt, F.m);
+            } else if (F.n_walk < F.n_int) {
+                for (uint32_t e = lane; e < 3u * F.n_int; e += 32u) {
+                    const uint32_t i = e / 3u, d = e - 3u * i;
+                    a.pos[3ull * F.row0 + e] = p5_world(a, planes[(3u * j + d) * L.axis + F.n_bnd + i], d);
+                }
+            }
+        }
+    }
+}
+
+__global__ void p5_world_kernel(P5Args a, unsigned long long n) {
     const unsigned long long i = blockIdx.x * static_cast<unsigned long long>(blockDim.x) + threadIdx.x;
-    if (i >= 3ull * n) return;
-    const int d = static_cast<int>(i % 3ull);
-    const double c = d == 0 ? c0 : (d == 1 ? c1 : c2);
-    pos[i] = __double2float_rn(__dadd_rn(__dmul_rn(rows[i], scale), c));
+    if (i < 3ull * n) a.pos[i] = p5_world(a, a.rows[i], static_cast<uint32_t>(i % 3ull));
+}
+
+constexpr uint32_t kP5Eight = 8u * 2u * 152u;  // meshlets that CTAs of eight take at once
+constexpr uint32_t kP5Two = 103u << 10;        // two CTAs to an SM
+// eight meshlets of the largest size that is accepted (197 KB) and the static part, in an SM's 227 KB
+constexpr uint32_t kP5MaxSmem = 200u << 10;
+
+template <uint32_t M>
+cudaError_t p5_team_prepare() {
+    cudaError_t e = cudaFuncSetAttribute(p5_team_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(kP5MaxSmem));
+    if (e != cudaSuccess) return e;
+    // global data is read through L2 only
+    return cudaFuncSetAttribute(p5_team_kernel<M>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                cudaSharedmemCarveoutMaxShared);
+}
+
+template <uint32_t M>
+cudaError_t p5_team_launch(const P5Args& a, const P5Team& room, cudaStream_t s) {
+    p5_team_kernel<M><<<(a.n_meshlets + M - 1u) / M, p5_team_threads<M>(), p5_team_bytes(room, M), s>>>(a, room);
+    return cudaGetLastError();
 }
 
 // ---- host side ------------------------------------------------------------
@@ -510,9 +1218,11 @@ struct pldt5_handle {
     size_t len = 0;
     uint8_t* d_blob = nullptr;
     uint32_t* d_meta = nullptr;  // start (n + 1) | row_base (n) | tri_base (n) | ref_base (n)
-    uint32_t* d_refs = nullptr;
+    uint32_t* d_refs = nullptr;  // refs, walk: the general kernel's
     uint32_t* d_walk = nullptr;
-    double* d_rows = nullptr;
+    double* d_rows = nullptr;    // the boundary's, and for the general kernel all
+    uint32_t team = 0;           // meshlets per CTA of the team kernel, 0: the general kernel
+    P5Team room;
     Status* d_status = nullptr;
     Status* h_status = nullptr;
     cudaEvent_t done = nullptr;
@@ -541,6 +1251,8 @@ struct P5Host {
     std::vector<double> rows0;    // boundary rows, n_boundary x 3
     std::vector<uint32_t> meta;   // start (M + 1) | row_base (M) | tri_base (M) | ref_base (M)
     uint64_t refs = 0;
+    // the largest meshlet's
+    uint32_t most_local = 0, most_tris = 0, most_tokens = 0, most_bytes = 0;
 };
 
 static int p5_host_parse_sized(const uint8_t* data, size_t len, P5Host& H);
@@ -639,6 +1351,13 @@ static int p5_host_parse_sized(const uint8_t* data, size_t len, P5Host& H) {
         const uint32_t n_bnd = static_cast<uint32_t>(hb.read(16));
         const uint32_t n_int = static_cast<uint32_t>(hb.read(16));
         const uint32_t n_tris = static_cast<uint32_t>(hb.read(16));
+        const uint32_t n_strips = static_cast<uint32_t>(hb.read(16));
+        H.most_local = std::max(H.most_local, n_bnd + n_int);
+        H.most_tris = std::max(H.most_tris, n_tris);
+        H.most_tokens = std::max(H.most_tokens, n_tris + 2u * n_strips);
+        // staged: from the 16 bytes of its first bit to those of its last
+        const uint64_t first = (start[m] >> 3) & ~15ull, end = ((start[m + 1] + 127ull) >> 7) << 4;
+        H.most_bytes = std::max(H.most_bytes, static_cast<uint32_t>(std::min<uint64_t>(end - first, 0xFFFFFFF0u)));
         if (n_bnd + n_int > static_cast<uint32_t>(kP5MaxLocal))
             return fail(STRIDE_ERR_UNSUPPORTED, "meshlet %llu has %u local vertices (at most 256)",
                         (unsigned long long)m, n_bnd + n_int);
@@ -656,6 +1375,29 @@ static int p5_host_parse_sized(const uint8_t* data, size_t len, P5Host& H) {
     info.nbytes = len;
     H.refs = refs;
     return STRIDE_OK;
+}
+
+// Room and launch shape for a stream: the team kernel takes meshlets of up to
+// kTeamTokens tokens and kP5MaxStage bytes (encoded meshlets of 256 vertices
+// have half as many and a tenth), the general kernel streams with larger ones.
+static cudaError_t p5_plan(const P5Host& H, uint32_t& team, P5Team& room) {
+    team = 0;
+    room = P5Team{};
+    if (H.info.n_meshlets == 0 || H.most_tokens > kTeamTokens || H.most_bytes > kP5MaxStage) return cudaSuccess;
+    room.bits = H.most_bytes | 16u;
+    room.axis = H.most_local | 1u;
+    room.walk = H.most_local | 1u;
+    room.tok = team_tok_words(H.most_tokens);
+    room.asm_w = team_asm_words(H.most_tris);
+    room.tab = H.most_local | 1u;
+    // Eight meshlets per CTA as long as the CTAs are on the chip at once, two
+    // to an SM; above, sixteen where two such CTAs fit an SM: a decode then
+    // takes the CTAs' waves, and a CTA's chains hardly depend on its number of
+    // meshlets (sixteen against eight: meshlets of up to 64 vertices, 3,072 of
+    // them, 64 us against 81, 23,843 211 against 298; of up to 189 vertices,
+    // 10 79 against 75, 1,295 90 against 90, 9,921 211 against 250).
+    team = H.info.n_meshlets > kP5Eight && p5_team_bytes(room, 16u) <= kP5Two ? 16u : 8u;
+    return team == 8u ? p5_team_prepare<8>() : p5_team_prepare<16>();
 }
 
 extern "C" {
@@ -681,13 +1423,18 @@ int pldt5_open(const uint8_t* data, size_t len, pldt5_handle** out) {
     }
     h->scale = static_cast<double>(info.scale);
     h->delta = 2.0 * static_cast<double>(per_coord_err);
-    cudaError_t e;
+    cudaError_t e = p5_plan(H, h->team, h->room);
+    if (e != cudaSuccess) {
+        pldt5_free(h);
+        return cuda_fail(e, "pldt5_open");
+    }
+    const uint64_t gen = h->team ? 0 : 1;  // buffers of the general kernel
     const size_t blob = blob_alloc_bytes(len);
     if ((e = cudaMalloc(&h->d_blob, blob)) != cudaSuccess ||
         (e = cudaMalloc(&h->d_meta, 4 * meta.size())) != cudaSuccess ||
-        (e = cudaMalloc(&h->d_refs, 4 * std::max<uint64_t>(refs, 1))) != cudaSuccess ||
-        (e = cudaMalloc(&h->d_walk, 4 * std::max<uint64_t>(rows, 1))) != cudaSuccess ||
-        (e = cudaMalloc(&h->d_rows, 24 * std::max<uint64_t>(rows, 1))) != cudaSuccess ||
+        (e = cudaMalloc(&h->d_refs, 4 * std::max<uint64_t>(gen * refs, 1))) != cudaSuccess ||
+        (e = cudaMalloc(&h->d_walk, 4 * std::max<uint64_t>(gen * rows, 1))) != cudaSuccess ||
+        (e = cudaMalloc(&h->d_rows, 24 * std::max<uint64_t>(gen ? rows : nb, 1))) != cudaSuccess ||
         (e = cudaMalloc(&h->d_status, sizeof(Status))) != cudaSuccess ||
         (e = cudaHostAlloc(reinterpret_cast<void**>(&h->h_status), sizeof(Status), cudaHostAllocDefault)) !=
             cudaSuccess ||
@@ -726,36 +1473,43 @@ int pldt5_decode(pldt5_handle* h, void* stream, uint32_t* d_idx, float* d_pos) {
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const uint64_t M = h->info.n_meshlets, nb = h->info.n_boundary, rows = h->info.n_v;
     cudaError_t e;
-    if ((e = cudaMemsetAsync(h->d_status, 0, sizeof(Status), s)) != cudaSuccess ||
-        (rows > nb && (e = cudaMemsetAsync(h->d_rows + 3 * nb, 0, 24 * (rows - nb), s)) != cudaSuccess))
-        return cuda_fail(e, "pldt5_decode");
-    if (M) {
-        P5Args a;
-        a.blob = h->d_blob;
-        a.nbits = 8ull * h->len;
-        a.start = h->d_meta;
-        a.row_base = h->d_meta + M + 1;
-        a.tri_base = a.row_base + M;
-        a.ref_base = a.tri_base + M;
-        a.n_meshlets = static_cast<uint32_t>(M);
-        a.n_boundary = static_cast<uint32_t>(nb);
-        a.rows = h->d_rows;
-        a.refs = h->d_refs;
-        a.walk = h->d_walk;
-        a.idx = d_idx;
-        a.w0 = h->w[0];
-        a.w1 = h->w[1];
-        a.w2 = h->w[2];
-        a.delta = h->delta;
-        a.status = h->d_status;
-        // one lane per meshlet (kP5Threads per block)
-        p5_decode_kernel<<<static_cast<uint32_t>((M + kP5Threads - 1) / kP5Threads), kP5Threads, 0, s>>>(a);
-        if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "p5_decode_kernel");
-    }
-    if (rows) {
-        p5_world_kernel<<<static_cast<uint32_t>((3 * rows + 255) / 256), 256, 0, s>>>(
-            h->d_rows, rows, h->scale, h->center[0], h->center[1], h->center[2], d_pos);
-        if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "p5_world_kernel");
+    P5Args a;
+    a.blob = h->d_blob;
+    a.nbits = 8ull * h->len;
+    a.start = h->d_meta;
+    a.row_base = h->d_meta + M + 1;
+    a.tri_base = a.row_base + M;
+    a.ref_base = a.tri_base + M;
+    a.n_meshlets = static_cast<uint32_t>(M);
+    a.n_boundary = static_cast<uint32_t>(nb);
+    a.rows = h->d_rows;
+    a.refs = h->d_refs;
+    a.walk = h->d_walk;
+    a.idx = d_idx;
+    a.pos = d_pos;
+    a.w0 = h->w[0];
+    a.w1 = h->w[1];
+    a.w2 = h->w[2];
+    a.delta = h->delta;
+    a.scale = h->scale;
+    for (int d = 0; d < 3; d++) a.center[d] = h->center[d];
+    a.status = h->d_status;
+    if ((e = cudaMemsetAsync(h->d_status, 0, sizeof(Status), s)) != cudaSuccess) return cuda_fail(e, "pldt5_decode");
+    if (h->team) {
+        e = h->team == 8 ? p5_team_launch<8>(a, h->room, s) : p5_team_launch<16>(a, h->room, s);
+        if (e != cudaSuccess) return cuda_fail(e, "p5_team_kernel");
+    } else {
+        if (rows > nb && (e = cudaMemsetAsync(h->d_rows + 3 * nb, 0, 24 * (rows - nb), s)) != cudaSuccess)
+            return cuda_fail(e, "pldt5_decode");
+        if (M) {
+            // one lane per meshlet (kP5Threads per block)
+            p5_decode_kernel<<<static_cast<uint32_t>((M + kP5Threads - 1) / kP5Threads), kP5Threads, 0, s>>>(a);
+            if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "p5_decode_kernel");
+        }
+        if (rows) {
+            p5_world_kernel<<<static_cast<uint32_t>((3 * rows + 255) / 256), 256, 0, s>>>(a, rows);
+            if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "p5_world_kernel");
+        }
     }
     if ((e = cudaMemcpyAsync(h->h_status, h->d_status, sizeof(Status), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
         (e = cudaEventRecord(h->done, s)) != cudaSuccess)
