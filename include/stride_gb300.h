@@ -178,6 +178,12 @@ int stride_decode_host(stride_handle* h, void* stream, uint32_t* h_idx, float* h
  * *bad_meshlet (optional) receives the first failing meshlet. */
 int stride_status(stride_handle* h, int wait, uint32_t* bad_meshlet);
 
+/* Wait for the last decode, on the stream it was enqueued on (another one is
+ * ordered behind it), and return its status like stride_status(h, 1, ...):
+ * cheaper, as the status comes back behind the decode instead of in a copy of
+ * its own. */
+int stride_finish(stride_handle* h, void* stream, uint32_t* bad_meshlet);
+
 /* The side table of the last decode, derived on the device: per meshlet the
  * stream bit where its anchor (residual part) starts (d_resid_bit, n_meshlets
  * uint64) and the starts of the dy, dz, px, py, pz substreams relative to it
@@ -307,6 +313,8 @@ int stride_batch_launch_graph(stride_batch* b, void* stream);
 int stride_batch_autotune(stride_batch* b, void* stream, uint32_t* d_idx, float* d_pos,
                           int iters, stride_launch_cfg* best, float* best_ms);
 int stride_batch_status(stride_batch* b, int wait, uint32_t* bad_mesh, uint32_t* bad_meshlet);
+/* Like stride_finish. */
+int stride_batch_finish(stride_batch* b, void* stream, uint32_t* bad_mesh, uint32_t* bad_meshlet);
 void stride_batch_destroy(stride_batch* b);
 
 /* ---- serving: continuous batching over a device-resident arena ----------

@@ -102,6 +102,7 @@ SIGNATURES = [
     ("stride_normalise_codes", _I, [_P, _P, _P, _P]),
     ("stride_decode_host", _I, [_P, _P, _P, _P]),
     ("stride_status", _I, [_P, _I, ctypes.POINTER(_U32)]),
+    ("stride_finish", _I, [_P, _P, ctypes.POINTER(_U32)]),
     ("stride_decode_timed", _I, [_P, _P, _P, _P, _P]),
     ("stride_side_table", _I, [_P, _P, _P, _P]),
     ("stride_meshlet_ranges", _I, [_P, _P, _P, _P]),
@@ -126,6 +127,7 @@ SIGNATURES = [
     ("stride_batch_autotune", _I, [_P, _P, _P, _P, _I, ctypes.POINTER(LaunchCfg),
                                    ctypes.POINTER(ctypes.c_float)]),
     ("stride_batch_status", _I, [_P, _I, ctypes.POINTER(_U32), ctypes.POINTER(_U32)]),
+    ("stride_batch_finish", _I, [_P, _P, ctypes.POINTER(_U32), ctypes.POINTER(_U32)]),
     ("stride_batch_destroy", None, [_P]),
     ("stride_server_create", _I, [ctypes.POINTER(ServerOpts), ctypes.POINTER(_P)]),
     ("stride_server_submit", _I, [_P, _P, _SZ, ctypes.POINTER(_U64)]),

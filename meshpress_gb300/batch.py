@@ -67,9 +67,11 @@ class BatchDecoder:
     def decode(self, *, stream=None, check: bool = True):
         """-> (triangles uint32 (n_t, 3), positions float32 (n_v, 3)), device."""
         i, p = self._ptrs()
-        _lib.check(self._lib.stride_batch_decode(self._h, self._stream(stream), i, p), "stride_batch_decode")
-        if check:
-            self.check()
+        s = self._stream(stream)
+        _lib.check(self._lib.stride_batch_decode(self._h, s, i, p), "stride_batch_decode")
+        if check:  # check() on the decode's stream, which a new copy of the status need not wait for
+            bm, bl = ctypes.c_uint32(), ctypes.c_uint32()
+            _lib.check(self._lib.stride_batch_finish(self._h, s, ctypes.byref(bm), ctypes.byref(bl)), "batch decode")
         return self.d_tris, self.d_verts
 
     def decode_timed(self, *, stream=None):

@@ -1237,7 +1237,7 @@ static void pldt5_free(pldt5_handle* h) {
     cudaFree(h->d_walk);
     cudaFree(h->d_rows);
     cudaFree(h->d_status);
-    if (h->h_status) cudaFreeHost(h->h_status);
+    pinned_give(h->h_status);
     if (h->done) cudaEventDestroy(h->done);
     delete h;
 }
@@ -1436,8 +1436,7 @@ int pldt5_open(const uint8_t* data, size_t len, pldt5_handle** out) {
         (e = cudaMalloc(&h->d_walk, 4 * std::max<uint64_t>(gen * rows, 1))) != cudaSuccess ||
         (e = cudaMalloc(&h->d_rows, 24 * std::max<uint64_t>(gen ? rows : nb, 1))) != cudaSuccess ||
         (e = cudaMalloc(&h->d_status, sizeof(Status))) != cudaSuccess ||
-        (e = cudaHostAlloc(reinterpret_cast<void**>(&h->h_status), sizeof(Status), cudaHostAllocDefault)) !=
-            cudaSuccess ||
+        (e = pinned_take(sizeof(Status), reinterpret_cast<void**>(&h->h_status))) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&h->done, cudaEventDisableTiming)) != cudaSuccess) {
         pldt5_free(h);
         return cuda_fail(e, "pldt5_open");

@@ -3,11 +3,16 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <bitset>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
+#include <new>
 #include <string>
+#include <unordered_map>
+#include <vector>
 
 #include "stride_common.cuh"
 #include "stride_gb300.h"
@@ -158,28 +163,36 @@ unsigned long long plan_luts(MeshParams* p, uint32_t n, uint32_t* meshes, uint32
 
 }  // namespace stride
 
+// What a handle keeps on the device whatever its stream: uploaded at once.
+struct HandleFixed {
+    MeshParams params;
+    alignas(16) Status status;
+    uint32_t lut_mesh;  // the one-entry mesh list {0}
+};
+
 struct stride_handle {
     int device = 0;
     size_t len = 0, cap_bytes = 0;
     uint32_t cap_meshlets = 0;
+    HandleFixed* d_fixed = nullptr;
+    uint8_t* d_mem = nullptr;  // the buffers below
     uint8_t* d_blob = nullptr;
     MeshParams params;
-    MeshParams* d_params = nullptr;
     MeshletDesc* d_descs = nullptr;
     uint4* d_blk_sums = nullptr;
     BlockPrefix* d_blk_prefix = nullptr;
     uint32_t* d_walk_scratch = nullptr;
     unsigned long long walk_cap = 0;
-    Status* d_status = nullptr;
-    uint32_t* d_idx = nullptr;
-    float* d_pos = nullptr;
-    size_t cap_v = 0, cap_t = 0;
     float* d_lut = nullptr;             // dequantisation tables
     unsigned long long lut_cap = 0;     // floats
-    uint32_t* d_lut_mesh = nullptr;     // the one-entry mesh list {0}
     uint32_t n_lut = 0, lut_max = 0;
+    uint8_t* d_out = nullptr;           // stride_decode_host's outputs: triangles, positions
+    size_t cap_v = 0, cap_t = 0;
     cudaEvent_t done = nullptr;
+    Status* h_status = nullptr;         // pinned: stride_finish's copy
     bool launched = false;
+    bool known = false;                 // last: the last decode's status
+    Status last;
     LaunchCfg cfg;
     bool cfg_set = false;               // stride_set_config called: keep cfg across reloads
     long long wait_clocks = 1ll << 31;  // DecodeArgs::wait_clocks of this handle's decodes
@@ -196,6 +209,165 @@ static cudaError_t wait_upload(stride_handle* h, cudaStream_t s) {
 
 namespace stride {
 
+namespace {
+// Pinned memory for status words and part ends: cudaHostAlloc and
+// cudaFreeHost take 100 and 150 us a piece.  One slab of 64 KB, pinned on
+// first use and kept; slots go back to it, and what it has no room for is
+// pinned by itself.
+struct PinnedSlab {
+    static constexpr size_t kSlot = 256, kSlots = 256;
+    std::mutex mu;
+    uint8_t* base = nullptr;
+    std::bitset<kSlots> used;
+};
+PinnedSlab& pinned_slab() {
+    static PinnedSlab* s = new PinnedSlab;  // never destroyed: handles may outlive static objects
+    return *s;
+}
+}  // namespace
+
+cudaError_t pinned_take(size_t bytes, void** out) {
+    *out = nullptr;
+    if (bytes <= PinnedSlab::kSlot) {
+        PinnedSlab& s = pinned_slab();
+        std::lock_guard<std::mutex> g(s.mu);
+        if (!s.base && cudaHostAlloc(reinterpret_cast<void**>(&s.base), PinnedSlab::kSlot * PinnedSlab::kSlots,
+                                     cudaHostAllocPortable) != cudaSuccess) {
+            s.base = nullptr;
+            cudaGetLastError();
+        }
+        for (size_t i = 0; s.base && i < PinnedSlab::kSlots; i++) {
+            if (s.used[i]) continue;
+            s.used[i] = true;
+            *out = s.base + PinnedSlab::kSlot * i;
+            return cudaSuccess;
+        }
+    }
+    return cudaHostAlloc(out, bytes, cudaHostAllocPortable);
+}
+
+void pinned_give(void* p) {
+    if (!p) return;
+    PinnedSlab& s = pinned_slab();
+    {
+        std::lock_guard<std::mutex> g(s.mu);
+        const uint8_t* b = static_cast<uint8_t*>(p);
+        if (s.base && b >= s.base && b < s.base + PinnedSlab::kSlot * PinnedSlab::kSlots) {
+            s.used[static_cast<size_t>(b - s.base) / PinnedSlab::kSlot] = false;
+            return;
+        }
+    }
+    cudaFreeHost(p);
+}
+
+namespace {
+// Device blocks of closed handles for the next ones: a cudaMalloc and its
+// cudaFree take 60 us.  At most kBlocks blocks and kBytes bytes per process;
+// the oldest go back to the driver beyond that, all of them when an allocation
+// fails.  A block comes in once its device is idle (as cudaFree would wait),
+// so whoever takes it, on whatever stream, finds it unused.
+struct DeviceBlocks {
+    static constexpr size_t kBlocks = 16, kBytes = size_t(32) << 20;
+    struct Block {
+        void* p;
+        size_t bytes;
+        int device;
+    };
+    std::mutex mu;
+    std::vector<Block> free;               // the oldest first
+    std::unordered_map<void*, Block> out;  // in use
+    size_t bytes = 0;                      // of the free ones
+};
+DeviceBlocks& device_blocks() {
+    static DeviceBlocks* b = new DeviceBlocks;  // never destroyed: handles may outlive static objects
+    return *b;
+}
+}  // namespace
+
+static cudaError_t block_take(size_t bytes, void** out) {
+    *out = nullptr;
+    bytes = (std::max<size_t>(bytes, 1) + 255) & ~static_cast<size_t>(255);
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    DeviceBlocks& B = device_blocks();
+    try {
+        std::lock_guard<std::mutex> g(B.mu);
+        size_t best = B.free.size();
+        for (size_t i = 0; i < B.free.size(); i++) {
+            const DeviceBlocks::Block& b = B.free[i];
+            // not more than twice what is asked for, and 4 KB
+            if (b.device == dev && b.bytes >= bytes && b.bytes <= 2 * bytes + 4096 &&
+                (best == B.free.size() || b.bytes < B.free[best].bytes))
+                best = i;
+        }
+        if (best < B.free.size()) {
+            const DeviceBlocks::Block b = B.free[best];
+            B.out.emplace(b.p, b);
+            B.free.erase(B.free.begin() + static_cast<std::ptrdiff_t>(best));
+            B.bytes -= b.bytes;
+            *out = b.p;
+            return cudaSuccess;
+        }
+        void* p = nullptr;
+        e = cudaMalloc(&p, bytes);
+        if (e != cudaSuccess && !B.free.empty()) {
+            cudaGetLastError();
+            for (const DeviceBlocks::Block& b : B.free) cudaFree(b.p);
+            B.free.clear();
+            B.bytes = 0;
+            e = cudaMalloc(&p, bytes);
+        }
+        if (e != cudaSuccess) return e;
+        try {
+            B.out.emplace(p, DeviceBlocks::Block{p, bytes, dev});
+        } catch (const std::bad_alloc&) {
+            cudaFree(p);
+            return cudaErrorMemoryAllocation;
+        }
+        *out = p;
+        return cudaSuccess;
+    } catch (const std::bad_alloc&) {
+        return cudaErrorMemoryAllocation;
+    }
+}
+
+// `idle`: the caller has waited for the device the block is on.
+static void block_give(void* p, bool idle) {
+    if (!p) return;
+    DeviceBlocks& B = device_blocks();
+    std::lock_guard<std::mutex> g(B.mu);
+    const auto it = B.out.find(p);
+    bool kept = false;
+    if (it != B.out.end()) {
+        const DeviceBlocks::Block b = it->second;
+        B.out.erase(it);
+        if (idle && b.bytes <= DeviceBlocks::kBytes) {
+            try {
+                B.free.push_back(b);
+                B.bytes += b.bytes;
+                kept = true;
+            } catch (const std::bad_alloc&) {
+            }
+            while (B.free.size() > DeviceBlocks::kBlocks || B.bytes > DeviceBlocks::kBytes) {
+                cudaFree(B.free.front().p);
+                B.bytes -= B.free.front().bytes;
+                B.free.erase(B.free.begin());
+            }
+        }
+    }
+    if (!kept) cudaFree(p);
+}
+
+// Whether device `dev` has nothing left to do.
+static bool device_idle(int dev) {
+    int now = -1;
+    if (cudaGetDevice(&now) != cudaSuccess || now != dev) return false;
+    if (cudaDeviceSynchronize() == cudaSuccess) return true;
+    cudaGetLastError();
+    return false;
+}
+
 static void for_link_events(HostLink& L, void (*f)(cudaEvent_t*, cudaError_t*), cudaError_t* e) {
     for (cudaEvent_t* ev : {&L.conn_done, &L.vert_done, &L.done, &L.copied[0], &L.copied[1], &L.before_up})
         f(ev, e);
@@ -207,9 +379,9 @@ void host_link_free(HostLink& L) {
     for (cudaStream_t* c : {&L.copy[0], &L.copy[1], &L.up})
         if (*c) cudaStreamDestroy(*c), *c = nullptr;
     for_link_events(L, [](cudaEvent_t* ev, cudaError_t*) { if (*ev) cudaEventDestroy(*ev), *ev = nullptr; }, nullptr);
-    cudaFreeHost(L.h_end);
+    pinned_give(L.h_end);
     L.h_end = nullptr;
-    cudaFreeHost(L.h_status);
+    pinned_give(L.h_status);
     L.h_status = nullptr;
 }
 
@@ -221,8 +393,8 @@ cudaError_t host_link_init(HostLink& L) {
     for_link_events(L, [](cudaEvent_t* ev, cudaError_t* err) {
         if (*err == cudaSuccess) *err = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
     }, &e);
-    if (e == cudaSuccess) e = cudaHostAlloc(&L.h_status, sizeof(Status), cudaHostAllocDefault);
-    if (e == cudaSuccess) e = cudaHostAlloc(&L.h_end, kHostParts * sizeof(PartEnd), cudaHostAllocDefault);
+    if (e == cudaSuccess && !L.h_status) e = pinned_take(sizeof(Status), reinterpret_cast<void**>(&L.h_status));
+    if (e == cudaSuccess) e = pinned_take(kHostParts * sizeof(PartEnd), reinterpret_cast<void**>(&L.h_end));
     if (e != cudaSuccess) host_link_free(L);
     return e;
 }
@@ -238,9 +410,9 @@ void host_part_groups(uint32_t total_meshlets, uint32_t* part_g) {
 int decode_to_host(HostLink& L, const DecodeArgs& a, LaunchCfg cfg, void* stream, uint64_t n_t, uint64_t n_v,
                    uint32_t* h_idx, float* h_pos, const cudaEvent_t* bytes_in, uint32_t* bad, bool* ran) {
     *ran = false;
-    cudaError_t e = host_link_init(L);
-    if (e != cudaSuccess) return cuda_fail(e, "copy streams");
+    cudaError_t e;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const size_t ib = 12 * n_t, pb = 12 * n_v;
     // a failure once work is queued: nothing may still run on the buffers
     // or write the host outputs when this returns
     auto drain = [&]() {
@@ -258,7 +430,26 @@ int decode_to_host(HostLink& L, const DecodeArgs& a, LaunchCfg cfg, void* stream
         two.persistent = 1;
         if (check_config(two, a.wide_codes) == STRIDE_OK) cfg = two;
     }
-    const size_t ib = 12 * n_t, pb = 12 * n_v;
+    if (cfg.persistent >= 2) {
+        // One kernel, so nothing to copy beside it: everything on the decode's
+        // own stream (14-bit heightfields into pageable memory, 10 / 336 / 1,295
+        // / 2,631 meshlets: 73 / 79 / 102 / 143 us, by two copy streams 98 / 105
+        // / 128 / 168; pinned 64 / 70 / 92 / 136 and 71 / 78 / 98 / 139).
+        if (!L.h_status && (e = pinned_take(sizeof(Status), reinterpret_cast<void**>(&L.h_status))) != cudaSuccess)
+            return cuda_fail(e, "pinned status");
+        if (bytes_in && (e = cudaStreamWaitEvent(s, bytes_in[kHostParts - 1], 0)) != cudaSuccess)
+            return cuda_fail(e, "decode to host: upload");
+        const int rc = enqueue_decode(a, cfg, stream);
+        if (rc) return fail(rc, "decode launch failed: %s", cudaGetErrorString(cudaGetLastError()));
+        e = cudaMemcpyAsync(L.h_status, a.status, sizeof(Status), cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess && ib) e = cudaMemcpyAsync(h_idx, a.idx, ib, cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess && pb) e = cudaMemcpyAsync(h_pos, a.pos, pb, cudaMemcpyDeviceToHost, s);
+        const cudaError_t e2 = cudaStreamSynchronize(s);  // in any case: nothing may still write the host outputs
+        if (e != cudaSuccess || (e = e2) != cudaSuccess) return cuda_fail(e, "decode to host: copies");
+        *ran = true;
+        return status_to_code(*L.h_status, bad);
+    }
+    if ((e = host_link_init(L)) != cudaSuccess) return cuda_fail(e, "copy streams");
     const bool parts = cfg.persistent < 2 && host_parts(n_t, a.total_meshlets);
     if (parts) {
         // Part by part: its scan, the read-back of its end (the next part's
@@ -338,78 +529,53 @@ int decode_to_host(HostLink& L, const DecodeArgs& a, LaunchCfg cfg, void* stream
 }  // namespace stride
 
 static void free_buffers(stride_handle* h) {
-    cudaFree(h->d_blob);
-    cudaFree(h->d_params);
-    cudaFree(h->d_descs);
-    cudaFree(h->d_blk_sums);
-    cudaFree(h->d_blk_prefix);
-    cudaFree(h->d_walk_scratch);
-    cudaFree(h->d_status);
-    cudaFree(h->d_idx);
-    cudaFree(h->d_pos);
-    cudaFree(h->d_lut);
-    cudaFree(h->d_lut_mesh);
-    h->d_lut = nullptr;
-    h->d_lut_mesh = nullptr;
-    h->lut_cap = 0;
-    h->d_walk_scratch = nullptr;
-    h->walk_cap = 0;
-    h->d_blob = nullptr;
-    h->d_params = nullptr;
-    h->d_descs = nullptr;
-    h->d_blk_sums = nullptr;
-    h->d_blk_prefix = nullptr;
-    h->d_status = nullptr;
-    h->d_idx = nullptr;
-    h->d_pos = nullptr;
+    const bool idle = device_idle(h->device);
+    block_give(h->d_fixed, idle);
+    block_give(h->d_mem, idle);
+    block_give(h->d_out, idle);
+    pinned_give(h->h_status);
 }
 
-// Buffers for a stream of this size; also plans the dequantisation tables
-// of `p` (has_lut, lut_off) and sizes their buffer.
+// Buffers for a stream of this size, in one block; also plans the
+// dequantisation tables of `p` (has_lut, lut_off).  (A mesh of 23,254 triangles
+// decoded once, from open to close: 833 us with nine allocations, pinned words
+// and copy streams of its own, 124 now.)
 static int ensure_capacity(stride_handle* h, size_t len, MeshParams& p) {
-    const uint32_t n_meshlets = p.n_meshlets;
-    const uint64_t n_v = p.n_v;
-    cudaError_t e;
     const unsigned long long lut = plan_luts(&p, 1, nullptr, 1, &h->n_lut, &h->lut_max, true);
-    if (!h->d_lut_mesh) {
-        const uint32_t zero = 0u;
-        if ((e = cudaMalloc(&h->d_lut_mesh, sizeof(uint32_t))) != cudaSuccess ||
-            (e = cudaMemcpy(h->d_lut_mesh, &zero, sizeof(zero), cudaMemcpyHostToDevice)) != cudaSuccess)
-            return cuda_fail(e, "cudaMalloc(table list)");
-    }
-    if (lut > h->lut_cap) {
-        cudaFree(h->d_lut);
-        h->d_lut = nullptr;
-        if ((e = cudaMalloc(&h->d_lut, 4ull * lut)) != cudaSuccess) return cuda_fail(e, "cudaMalloc(tables)");
-        h->lut_cap = lut;
-    }
-    const unsigned long long ww = walk_scratch_words(n_v, n_meshlets);
-    if (ww > h->walk_cap) {
-        cudaFree(h->d_walk_scratch);
-        h->d_walk_scratch = nullptr;
-        if ((e = cudaMalloc(&h->d_walk_scratch, 4ull * ww)) != cudaSuccess) return cuda_fail(e, "cudaMalloc(scratch)");
-        h->walk_cap = ww;
-    }
-    if (blob_alloc_bytes(len) > h->cap_bytes) {
-        cudaFree(h->d_blob);
-        h->d_blob = nullptr;
-        h->cap_bytes = blob_alloc_bytes(len);
-        if ((e = cudaMalloc(&h->d_blob, h->cap_bytes)) != cudaSuccess) return cuda_fail(e, "cudaMalloc(stream)");
-    }
-    if (n_meshlets > h->cap_meshlets) {
-        cudaFree(h->d_descs);
-        cudaFree(h->d_blk_sums);
-        cudaFree(h->d_blk_prefix);
-        h->d_descs = nullptr;
-        h->d_blk_sums = nullptr;
-        h->d_blk_prefix = nullptr;
-        const uint32_t nb = scan_blocks(n_meshlets);
-        if ((e = cudaMalloc(&h->d_descs, sizeof(MeshletDesc) * n_meshlets)) != cudaSuccess ||
-            (e = cudaMalloc(&h->d_blk_sums, sizeof(uint4) * nb)) != cudaSuccess ||
-            (e = cudaMalloc(&h->d_blk_prefix, sizeof(BlockPrefix) * nb)) != cudaSuccess)
-            return cuda_fail(e, "cudaMalloc(scratch)");
-        h->cap_meshlets = n_meshlets;
-    }
+    const unsigned long long ww = walk_scratch_words(p.n_v, p.n_meshlets);
+    const size_t blob = blob_alloc_bytes(len);
+    if (h->d_mem && lut <= h->lut_cap && ww <= h->walk_cap && blob <= h->cap_bytes && p.n_meshlets <= h->cap_meshlets)
+        return STRIDE_OK;
+    const unsigned long long c_lut = std::max(lut, h->lut_cap), c_ww = std::max(ww, h->walk_cap);
+    const size_t c_blob = std::max(blob, h->cap_bytes);
+    const uint32_t c_m = std::max(p.n_meshlets, h->cap_meshlets), nb = scan_blocks(c_m);
+    size_t total = 0;
+    auto place = [&](unsigned long long bytes) {
+        const size_t at = total;
+        total += (static_cast<size_t>(bytes) + 255) & ~static_cast<size_t>(255);
+        return at;
+    };
+    const size_t o_blob = place(c_blob), o_descs = place(sizeof(MeshletDesc) * static_cast<unsigned long long>(c_m)),
+                 o_sums = place(sizeof(uint4) * static_cast<unsigned long long>(nb)),
+                 o_prefix = place(sizeof(BlockPrefix) * static_cast<unsigned long long>(nb)), o_walk = place(4ull * c_ww),
+                 o_lut = place(4ull * c_lut);
+    block_give(h->d_mem, false);  // cudaFree: after the work queued on it
+    h->d_mem = nullptr;
+    h->cap_bytes = 0;
+    h->cap_meshlets = 0;
+    h->walk_cap = h->lut_cap = 0;
+    const cudaError_t e = block_take(total, reinterpret_cast<void**>(&h->d_mem));
+    if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(stream, scratch)");
+    h->d_blob = h->d_mem + o_blob;
+    h->d_descs = reinterpret_cast<MeshletDesc*>(h->d_mem + o_descs);
+    h->d_blk_sums = reinterpret_cast<uint4*>(h->d_mem + o_sums);
+    h->d_blk_prefix = reinterpret_cast<BlockPrefix*>(h->d_mem + o_prefix);
+    h->d_walk_scratch = reinterpret_cast<uint32_t*>(h->d_mem + o_walk);
+    h->d_lut = reinterpret_cast<float*>(h->d_mem + o_lut);
+    h->cap_bytes = c_blob;
+    h->cap_meshlets = c_m;
+    h->walk_cap = c_ww;
+    h->lut_cap = c_lut;
     return STRIDE_OK;
 }
 
@@ -492,12 +658,14 @@ int stride_open(const uint8_t* data, size_t len, stride_handle** out) {
         delete h;
         return rc;
     }
-    if ((e = cudaMalloc(&h->d_params, sizeof(MeshParams))) != cudaSuccess ||
-        (e = cudaMalloc(&h->d_status, sizeof(Status))) != cudaSuccess ||
+    HandleFixed fixed;
+    std::memset(&fixed, 0, sizeof(fixed));
+    fixed.params = h->params;
+    if ((e = block_take(sizeof(HandleFixed), reinterpret_cast<void**>(&h->d_fixed))) != cudaSuccess ||
+        (e = pinned_take(sizeof(Status), reinterpret_cast<void**>(&h->h_status))) != cudaSuccess ||
         (e = cudaMemcpy(h->d_blob, data, len, cudaMemcpyHostToDevice)) != cudaSuccess ||
         (e = cudaMemset(h->d_blob + len, 0, h->cap_bytes - len)) != cudaSuccess ||
-        (e = cudaMemcpy(h->d_params, &h->params, sizeof(MeshParams), cudaMemcpyHostToDevice)) != cudaSuccess ||
-        (e = cudaMemset(h->d_status, 0, sizeof(Status))) != cudaSuccess ||
+        (e = cudaMemcpy(h->d_fixed, &fixed, sizeof(HandleFixed), cudaMemcpyHostToDevice)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&h->done, cudaEventDisableTiming)) != cudaSuccess) {
         free_buffers(h);
         delete h;
@@ -544,7 +712,7 @@ int stride_reload(stride_handle* h, const uint8_t* data, size_t len, void* strea
             return cuda_fail(e, "stride_reload");
         // the mesh record first: a copy queued on `stream` would go after
         // every part on the copy engine, and the first part's scan needs it
-        if ((e = cudaMemcpyAsync(h->d_params, &h->params, sizeof(MeshParams), cudaMemcpyHostToDevice, L.up)) !=
+        if ((e = cudaMemcpyAsync(&h->d_fixed->params, &h->params, sizeof(MeshParams), cudaMemcpyHostToDevice, L.up)) !=
             cudaSuccess)
             return cuda_fail(e, "stride_reload");
         for (int q = 0; q < kHostParts; q++) {
@@ -559,7 +727,7 @@ int stride_reload(stride_handle* h, const uint8_t* data, size_t len, void* strea
         h->up_parts = true;
     } else if ((e = cudaMemcpyAsync(h->d_blob, data, len, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
                (e = cudaMemsetAsync(h->d_blob + len, 0, pad, s)) != cudaSuccess ||
-               (e = cudaMemcpyAsync(h->d_params, &h->params, sizeof(MeshParams), cudaMemcpyHostToDevice, s)) !=
+               (e = cudaMemcpyAsync(&h->d_fixed->params, &h->params, sizeof(MeshParams), cudaMemcpyHostToDevice, s)) !=
                    cudaSuccess) {
         return cuda_fail(e, "stride_reload");
     }
@@ -578,7 +746,7 @@ static DecodeArgs handle_args(stride_handle* h, uint32_t* d_idx, float* d_pos, i
     DecodeArgs a;
     a.wait_clocks = h->wait_clocks;
     a.arena = h->d_blob;
-    a.meshes = h->d_params;
+    a.meshes = &h->d_fixed->params;
     a.meshlet_mesh = nullptr;
     a.total_meshlets = h->params.n_meshlets;
     a.n_meshes = 1;
@@ -587,13 +755,13 @@ static DecodeArgs handle_args(stride_handle* h, uint32_t* d_idx, float* d_pos, i
     a.blk_prefix = h->d_blk_prefix;
     a.walk_scratch = h->d_walk_scratch;
     a.walk_cap = h->walk_cap;
-    a.status = h->d_status;
+    a.status = &h->d_fixed->status;
     a.idx = d_idx;
     a.pos = d_pos;
     a.codes = d_codes;
     a.wide_codes = h->params.g_bits[0] > 16 || h->params.g_bits[1] > 16 || h->params.g_bits[2] > 16;
     a.lut = h->d_lut;
-    a.lut_meshes = h->d_lut_mesh;
+    a.lut_meshes = &h->d_fixed->lut_mesh;
     a.n_lut_meshes = h->n_lut;
     a.lut_max = h->lut_max;
     a.hint_bytes = h->len;
@@ -602,13 +770,18 @@ static DecodeArgs handle_args(stride_handle* h, uint32_t* d_idx, float* d_pos, i
     return a;
 }
 
+// After a reload that could not allocate, until one that could.
+static int no_buffers() { return fail(STRIDE_ERR_CUDA, "the last reload could not allocate the handle's buffers"); }
+
 int stride_decode_timed(stride_handle* h, void* stream, uint32_t* d_idx, float* d_pos, float* kernel_ms) {
     if (!h || !d_idx || !d_pos) return fail(STRIDE_ERR_ARG, "null argument");
+    if (!h->d_mem) return no_buffers();
     if ((reinterpret_cast<uintptr_t>(d_idx) & 15u) || (reinterpret_cast<uintptr_t>(d_pos) & 3u))
         return fail(STRIDE_ERR_ARG, "index output must be 16-byte aligned, positions 4-byte aligned");
     cudaEvent_t ev[4];
     for (auto& e : ev) cudaEventCreate(&e);
     void* evp[4] = {ev[0], ev[1], ev[2], ev[3]};
+    h->known = false;
     int rc = wait_upload(h, static_cast<cudaStream_t>(stream)) == cudaSuccess
                  ? enqueue_decode(handle_args(h, d_idx, d_pos, nullptr), h->cfg, stream, evp)
                  : STRIDE_ERR_CUDA;
@@ -632,11 +805,13 @@ int stride_decode_timed(stride_handle* h, void* stream, uint32_t* d_idx, float* 
 int stride_decode(stride_handle* h, void* stream, uint32_t* d_idx, float* d_pos, int32_t* d_codes) {
     if (!h) return fail(STRIDE_ERR_ARG, "null handle");
     if ((!d_idx && h->params.n_t) || (!d_pos && h->params.n_v)) return fail(STRIDE_ERR_ARG, "null output pointer");
+    if (!h->d_mem) return no_buffers();
     if ((reinterpret_cast<uintptr_t>(d_idx) & 15u) || (reinterpret_cast<uintptr_t>(d_pos) & 3u) ||
         (reinterpret_cast<uintptr_t>(d_codes) & 3u))
         return fail(STRIDE_ERR_ARG, "index output must be 16-byte aligned, positions and codes 4-byte aligned");
     if (wait_upload(h, static_cast<cudaStream_t>(stream)) != cudaSuccess)
         return fail(STRIDE_ERR_CUDA, "decode launch failed: %s", cudaGetErrorString(cudaGetLastError()));
+    h->known = false;
     const int rc = enqueue_decode(handle_args(h, d_idx, d_pos, d_codes), h->cfg, stream);
     if (rc) return fail(rc, "decode launch failed: %s", cudaGetErrorString(cudaGetLastError()));
     last_launch(&h->launch_smem, &h->launch_grid);
@@ -646,20 +821,41 @@ int stride_decode(stride_handle* h, void* stream, uint32_t* d_idx, float* d_pos,
     return STRIDE_OK;
 }
 
+static int say_status(const Status& st, uint32_t* bad_meshlet) {
+    uint32_t bad = 0;
+    const int rc = status_to_code(st, &bad);
+    if (bad_meshlet) *bad_meshlet = bad;
+    return rc ? fail(rc, "%s (meshlet %u)", status_message(rc), bad) : STRIDE_OK;
+}
+
 int stride_status(stride_handle* h, int wait, uint32_t* bad_meshlet) {
     if (!h) return fail(STRIDE_ERR_ARG, "null handle");
     if (!h->launched) return STRIDE_OK;
+    if (h->known) return say_status(h->last, bad_meshlet);
     cudaError_t e = wait ? cudaEventSynchronize(h->done) : cudaEventQuery(h->done);
     if (e == cudaErrorNotReady) return STRIDE_ERR_BUSY;
     if (e != cudaSuccess) return cuda_fail(e, "decode");
     Status st;
-    if ((e = cudaMemcpy(&st, h->d_status, sizeof(st), cudaMemcpyDeviceToHost)) != cudaSuccess)
+    if ((e = cudaMemcpy(&st, &h->d_fixed->status, sizeof(st), cudaMemcpyDeviceToHost)) != cudaSuccess)
         return cuda_fail(e, "cudaMemcpy(status)");
-    uint32_t bad = 0;
-    const int rc = status_to_code(st, &bad);
-    if (bad_meshlet) *bad_meshlet = bad;
-    if (rc) return fail(rc, "%s (meshlet %u)", status_message(rc), bad);
-    return STRIDE_OK;
+    return say_status(st, bad_meshlet);
+}
+
+// The status comes back on the decode's stream, queued behind it: a copy
+// that starts when the host has seen the decode's end costs 11 us more.
+int stride_finish(stride_handle* h, void* stream, uint32_t* bad_meshlet) {
+    if (!h) return fail(STRIDE_ERR_ARG, "null handle");
+    if (!h->launched) return STRIDE_OK;
+    if (h->known) return say_status(h->last, bad_meshlet);
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    cudaError_t e = cudaStreamWaitEvent(s, h->done, 0);  // another stream's decode
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h->h_status, &h->d_fixed->status, sizeof(Status), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaEventRecord(h->done, s);
+    if (e == cudaSuccess) e = cudaEventSynchronize(h->done);
+    if (e != cudaSuccess) return cuda_fail(e, "decode");
+    h->last = *h->h_status;
+    h->known = true;
+    return say_status(h->last, bad_meshlet);
 }
 
 int stride_side_table(stride_handle* h, void* stream, uint64_t* d_resid_bit, uint16_t* d_sub_offs) {
@@ -733,19 +929,20 @@ int stride_cull_meshlets(const float* d_bounds, uint32_t n, const float* planes,
 
 int stride_decode_host(stride_handle* h, void* stream, uint32_t* h_idx, float* h_pos) {
     if (!h || (!h_idx && h->params.n_t) || (!h_pos && h->params.n_v)) return fail(STRIDE_ERR_ARG, "null argument");
-    cudaError_t e;
-    if (h->params.n_v > h->cap_v) {
-        cudaFree(h->d_pos);
-        h->d_pos = nullptr;
-        if ((e = cudaMalloc(&h->d_pos, 12 * h->params.n_v)) != cudaSuccess) return cuda_fail(e, "cudaMalloc(pos)");
-        h->cap_v = h->params.n_v;
+    if (!h->d_mem) return no_buffers();
+    if (h->params.n_v > h->cap_v || h->params.n_t > h->cap_t) {
+        const size_t cv = std::max<size_t>(h->params.n_v, h->cap_v), ct = std::max<size_t>(h->params.n_t, h->cap_t);
+        block_give(h->d_out, false);
+        h->d_out = nullptr;
+        h->cap_v = h->cap_t = 0;
+        const cudaError_t e = block_take(((12 * ct + 255) & ~static_cast<size_t>(255)) + 12 * cv,
+                                         reinterpret_cast<void**>(&h->d_out));
+        if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(outputs)");
+        h->cap_v = cv;
+        h->cap_t = ct;
     }
-    if (h->params.n_t > h->cap_t) {
-        cudaFree(h->d_idx);
-        h->d_idx = nullptr;
-        if ((e = cudaMalloc(&h->d_idx, 12 * h->params.n_t)) != cudaSuccess) return cuda_fail(e, "cudaMalloc(idx)");
-        h->cap_t = h->params.n_t;
-    }
+    uint32_t* d_idx = reinterpret_cast<uint32_t*>(h->d_out);
+    float* d_pos = reinterpret_cast<float*>(h->d_out + ((12 * h->cap_t + 255) & ~static_cast<size_t>(255)));
     uint32_t bad = 0;
     bool ran = false;
     // after a reload by parts, each part of the decode starts when its
@@ -754,9 +951,14 @@ int stride_decode_host(stride_handle* h, void* stream, uint32_t* h_idx, float* h
     // scan, whatever the bytes not yet in hold (which of its faults the
     // error names can then differ from a decode after the whole upload)
     const cudaEvent_t* bytes_in = h->up_parts ? h->link.bytes_in : nullptr;
-    const int rc = decode_to_host(h->link, handle_args(h, h->d_idx, h->d_pos, nullptr), h->cfg, stream,
+    const int rc = decode_to_host(h->link, handle_args(h, d_idx, d_pos, nullptr), h->cfg, stream,
                                   h->params.n_t, h->params.n_v, h_idx, h_pos, bytes_in, &bad, &ran);
-    if (!ran) return rc;
+    if (!ran) {
+        h->known = false;
+        return rc;
+    }
+    h->last = *h->link.h_status;
+    h->known = true;
     h->launched = true;  // later status queries see this decode
     cudaEventRecord(h->done, static_cast<cudaStream_t>(stream));
     return rc ? fail(rc, "%s (meshlet %u)", status_message(rc), bad) : STRIDE_OK;

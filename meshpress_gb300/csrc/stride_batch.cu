@@ -38,6 +38,7 @@ struct stride_batch {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     cudaEvent_t done = nullptr;
+    Status* h_status = nullptr;  // pinned: stride_batch_finish's copy
     bool launched = false;
     HostLink link;          // stride_batch_decode_to_host, and an upload by parts
     bool up_parts = false;  // the last stride_batch_upload went by parts (link.bytes_in)
@@ -87,6 +88,7 @@ int build_mesh_table(const uint8_t* const* blobs, const size_t* lens, uint32_t n
 
 static void batch_free(stride_batch* b) {
     host_link_free(b->link);
+    pinned_give(b->h_status);
     if (b->exec) cudaGraphExecDestroy(b->exec);
     if (b->graph) cudaGraphDestroy(b->graph);
     if (b->done) cudaEventDestroy(b->done);
@@ -493,6 +495,21 @@ int stride_batch_status(stride_batch* b, int wait, uint32_t* bad_mesh, uint32_t*
         return cuda_fail(e, "cudaMemcpy(status)");
     uint32_t bad = 0;
     const int rc = status_to_code(st, &bad);
+    return rc ? batch_error(b, rc, bad, bad_mesh, bad_meshlet) : STRIDE_OK;
+}
+
+int stride_batch_finish(stride_batch* b, void* stream, uint32_t* bad_mesh, uint32_t* bad_meshlet) {
+    if (!b) return fail(STRIDE_ERR_ARG, "null batch");
+    if (!b->launched) return STRIDE_OK;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    cudaError_t e = b->h_status ? cudaSuccess : pinned_take(sizeof(Status), reinterpret_cast<void**>(&b->h_status));
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(s, b->done, 0);  // another stream's decode
+    if (e == cudaSuccess) e = cudaMemcpyAsync(b->h_status, b->d_status, sizeof(Status), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaEventRecord(b->done, s);
+    if (e == cudaSuccess) e = cudaEventSynchronize(b->done);
+    if (e != cudaSuccess) return cuda_fail(e, "batch decode");
+    uint32_t bad = 0;
+    const int rc = status_to_code(*b->h_status, &bad);
     return rc ? batch_error(b, rc, bad, bad_mesh, bad_meshlet) : STRIDE_OK;
 }
 

@@ -59,6 +59,10 @@ struct HostLink {
     PartEnd* h_end = nullptr;   // pinned, kHostParts entries
     Status* h_status = nullptr; // pinned: the decode's status, copied out with the outputs
 };
+// Pinned host memory for small blocks, and back.
+cudaError_t pinned_take(size_t bytes, void** out);
+void pinned_give(void* p);
+
 cudaError_t host_link_init(HostLink& L);
 void host_link_free(HostLink& L);
 

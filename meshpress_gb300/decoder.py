@@ -127,11 +127,16 @@ class ParaDeltaV5GpuDecoder:
         if codes is not None:
             assert codes.dtype == torch.int32 and codes.is_cuda and codes.numel() >= 3 * self.n_v_total
             cptr = ctypes.c_void_p(codes.data_ptr())
-        rc = self._lib.stride_decode(self._h, ctypes.c_void_p(_stream_handle(stream)),
-                                     ctypes.c_void_p(d_idx.data_ptr()), ctypes.c_void_p(d_pos.data_ptr()), cptr)
+        s = ctypes.c_void_p(_stream_handle(stream))
+        rc = self._lib.stride_decode(self._h, s, ctypes.c_void_p(d_idx.data_ptr()), ctypes.c_void_p(d_pos.data_ptr()), cptr)
         _lib.check(rc, "stride_decode")
         if check:
-            self.check()
+            self._finish(s)
+
+    def _finish(self, s):
+        """check() on the decode's stream, which a new copy of the status need not wait for."""
+        bad = ctypes.c_uint32()
+        _lib.check(self._lib.stride_finish(self._h, s, ctypes.byref(bad)), "stride decode")
 
     def check(self):
         """Wait for the last decode and raise if the stream was invalid."""
@@ -209,7 +214,7 @@ class ParaDeltaV5GpuDecoder:
                                                   ctypes.c_void_p(codes.data_ptr()), ctypes.c_void_p(vn.data_ptr()))
             _lib.check(rc, "stride_normalise_codes")
         if check:
-            self.check()
+            self._finish(ctypes.c_void_p(_stream_handle(s)))
         self.d_verts_norm = vn
         return self.d_verts_norm, tris.view(torch.int32)
 
