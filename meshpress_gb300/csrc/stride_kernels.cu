@@ -1224,13 +1224,13 @@ int check_config(const LaunchCfg& cfg, bool wide) {
 // such waves.  Step in us, L2 flushed, 12-bit heightfields, every output
 // bit-identical; before: the fused kernel up to 128 groups, then the two
 // kernels:
-//   meshlets            10   158   650  1295  2631  4090  5221  7503  9229  10584
-//   before              99   110   114   112   112   116   119   118   122    124
-//   4 per CTA           38    37    39    63    95   128
-//   8 per CTA           38    40    40    46    71    79   108   136   151    177
-//   16 per CTA          50    50    48    50    58    60   100   106   110    146
-// (14-bit spheres of 103 and 1,738 meshlets: 220 -> 56, 196 -> 58 us; 20-bit
-// heightfield of 5,221: 245 -> 108 us.)
+//   meshlets            10   158   650  1295  2631  4090  5221  7503  9101  10584
+//   before              97   110   112   112   110   114   116   118   120    124
+//   4 per CTA           32    34    36    57    87   118   142   189   228    259
+//   8 per CTA           34    36    36    42    65    73    97   122   136    163
+//   16 per CTA          44    46    46    46    54    58    93    99   106    138
+// (14-bit spheres of 103 and 1,738 meshlets: 220 -> 48, 196 -> 52 us; 20-bit
+// heightfield of 5,221: 245 -> 96 us.)
 constexpr uint32_t kTeam4 = 700u, kTeam8 = 2432u, kTeamMost = 9728u;
 
 LaunchCfg default_config(uint32_t total_meshlets) {

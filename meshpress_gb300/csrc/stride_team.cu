@@ -20,6 +20,7 @@
 //              last edge-code-0 token), triangles, first occurrences, walk.
 //  3. walk     lane per (meshlet, axis): a decoder warp finds the substreams
 //              and reads residuals, a predictor warp behind it runs IRLP.
+//              The other warps meanwhile put out the triangles.
 //  4. emit     a warp per meshlet, lane per vertex: exact positions.
 //
 // Loops that carry a chain are unrolled, free of branches and of the same
@@ -48,13 +49,12 @@ constexpr uint32_t kTeamThreads = 32u * (kTeamAsm + 2u);
 constexpr uint32_t kTeamRes = 16u;    // residuals between hand-overs from decoder to predictor warps
 
 // Shared memory of a round: staged bytes, walks, then the token records and
-// the assembly's words (each id's last token, the triangles), whose place the
-// code planes take when the walk starts.  Laid out by what the round's
-// meshlets need.
-__host__ __device__ inline uint32_t team_bytes(uint32_t bits, uint32_t walk, uint32_t tok, uint32_t asm_words,
-                                               uint32_t plane) {
-    const uint32_t uni = tok + asm_words > plane ? tok + asm_words : plane;
-    const uint32_t rest = 4u * (walk + uni);
+// each id's last token, whose place the code planes take when the walk starts,
+// then the triangles.  Laid out by what the round's meshlets need.
+__host__ __device__ inline uint32_t team_bytes(uint32_t bits, uint32_t walk, uint32_t tok, uint32_t last,
+                                               uint32_t plane, uint32_t tri) {
+    const uint32_t uni = tok + last > plane ? tok + last : plane;
+    const uint32_t rest = 4u * (walk + uni + tri);
     return bits + (rest > kTeamSlack ? rest : kTeamSlack);
 }
 // A meshlet's words in each.
@@ -97,40 +97,95 @@ struct TeamFacts : TeamSize {
     uint32_t mi;                        // its mesh
     uint32_t n_strips;
     uint32_t start_bit, end_bit, ssz;   // ssz: bytes staged
-    uint32_t bit_off, walk_off, tok_off, asm_off, plane_off;  // bytes, then words
+    uint32_t bit_off, walk_off, tok_off, last_off, plane_off, tri_off;  // bytes, then words
     uint32_t axis_words;                // one axis' code plane
     // found on the way
     uint32_t anchor;                    // the stream bit after the connectivity
     uint32_t walk;                      // n_kind0 | n_walk << 16
+    uint32_t tcnt;                      // triangles
     uint32_t bad;                       // invalid connectivity: reported, the later phases skip it
     uint32_t wbad;                      // invalid walk
     uint32_t slow[3];                   // the axis is decoded by team_walk_slow
 };
 
+// A lane's 96 bits at bit `pos` of the words at shared address `base`.
+__device__ __forceinline__ void team_window96(uint32_t base, uint32_t pos, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+    const uint32_t a = mad_u32(pos >> 5, 4u, base), o = pos & 31u;
+    uint32_t w0, w1, w2, w3;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w0) : "r"(a));
+    asm volatile("ld.shared.u32 %0, [%1+4];" : "=r"(w1) : "r"(a));
+    asm volatile("ld.shared.u32 %0, [%1+8];" : "=r"(w2) : "r"(a));
+    asm volatile("ld.shared.u32 %0, [%1+12];" : "=r"(w3) : "r"(a));
+    hi = __funnelshift_l(w1, w0, o);
+    mid = __funnelshift_l(w2, w1, o);
+    lo = __funnelshift_l(w3, w2, o);
+}
+
+// Four codewords from bit `pos`, the first n of them, as zigzag values; true
+// when one is longer than 32 bits or starts beyond the window (the caller then
+// takes them again by the general reader).  A window read once for four leaves
+// the leading zeros, a multiply-add and a funnel shift between one codeword and
+// the next: 73 cycles a residual on one warp, with its store, against 87 with a
+// window refilled at each codeword.
+struct TeamCode {
+    uint32_t em, k1, zmul, pow;  // a codeword of z leading zeros has z * em + k1 bits
+    __device__ __forceinline__ explicit TeamCode(uint32_t tk) {
+        const uint32_t k = tk & 0x3Fu;
+        const bool eg = (tk & 0x80u) != 0u;
+        em = eg ? 2u : 1u;
+        k1 = k + 1u;
+        pow = 1u << k;
+        zmul = eg ? 0u : pow;
+    }
+};
+__device__ __forceinline__ bool team_four(uint32_t base, uint32_t& pos, const TeamCode& C, int n, uint32_t* u) {
+    uint32_t hi, mid, lo;
+    team_window96(base, pos, hi, mid, lo);
+    uint32_t used = 0u, longest = 0u, before = 0u;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const uint32_t z = __clz(hi), len = mad_u32(z, C.em, C.k1);
+        // the value bits with the terminator as their leading one: 2^nb + value
+        u[i] = mad_u32(z, C.zmul, __funnelshift_rc(hi, 0u, 32u - len) - C.pow);
+        const uint32_t take = i < n ? len : 0u;
+        longest = max(longest, take);
+        before = used;
+        used += take;
+        hi = __funnelshift_lc(mid, hi, take);
+        mid = __funnelshift_lc(lo, mid, take);
+        lo = __funnelshift_lc(0u, lo, take);
+    }
+    pos += used;
+    return (longest > 32u) | (before > 64u);
+}
+
 // Skip n codewords of one substream from bit `pos` of w (their lengths are
 // not stored), n its own in every lane of the warp (0: none).  Unary
 // (Rice(0)) codewords end at a one bit each: when every lane's are, whole
-// windows by their count of one bits, then the last one by halving.  Others
+// windows by their count of one bits, then the last word by halving.  Others
 // eight at a time; a lane that met one longer than the window takes its eight
 // again by the general reader.  False for a malformed one.
 __device__ __forceinline__ bool team_skip(const uint32_t* __restrict__ w, uint32_t& pos, uint32_t tk, uint32_t n,
                                           uint32_t limit) {
     const uint32_t most = __reduce_max_sync(kFull, n);
     if (most == 0u) return true;
+    const uint32_t base = smem_addr(w);
     bool ok = true;
-    BitBuf<true> b;
-    b.w = w;
-    b.end_word = 0u;
-    b.seek(pos);
     if (__all_sync(kFull, tk == 0u || n == 0u)) {
-        uint32_t c;
-        while ((c = __popc(b.hi)) < n) {
-            b.skip(32u);
-            n -= c;
-            if (b.at() > limit) break;  // only a corrupt stream runs past its meshlet
+        uint32_t hi, mid, lo, c0, c1, c2;  // one bits up to each word's end
+        for (;;) {
+            team_window96(base, pos, hi, mid, lo);
+            c0 = __popc(hi);
+            c1 = c0 + __popc(mid);
+            c2 = c1 + __popc(lo);
+            if (c2 >= n) break;
+            pos += 96u;
+            n -= c2;
+            if (pos > limit) break;  // only a corrupt stream runs past its meshlet
         }
         __syncwarp();
-        uint32_t y = b.hi, at = 0u, need = n;
+        uint32_t y = n > c1 ? lo : (n > c0 ? mid : hi), need = n - (n > c1 ? c1 : (n > c0 ? c0 : 0u));
+        uint32_t at = n > c1 ? 64u : (n > c0 ? 32u : 0u);
 #pragma unroll
         for (uint32_t wd = 16u; wd >= 1u; wd >>= 1) {
             const uint32_t t = __popc(y >> (32u - wd));  // ones in the top wd bits
@@ -139,30 +194,25 @@ __device__ __forceinline__ bool team_skip(const uint32_t* __restrict__ w, uint32
             y = more ? (y << wd) : y;
             at += more ? wd : 0u;
         }
-        b.skip(n ? at + 1u : 0u);
+        pos += n ? at + 1u : 0u;
     } else {
-        const uint32_t k1 = (tk & 0x3Fu) + 1u, em = (tk & 0x80u) ? 2u : 1u;
+        const TeamCode C(tk);
         for (uint32_t i0 = 0; i0 < most; i0 += 8u) {
-            uint32_t from = b.at();
-            bool longc = false;
-#pragma unroll
-            for (uint32_t i = 0; i < 8u; i++) {
-                const bool on = i0 + i < n;
-                const uint32_t len = __clz(b.hi) * em + k1;
-                longc = longc | (on & (len > 32u));
-                b.skip(on ? min(len, 32u) : 0u);
-            }
-            if (longc) {
-                const uint32_t m = min(8u, n - i0);
+            const int left = static_cast<int>(n) - static_cast<int>(i0);
+            uint32_t from = pos, u[4];
+            bool far = team_four(base, pos, C, left, u);
+            far = team_four(base, pos, C, left - 4, u) | far;
+            if (far) {
+                const int m = min(8, left);
                 int32_t r;
-                for (uint32_t i = 0; i < m; i++) ok = residual<true>(w, 0u, from, tk, limit, r) & ok;
-                b.seek(from);
+                for (int i = 0; i < m; i++) ok = residual<true>(w, 0u, from, tk, limit, r) & ok;
+                pos = from;
             }
-            if (b.at() > limit) b.seek(limit), ok = false;
+            ok = ok & (pos <= limit);
+            pos = min(pos, limit);
             __syncwarp();
         }
     }
-    pos = b.at();
     return ok & (pos <= limit);
 }
 
@@ -215,68 +265,69 @@ __device__ __forceinline__ void team_axis_open(TeamAxis& X, const MeshParams* __
     X.tp = d == 0u ? X.tk[3] : (d == 1u ? X.tk[4] : X.tk[5]);
 }
 
-// Eight codewords of a parallelogram substream as residuals into the code
-// plane at their vertices, the first n of the eight bytes at `list`.  A lane that
-// met one longer than the window takes its eight again by the general
-// reader.  A residual that does not fit the plane sets `slow`; false for a
-// malformed codeword.
-// kDown: the list runs backwards; kStore false: only skipped.
-template <bool kWide, bool kDown>
-__device__ __forceinline__ bool team_decode(BitBuf<true>& b, uint32_t tk, uint32_t limit,
+// kN codewords (8 or 16) of a substream as residuals into the code plane at
+// their vertices, the first n of the kN bytes at `list`.  A lane that met one
+// longer than the window takes all of them again by the general reader.  A
+// residual that does not fit the plane sets `slow`; false for a malformed
+// codeword.  kDown: the list runs backwards; store false: only skipped.
+template <uint32_t kN, bool kWide, bool kDown>
+__device__ __forceinline__ bool team_decode(const uint32_t* __restrict__ w, uint32_t& pos, uint32_t tk, uint32_t limit,
                                             const uint8_t* __restrict__ list, int n, bool store, uint32_t plane,
                                             bool& slow) {
     constexpr uint32_t kSize = sizeof(PlaneT<kWide>);
-    const uint32_t k = tk & 0x3Fu, k1 = k + 1u;
-    const bool eg = (tk & 0x80u) != 0u;
-    const uint32_t em = eg ? 2u : 1u, zmul = eg ? 0u : 1u << k, pow = 1u << k;
-    uint32_t l0 = 0u, l1 = 0u;
+    const TeamCode C(tk);
+    const uint32_t base = smem_addr(w);
+    uint32_t l[kN / 4u];
     if constexpr (!kDown) {
-        l0 = reinterpret_cast<const uint32_t*>(list)[0];
-        l1 = reinterpret_cast<const uint32_t*>(list)[1];
-    }
-    uint32_t from = b.at(), u[8];
-    bool longc = false, ok = true;
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-        const uint32_t z = __clz(b.hi);
-        const uint32_t len = z * em + k1;
-        longc = longc | ((i < n) & (len > 32u));
-        // the value bits with the terminator as their leading one: 2^nb + value
-        u[i] = z * zmul + ((b.hi >> ((32u - len) & 31u)) - pow);
-        b.skip(i < n ? min(len, 32u) : 0u);
+        for (uint32_t q = 0; q < kN / 4u; q++) l[q] = reinterpret_cast<const uint32_t*>(list)[q];
     }
-    if (longc) {
+    uint32_t from = pos, big = 0u;
+    bool far = false;
+    auto put = [&](int i, uint32_t u, bool on) {
+        uint32_t v;
+        if constexpr (kDown) {
+            v = on ? list[-i] : 0u;
+        } else {
+            v = __byte_perm(l[i / 4], 0u, 0x4440u | (i & 3));
+        }
+        const uint32_t at = mad_u32(v, kSize, plane), act = static_cast<uint32_t>(on);
+        const int32_t r = unzigzag(u);
+        if constexpr (kWide) {
+            asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %2, 0;\n@p st.shared.u32 [%0], %1;\n}" ::"r"(at), "r"(r), "r"(act)
+                         : "memory");
+        } else {
+            asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %2, 0;\n@p st.shared.u16 [%0], %1;\n}" ::"r"(at),
+                         "h"(static_cast<short>(r)), "r"(act)
+                         : "memory");
+            big |= on ? u : 0u;
+        }
+    };
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-            if (i < n) {
-                int32_t r;
-                ok = residual<true>(b.w, 0u, from, tk, limit, r) & ok;
-                u[i] = (static_cast<uint32_t>(r) << 1) ^ static_cast<uint32_t>(r >> 31);
+    for (int h = 0; h < static_cast<int>(kN); h += 4) {
+        uint32_t u[4];
+        far = team_four(base, pos, C, n - h, u) | far;
+#pragma unroll
+        for (int i = 0; i < 4; i++) put(h + i, u[i], store & (h + i < n));
+    }
+    bool ok = true;
+    if (far) {  // (what was put is put again)
+        big = 0u;
+        for (int i = 0; i < min(static_cast<int>(kN), n); i++) {
+            int32_t r;
+            ok = residual<true>(w, 0u, from, tk, limit, r) & ok;
+            const uint32_t u = (static_cast<uint32_t>(r) << 1) ^ static_cast<uint32_t>(r >> 31);
+            if (store) {
+                const uint32_t v = kDown ? list[-i] : list[i];
+                reinterpret_cast<PlaneT<kWide>*>(__cvta_shared_to_generic(plane))[v] = static_cast<PlaneT<kWide>>(r);
+                big |= u;
             }
         }
-        b.seek(from);
+        pos = from;
     }
-    uint32_t big = 0u;
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        const bool on = store & (i < n);
-        const uint32_t v = kDown ? (on ? list[-i] : 0u) : __byte_perm(i < 4 ? l0 : l1, 0u, 0x4440u | (i & 3));
-        const uint32_t at = mad_u32(v, kSize, plane);
-        if (on) {
-            const int32_t r = unzigzag(u[i]);
-            if constexpr (kWide) {
-                asm volatile("st.shared.u32 [%0], %1;" ::"r"(at), "r"(r) : "memory");
-            } else {
-                asm volatile("st.shared.u16 [%0], %1;" ::"r"(at), "h"(static_cast<short>(r)) : "memory");
-                big |= u[i];
-            }
-        }
-    }
-    slow = slow | (big > 0xFFFFu);  // outside 16 bits
-    if (b.at() > limit) {
-        b.seek(limit);
-        ok = false;
-    }
+    slow = slow | (!kWide && big > 0xFFFFu);  // outside 16 bits
+    ok = ok & (pos <= limit);
+    pos = min(pos, limit);
     return ok;
 }
 
@@ -285,8 +336,9 @@ __device__ __forceinline__ bool team_decode(BitBuf<true>& b, uint32_t tk, uint32
 // plane's addresses are formed for all eight entries first, with multiply-adds
 // (the integer ALU, which issues every other cycle, has the byte extractions),
 // so that only loads, arithmetic and the store are between one code and the
-// next: 86 cycles an entry on one warp against 143 with the addresses where
-// they are used.
+// next, and an entry's codes are loaded before the one before it is stored and
+// taken from its register where they are that one: 59 cycles an entry on one
+// warp, 86 through shared memory, 143 with the addresses where they are used.
 template <bool kWide>
 __device__ __forceinline__ void team_predict(uint32_t plane, const uint32_t* __restrict__ walk, uint32_t h,
                                              uint32_t n_walk, int32_t n0, int32_t n1, int32_t n2, int32_t K,
@@ -303,32 +355,53 @@ __device__ __forceinline__ void team_predict(uint32_t plane, const uint32_t* __r
         ac[i] = mad_u32(e >> 24, kSize, plane);
         para[i] = av[i] != aa[i];  // roots are stored as (v, v, v, v)
     }
+    auto ld = [](uint32_t at) -> int32_t {  // a code
+        int32_t c;
+        if constexpr (kWide) {
+            asm volatile("ld.shared.s32 %0, [%1];" : "=r"(c) : "r"(at) : "memory");
+        } else {
+            asm volatile("ld.shared.u16 %0, [%1];" : "=r"(c) : "r"(at) : "memory");
+        }
+        return c;
+    };
+    int32_t r[8];
 #pragma unroll
     for (uint32_t i = 0; i < 8u; i++) {
-        const bool act = h + i < n_walk;
-        int32_t r, ca, cb, cc;
         if constexpr (kWide) {
-            asm volatile("ld.shared.s32 %0, [%1];" : "=r"(r) : "r"(av[i]) : "memory");
-            asm volatile("ld.shared.s32 %0, [%1];" : "=r"(ca) : "r"(aa[i]) : "memory");
-            asm volatile("ld.shared.s32 %0, [%1];" : "=r"(cb) : "r"(ab[i]) : "memory");
-            asm volatile("ld.shared.s32 %0, [%1];" : "=r"(cc) : "r"(ac[i]) : "memory");
+            asm volatile("ld.shared.s32 %0, [%1];" : "=r"(r[i]) : "r"(av[i]) : "memory");
         } else {
-            asm volatile("ld.shared.s16 %0, [%1];" : "=r"(r) : "r"(av[i]) : "memory");
-            asm volatile("ld.shared.u16 %0, [%1];" : "=r"(ca) : "r"(aa[i]) : "memory");
-            asm volatile("ld.shared.u16 %0, [%1];" : "=r"(cb) : "r"(ab[i]) : "memory");
-            asm volatile("ld.shared.u16 %0, [%1];" : "=r"(cc) : "r"(ac[i]) : "memory");
-            if (i == 0u) r = h == 0u ? r & 0xFFFF : r;  // the first entry is the anchor, a code
+            asm volatile("ld.shared.s16 %0, [%1];" : "=r"(r[i]) : "r"(av[i]) : "memory");
+            if (i == 0u) r[i] = h == 0u ? r[i] & 0xFFFF : r[i];  // the first entry is the anchor, a code
         }
-        const int32_t code = (para[i] ? (n0 * ca + n1 * cb + n2 * cc + half) >> K : prev) + r;
-        if (act) {
-            if constexpr (kWide) {
-                asm volatile("st.shared.u32 [%0], %1;" ::"r"(av[i]), "r"(code) : "memory");
-            } else {
-                asm volatile("st.shared.u16 [%0], %1;" ::"r"(av[i]), "h"(static_cast<short>(code)) : "memory");
-            }
-            codes |= static_cast<uint32_t>(code);
+    }
+    int32_t ca = ld(aa[0]), cb = ld(ab[0]), cc = ld(ac[0]);
+#pragma unroll
+    for (uint32_t i = 0; i < 8u; i++) {
+        const uint32_t act = static_cast<uint32_t>(h + i < n_walk);
+        int32_t na = 0, nb = 0, nc = 0;
+        if (i < 7u) {
+            na = ld(aa[i + 1u]);
+            nb = ld(ab[i + 1u]);
+            nc = ld(ac[i + 1u]);
         }
+        const int32_t code = (para[i] ? (n0 * ca + n1 * cb + n2 * cc + half) >> K : prev) + r[i];
+        if constexpr (kWide) {
+            asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %2, 0;\n@p st.shared.u32 [%0], %1;\n}" ::"r"(av[i]), "r"(code),
+                         "r"(act)
+                         : "memory");
+        } else {
+            asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %2, 0;\n@p st.shared.u16 [%0], %1;\n}" ::"r"(av[i]),
+                         "h"(static_cast<short>(code)), "r"(act)
+                         : "memory");
+        }
+        codes |= act ? static_cast<uint32_t>(code) : 0u;
         prev = code;
+        if (i < 7u) {
+            const int32_t kept = kWide ? code : code & 0xFFFF;  // as the plane keeps it
+            ca = aa[i + 1u] == av[i] ? kept : na;
+            cb = ab[i + 1u] == av[i] ? kept : nb;
+            cc = ac[i + 1u] == av[i] ? kept : nc;
+        }
     }
 }
 
@@ -477,11 +550,9 @@ __device__ __forceinline__ void team_round(const DecodeArgs& a, TeamShared<M>& s
         w = kShared ? bit_words : reinterpret_cast<const uint32_t*>(a.arena + F.P.blob_off);
         return kShared ? static_cast<uint32_t>((F.P.blob_off - F.src16 + F.bit_off) * 8ull) : 0u;
     };
-    // Output rows of the warp's meshlet, once the scan has ended: inside its
-    // mesh's (header n_v_total, n_t), and the last meshlet's end exactly there
+    // Output rows of a meshlet, once the scan has ended: inside its mesh's (header n_v_total, n_t), and the last meshlet's end exactly there
     // (see placement_ok).
     auto place = [&](TeamFacts& F) {
-        asm volatile("griddepcontrol.wait;" ::: "memory");
         if (lane == 0) {
             const MeshletDesc* D = a.descs + F.m;
             const BlockPrefix* bp = a.blk_prefix + F.m / kScanThreads;
@@ -496,7 +567,6 @@ __device__ __forceinline__ void team_round(const DecodeArgs& a, TeamShared<M>& s
         }
         __syncwarp();
     };
-    bool placed = false;
     for (uint32_t pass = 0; pass < 2u; pass++) {  // the second one with the exact FIFO, rarely
         const bool exact = pass != 0u;
         if (threadIdx.x == 0) s.redo = 0u;
@@ -561,18 +631,18 @@ __device__ __forceinline__ void team_round(const DecodeArgs& a, TeamShared<M>& s
             for (uint32_t q = 0; q < kPer; q++) {
                 const uint32_t j = aw0 + q * kTeamAsm;
                 if (j >= M || !((rmask >> j) & 1u)) continue;
-                uint4* last = reinterpret_cast<uint4*>(uni + s.f[j].asm_off);
+                uint4* last = reinterpret_cast<uint4*>(uni + s.f[j].last_off);
                 last[lane] = last[lane + 32] = make_uint4(0u, 0u, 0u, 0u);
             }
             __syncwarp();
             // the windows that the records fill (or end)
             auto windows = [&](TeamAsm& A, const TeamFacts& F) {
                 uint32_t* walk = walks + F.walk_off;
-                uint32_t* last = uni + F.asm_off;
+                uint32_t* last = uni + F.last_off;
                 const uint32_t have = A.t >= F.n_tok ? F.n_tok + 31u : A.t;
                 for (; A.t0 + 32u <= have; A.t0 += 32u)
                     team_window<true>(A, F, 0u, exact, A.t0, reinterpret_cast<const uint16_t*>(uni + F.tok_off) + 2, walk,
-                                reinterpret_cast<uint8_t*>(walk + F.n_local), last, last + 256, lane);
+                                reinterpret_cast<uint8_t*>(walk + F.n_local), last, uni + F.tri_off, lane);
             };
             auto chunk = [&](uint32_t c) {
 #pragma unroll
@@ -610,16 +680,10 @@ __device__ __forceinline__ void team_round(const DecodeArgs& a, TeamShared<M>& s
                 const uint32_t j = aw0 + q * kTeamAsm;
                 if (j >= M || !((rmask >> j) & 1u)) continue;
                 TeamFacts& F = s.f[j];
-                if (!placed) place(F);
-                // triangle indices are relative to the mesh's first vertex
-                const uint32_t vloc = static_cast<uint32_t>(F.v_base - F.P.v_offset);
-                if (F.placed)
-                    team_triangles(a.idx + 3ull * F.t_base, uni + F.asm_off + 256,
-                                   static_cast<uint32_t>(F.t_base) & 3u, min(S[q].tcnt, F.n_tris),
-                                   [&](uint32_t v) { return vloc + v; }, lane);
-                const bool bad = __any_sync(kFull, S[q].out) || S[q].tcnt != F.n_tris || !F.placed;
+                const bool bad = __any_sync(kFull, S[q].out) || S[q].tcnt != F.n_tris;
                 if (lane == 0) {
                     F.walk = S[q].kind0 | (min(S[q].wcnt, F.n_local) << 16);
+                    F.tcnt = min(S[q].tcnt, F.n_tris);
                     if (bad) atomicOr(&F.bad, 1u);
                     if (S[q].redo && !exact) s.redo = 1u;
                 }
@@ -628,7 +692,6 @@ __device__ __forceinline__ void team_round(const DecodeArgs& a, TeamShared<M>& s
         __syncthreads();
         asm volatile("griddepcontrol.wait;" ::: "memory");
         if (threadIdx.x < M && ((rmask >> threadIdx.x) & 1u)) a.descs[s.f[threadIdx.x].m].anchor_bit = s.f[threadIdx.x].anchor;
-        placed = true;
         if (s.redo == 0u || exact) break;
         __syncthreads();  // everyone has read it
     }
@@ -666,9 +729,7 @@ __device__ __forceinline__ void team_round(const DecodeArgs& a, TeamShared<M>& s
             const uint32_t limit = on ? F.end_bit + rbase : 0u;
             TeamAxis X;
             team_axis_open<kShared>(X, &P, d, on, F.anchor, F.end_bit, wk, w, rbase);
-            BitBuf<true> b;
-            b.w = w;
-            b.end_word = 0u;
+            uint32_t pos = 0u;
             const uint32_t plane_addr = smem_addr(plane);
             bool run = kShared && !X.bad;
             if constexpr (kShared) {
@@ -676,19 +737,18 @@ __device__ __forceinline__ void team_round(const DecodeArgs& a, TeamShared<M>& s
                 // parallelogram substreams before its own
                 const uint32_t nd = run ? X.n_delta : 0u;
                 const uint32_t most = __reduce_max_sync(kFull, nd);
-                b.seek(run ? X.pos0 : 0u);
+                pos = run ? X.pos0 : 0u;
 #pragma unroll
                 for (uint32_t e = 0; e < 3u; e++) {
-                    X.cdd = e == d ? b.at() : X.cdd;
+                    X.cdd = e == d ? pos : X.cdd;
 #pragma unroll 1
                     for (uint32_t i = 0; i < most; i += 8u) {
-                        run = team_decode<kWide, true>(b, X.tk[e], limit, vlist + nl - 2u - i,
+                        run = team_decode<8u, kWide, true>(w, pos, X.tk[e], limit, vlist + nl - 2u - i,
                                                        run ? static_cast<int>(nd) - static_cast<int>(i) : 0, e == d,
                                                        plane_addr, X.slow) & run;
                         __syncwarp();
                     }
                 }
-                uint32_t pos = b.at();
 #pragma unroll
                 for (uint32_t e = 0; e < 2u; e++) {
                     run = team_skip(w, pos, X.tk[3 + e], run && e < d ? X.n_para : 0u, limit) & run;
@@ -698,28 +758,24 @@ __device__ __forceinline__ void team_round(const DecodeArgs& a, TeamShared<M>& s
                 run = run && n_walk;
                 if (run) plane[vlist[nl - 1u]] = static_cast<PlaneT<kWide>>(X.anc);  // the first root is the anchor
                 X.bad = X.bad || (n_walk && !run);
-                b.seek(run ? X.cp : 0u);
+                pos = run ? X.cp : 0u;
             }
             const uint32_t np = run ? X.n_para : 0u;
             for (uint32_t c = 0; c <= chunks; c++) {
                 if constexpr (kShared) {
                     if (c < chunks) {
                         const uint32_t i0 = c * kTeamRes;
-#pragma unroll 1
-                        for (uint32_t h = 0; h < kTeamRes; h += 8u) {
-                            if (!team_decode<kWide, false>(b, X.tp, limit, vlist + i0 + h,
-                                                           static_cast<int>(np) - static_cast<int>(i0 + h), true,
-                                                           plane_addr, X.slow))
-                                X.bad = true;
-                            __syncwarp();
-                        }
+                        if (!team_decode<kTeamRes, kWide, false>(w, pos, X.tp, limit, vlist + i0,
+                                                                 static_cast<int>(np) - static_cast<int>(i0), true,
+                                                                 plane_addr, X.slow))
+                            X.bad = true;
                     }
                 }
                 if (c == chunks && on) F.slow[d] = X.slow ? 1u : 0u;
                 __syncwarp();
                 team_dec_bar(k);
             }
-            uint32_t cend = run ? b.at() : X.cp;
+            uint32_t cend = run ? pos : X.cp;
             team_dec_bar(k);  // the predictor has left the planes
             if (on && X.slow) {
                 TeamAxis Y = X;  // a copy: only this path keeps it in memory
@@ -762,6 +818,19 @@ __device__ __forceinline__ void team_round(const DecodeArgs& a, TeamShared<M>& s
             __syncwarp();
             team_dec_bar(k);
         }
+    } else {
+        // beside it the other warps: the rows that the scan gave the meshlets,
+        // and the triangles
+        for (uint32_t j = warp - 2u * kDec; j < M; j += kTeamAsm + 2u - 2u * kDec) {
+            if (!((rmask >> j) & 1u)) continue;
+            TeamFacts& F = s.f[j];
+            place(F);
+            // triangle indices are relative to the mesh's first vertex
+            const uint32_t vloc = static_cast<uint32_t>(F.v_base - F.P.v_offset);
+            if (F.placed)
+                team_triangles(a.idx + 3ull * F.t_base, uni + F.tri_off, static_cast<uint32_t>(F.t_base) & 3u, F.tcnt,
+                               [&](uint32_t v) { return vloc + v; }, lane);
+        }
     }
     __syncthreads();
     // 4. emit
@@ -769,7 +838,7 @@ __device__ __forceinline__ void team_round(const DecodeArgs& a, TeamShared<M>& s
         for (uint32_t j = aw0; j < M; j += kTeamAsm) {
             const TeamFacts& F = s.f[j];
             if (!((rmask >> j) & 1u)) continue;
-            if (F.bad | F.wbad) {
+            if (F.bad | F.wbad | (F.placed ^ 1u)) {
                 if (lane == 0) report(a.status, kErrCorrupt, F.m);
                 continue;
             }
@@ -789,7 +858,7 @@ __global__ void __launch_bounds__(kTeamThreads, 2) team_kernel(DecodeArgs a, uin
         s.masks[threadIdx.x] = threadIdx.x < 16u ? mtf_mask_row(threadIdx.x) : make_uint4(0u, 0u, 0u, 0u);
     const uint32_t warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
-    uint32_t todo = 0u, nb = 0u, nw = 0u, nt = 0u, na = 0u, np = 0u;
+    uint32_t todo = 0u, nb = 0u, nw = 0u, nt = 0u, nr = 0u, np = 0u;
     if (warp == 0u) {
         bool ok = false;
         if (static_cast<uint32_t>(lane) < M) {
@@ -821,7 +890,7 @@ __global__ void __launch_bounds__(kTeamThreads, 2) team_kernel(DecodeArgs a, uin
             nb = F.ssz + ((F.ssz & 16u) ? 0u : 16u);
             nw = team_walk_words(F.n_local);
             nt = team_tok_words(F.n_tok);
-            na = team_asm_words(F.n_tris);
+            nr = (F.n_tris + 3u) & ~3u;
             np = 3u * F.axis_words;
         }
         todo = __ballot_sync(kFull, ok);
@@ -829,22 +898,23 @@ __global__ void __launch_bounds__(kTeamThreads, 2) team_kernel(DecodeArgs a, uin
     for (;;) {  // rounds of as many meshlets as fit, in slot order (nearly always one)
         if (warp == 0u) {
             const bool in = (todo >> lane) & 1u;
-            uint32_t cb = in ? nb : 0u, cw = in ? nw : 0u, ct = in ? nt : 0u, ca = in ? na : 0u, cp = in ? np : 0u;
+            uint32_t cb = in ? nb : 0u, cw = in ? nw : 0u, ct = in ? nt : 0u, cr = in ? nr : 0u, cp = in ? np : 0u;
+            const uint32_t cl = 256u * __popc(todo & ((2u << lane) - 1u));
 #pragma unroll
             for (uint32_t o = 1; o < M; o <<= 1) {
                 const uint32_t t0 = __shfl_up_sync(kFull, cb, o), t1 = __shfl_up_sync(kFull, cw, o);
-                const uint32_t t2 = __shfl_up_sync(kFull, ct, o), t3 = __shfl_up_sync(kFull, ca, o);
+                const uint32_t t2 = __shfl_up_sync(kFull, ct, o), t3 = __shfl_up_sync(kFull, cr, o);
                 const uint32_t t4 = __shfl_up_sync(kFull, cp, o);
                 if (static_cast<uint32_t>(lane) >= o) {
                     cb += t0;
                     cw += t1;
                     ct += t2;
-                    ca += t3;
+                    cr += t3;
                     cp += t4;
                 }
             }
-            // (six words: alignments)
-            const bool fit = in && team_bytes(cb, cw, ct, ca, cp) + 24u <= smem_bytes;
+            // (ten words: alignments)
+            const bool fit = in && team_bytes(cb, cw, ct, cl, cp, cr) + 40u <= smem_bytes;
             uint32_t rmask = __ballot_sync(kFull, fit);
             const bool staged = rmask != 0u;
             // one meshlet whose bytes exceed the stage: read in place
@@ -853,17 +923,20 @@ __global__ void __launch_bounds__(kTeamThreads, 2) team_kernel(DecodeArgs a, uin
             const int end = rmask ? 31 - __clz(rmask) : 0;  // the round's last meshlet
             const uint32_t walk_base = staged ? __shfl_sync(kFull, cb, end) : 0u;
             const uint32_t tw = staged ? __shfl_sync(kFull, cw, end) : 0u, tt = staged ? __shfl_sync(kFull, ct, end) : 0u;
-            // the words after the walks and after the records start on 16 bytes
+            const uint32_t tp = staged ? __shfl_sync(kFull, cp, end) : 0u, tl = staged ? __shfl_sync(kFull, cl, end) : 0u;
+            // the words after the walks, the records and the planes start on 16 bytes
             const uint32_t uni_base = staged ? (walk_base + 4u * tw + 15u) & ~15u : 0u;
-            const uint32_t asm_base = (tt + 3u) & ~3u;
+            const uint32_t last_base = (tt + 3u) & ~3u;
+            const uint32_t tri_base = max(last_base + tl, (tp + 3u) & ~3u);
             const bool mine = (rmask >> lane) & 1u;
             if (mine) {
                 TeamFacts& F = s.f[lane];
                 F.bit_off = staged ? cb - nb : 0u;
                 F.walk_off = staged ? cw - nw : 0u;
                 F.tok_off = staged ? ct - nt : 0u;
-                F.asm_off = staged ? asm_base + ca - na : (nt + 3u) & ~3u;
+                F.last_off = staged ? last_base + cl - 256u : (nt + 3u) & ~3u;
                 F.plane_off = staged ? cp - np : 0u;
+                F.tri_off = staged ? tri_base + cr - nr : max(F.last_off + 256u, (np + 3u) & ~3u);
                 if (!staged) {
                     s.walk_base = 0u;
                     s.uni_base = (4u * nw + 15u) & ~15u;
@@ -905,9 +978,9 @@ uint32_t team_smem(const DecodeArgs& a, uint32_t m, bool wide) {
     const uint32_t by = (avg(a.hint_bytes, 1024u) + 63u) & ~31u;
     const uint32_t nv = std::min(avg(a.hint_v, 256u) + 4u, 256u), nt = std::min(avg(a.hint_t, 256u) + 8u, 256u);
     const uint32_t b = team_bytes(m * by, m * team_walk_words(nv), m * team_tok_words(nt + nt / 12u),
-                                  m * team_asm_words(nt), m * 3u * team_axis_words(nv, size)) + 32u;
-    const uint32_t least = team_bytes(0u, team_walk_words(256u), team_tok_words(kTeamTokens), team_asm_words(256u),
-                                      3u * team_axis_words(256u, size)) + 32u;
+                                  m * 256u, m * 3u * team_axis_words(nv, size), m * ((nt + 3u) & ~3u)) + 48u;
+    const uint32_t least = team_bytes(0u, team_walk_words(256u), team_tok_words(kTeamTokens), 256u,
+                                      3u * team_axis_words(256u, size), 256u) + 48u;
     return (std::max(b, least) + 15u) & ~15u;
 }
 

@@ -41,48 +41,6 @@ __device__ __forceinline__ void team_all_bar() {  // every warp, from its own lo
     asm volatile("bar.sync 4, %0;" ::"n"(kThreads) : "memory");
 }
 
-// A lane's next bits in registers: hi | mid | lo hold `cnt` (65..96) bits, the
-// next one the MSB of hi; nxt is the word after them.  Consuming bits is
-// three shifts, and neither the refill nor its load is on the chain from one
-// token or codeword to the next (branch-free: a taken branch costs a lone
-// warp about 20 cycles).
-template <bool kShared>
-struct BitBuf {
-    const uint32_t* w;
-    uint32_t hi, mid, lo, nxt, cnt, wi;  // wi: index of nxt
-    uint32_t end_word;                   // global reads stop here (a staged lane's overrun stays in shared memory)
-
-    __device__ __forceinline__ uint32_t load(uint32_t i) const {
-        return (kShared || i < end_word) ? ldw<kShared>(w, i) : 0u;
-    }
-    // at bit q of w
-    __device__ __forceinline__ void seek(uint32_t q) {
-        const uint32_t i = q >> 5, o = q & 31u;
-        const uint32_t a = load(i), b = load(i + 1u), c = load(i + 2u);
-        wi = i + 3u;
-        nxt = load(wi);
-        hi = __funnelshift_l(b, a, o);
-        mid = __funnelshift_l(c, b, o);
-        lo = c << o;
-        cnt = 96u - o;
-    }
-    __device__ __forceinline__ uint32_t at() const { return 32u * wi - cnt; }
-    // n <= 32
-    __device__ __forceinline__ void skip(uint32_t n) {
-        hi = __funnelshift_lc(mid, hi, n);
-        mid = __funnelshift_lc(lo, mid, n);
-        lo = __funnelshift_lc(0u, lo, n);
-        cnt -= n;
-        const bool refill = cnt <= 64u;  // lo is used up, mid holds cnt - 32 bits
-        const uint32_t t = __funnelshift_rc(nxt, 0u, cnt - 32u);
-        mid |= refill ? t : 0u;
-        lo = refill ? nxt << ((64u - cnt) & 31u) : lo;
-        cnt += refill ? 32u : 0u;
-        wi += refill ? 1u : 0u;
-        nxt = load(wi);
-    }
-};
-
 // a * b + c on the multiplier, which leaves the integer ALU to the rest.
 __device__ __forceinline__ uint32_t mad_u32(uint32_t a, uint32_t b, uint32_t c) {
     uint32_t d;
