@@ -508,32 +508,6 @@ __device__ __forceinline__ bool skip_codes(const uint32_t* w, uint32_t rbase, ui
     return ok;
 }
 
-// The same codeword read without a branch, for codewords that fit the
-// 32-bit window (prefix, terminator and value); a longer one sets `longc`
-// and leaves the result undefined.  The walk uses this form so that the
-// compiler can overlap consecutive walk entries (a branch per entry keeps
-// them apart: 5% of the fused kernel on the 2049^2 heightfield).
-template <bool kShared>
-__device__ __forceinline__ bool residual_fast(const uint32_t* w, uint32_t rbase, uint32_t& pos, uint32_t tk,
-                                              uint32_t limit, int32_t& r, bool& longc) {
-    const uint32_t x = peek32<kShared>(w, pos + rbase);
-    const uint32_t z = __clz(x);
-    const uint32_t k = tk & 0x3Fu;
-    const bool eg = (tk & 0x80u) != 0u;
-    const uint32_t nb = (eg ? z : 0u) + k;
-    const uint32_t len = z + 1u + nb;
-    const uint32_t t = __funnelshift_lc(0u, x, z + 1u);
-    const uint32_t val = __funnelshift_rc(t, 0u, 32u - nb);
-    const uint32_t base = eg ? ((1u << (z & 31u)) - 1u) : z;
-    const uint32_t u = (base << k) + val;
-    const uint32_t np = pos + len;
-    longc = longc | (len > 32u);
-    const bool ok = np <= limit;
-    pos = min(np, limit);
-    r = unzigzag(u);
-    return ok;
-}
-
 // Axis d of every vertex of the round's meshlets -> positions (and codes),
 // the warp working through one meshlet at a time (n_local <= kMaxLocal, so
 // a meshlet's table reads all go out before its first store: one L2 round

@@ -40,6 +40,7 @@
 #include "stride_common.cuh"
 #include "stride_device.cuh"
 #include "stride_gb300.h"
+#include "stride_team.cuh"
 
 namespace stride {
 namespace {
@@ -651,90 +652,171 @@ __device__ __forceinline__ uint32_t vert_header(const GroupLane& L, uint32_t d, 
 }
 
 // Integer codes of axis d in walk order (IRLP, paradelta_v5_dup.py:91-104
-// and 581-600).  Every walk vertex is a root (delta from the previous walk
-// vertex; the first one is the anchor) or a parallelogram vertex predicted
-// from three earlier ones.  Four walk entries per iteration (one 16-byte
-// load); entries past the end are masked, not branched around, and root and
-// parallelogram vertices differ only in selects.  The walk reads codewords
-// with the branch-free reader; a lane that met a codeword longer than its
-// window walks its axis again with the general reader (every plane entry
-// the walk reaches is written again, in the same order).
+// and 581-600), by the general reader: meshlets read in place, and lanes that
+// met a codeword longer than a window.  Every walk vertex is a root (delta from
+// the previous walk vertex; the first one is the anchor) or a parallelogram
+// vertex predicted from three earlier ones.
+// Returns the parallelogram cursor, and 2^32 when all was valid.
+template <bool kShared, bool kWide>
+__device__ __noinline__ unsigned long long vert_axis_general(const uint32_t* walk, uint32_t n_walk, const MeshParams* P,
+                                                             uint32_t d, const uint32_t* w, uint32_t rbase, uint32_t end,
+                                                             PlaneT<kWide>* plane, uint32_t cdd, uint32_t cp, uint32_t td,
+                                                             uint32_t tp, int32_t anc) {
+    const int32_t n0 = P->pred_n[3 * d], n1 = P->pred_n[3 * d + 1], n2 = P->pred_n[3 * d + 2];
+    const int32_t K = P->pred_k[d], half = P->pred_half[d];
+    const uint32_t cmax = P->code_max[d];
+    int32_t prev = anc;
+    bool ok = true;
+    auto step = [&](uint32_t e, uint32_t i) {
+        if (i >= n_walk) return;
+        const uint32_t v = e & 0xFFu, ra = (e >> 8) & 0xFFu;
+        const bool para = ra != v;  // roots are stored as (v, v, v, v)
+        int32_t code = prev;
+        if (i) {
+            uint32_t p = para ? cp : cdd;
+            int32_t r;
+            ok = residual<kShared>(w, rbase, p, para ? tp : td, end, r) & ok;
+            cp = para ? p : cp;
+            cdd = para ? cdd : p;
+            const int32_t ca = static_cast<int32_t>(plane[ra]), cb = static_cast<int32_t>(plane[(e >> 16) & 0xFFu]),
+                          cc = static_cast<int32_t>(plane[e >> 24]);
+            code = (para ? (n0 * ca + n1 * cb + n2 * cc + half) >> K : prev) + r;
+        }
+        ok = ok & (static_cast<uint32_t>(code) <= cmax);  // codes of a valid stream lie in [0, 2^g_bits)
+        plane[v] = static_cast<PlaneT<kWide>>(code);
+        prev = code;
+    };
+    const uint4* wq = reinterpret_cast<const uint4*>(walk);
+    uint4 qn = n_walk ? __ldcg(wq) : make_uint4(0u, 0u, 0u, 0u);
+    uint4 qm = n_walk > 4u ? __ldcg(wq + 1) : qn;
+    for (uint32_t i = 0; i < n_walk; i += 4u) {
+        const uint4 q = qn;
+        qn = qm;
+        if (i + 8u < n_walk) qm = __ldcg(wq + (i >> 2) + 2u);
+        step(q.x, i);
+        step(q.y, i + 1u);
+        step(q.z, i + 2u);
+        step(q.w, i + 3u);
+    }
+    return (ok ? 1ull << 32 : 0ull) | cp;
+}
+
+// The same from the stage, four walk entries per iteration (one 16-byte load).
+// Bound by the integer ALU, one instruction in two cycles: entries past the end
+// are masked, not branched around; a codeword is read by the same multiply-adds
+// whatever its tag, roots and parallelogram vertices differ in selects of their
+// factors; addresses are multiply-adds; ends and code ranges are checked after
+// the entries, by the cursors and the bits of all codes (fused kernel, 12-bit
+// heightfields of 21,307 and 43,086 meshlets: 179 -> 167 and 265 -> 251 us; vertex
+// kernel beside the connectivity kernel, 14-bit sphere of 6,719: both 155 -> 125).
+// A lane that met a codeword longer than its window walks its axis again by the
+// general reader (every plane entry the walk reaches is written again, in the
+// same order).
 template <bool kShared, bool kWide>
 __device__ __forceinline__ void vert_axis(const DecodeArgs& a, const GroupLane& L, uint32_t d,
                                           const uint32_t* __restrict__ w, uint32_t rbase,
                                           PlaneT<kWide>* __restrict__ plane, VertLane& S) {
     const uint32_t n_local = L.d.counts0 & 0xFFFFu;
     const uint32_t n_walk = L.d.walk >> 16;
-    const uint32_t end = L.d.end_bit;
-    const MeshParams* P = L.P;
     if (n_walk < n_local) {  // vertices the walk never reaches keep code 0
         uint32_t* z = reinterpret_cast<uint32_t*>(plane);
         const uint32_t nz = (n_local * static_cast<uint32_t>(sizeof(PlaneT<kWide>)) + 3u) >> 2;
         for (uint32_t i = 0; i < nz; i++) z[i] = 0u;
     }
-    const int32_t n0 = P->pred_n[3 * d], n1 = P->pred_n[3 * d + 1], n2 = P->pred_n[3 * d + 2];
-    const int32_t K = P->pred_k[d], half = P->pred_half[d];
-    const uint32_t cmax = P->code_max[d];
-    const uint32_t td = S.td, tp = S.tp;
-    const int32_t anc = S.anc;
-    uint32_t cdd = S.cdd, cp = S.cp;
-    int32_t prev = 0;
-    bool fail = false;
-    bool longc = false, fast = true;
-    auto step = [&](uint32_t e, bool valid, bool anchor) {
-        e = valid ? e : 0u;  // a masked entry reads plane[0] and commits nothing
-        const uint32_t v = e & 0xFFu;
-        const uint32_t ra = (e >> 8) & 0xFFu, rb = (e >> 16) & 0xFFu, rc = e >> 24;
-        const bool para = ra != v;  // roots are stored as (v, v, v, v)
-        const int32_t ca = static_cast<int32_t>(plane[ra]);
-        const int32_t cb = static_cast<int32_t>(plane[rb]);
-        const int32_t cc = static_cast<int32_t>(plane[rc]);
-        const int32_t pred = para ? (n0 * ca + n1 * cb + n2 * cc + half) >> K : prev;
-        uint32_t p = para ? cp : cdd;
-        int32_t r;
-        const bool okr = fast ? residual_fast<kShared>(w, rbase, p, para ? tp : td, end, r, longc)
-                              : residual<kShared>(w, rbase, p, para ? tp : td, end, r);
-        const bool commit = valid & !anchor;  // the anchor has no residual
-        cp = (commit & para) ? p : cp;
-        cdd = (commit & !para) ? p : cdd;
-        const int32_t code = anchor ? anc : pred + r;
-        // codes of a valid stream lie in [0, 2^g_bits)
-        fail = fail | (valid & ((!okr & !anchor) | (static_cast<uint32_t>(code) > cmax)));
-        if (valid) plane[v] = static_cast<PlaneT<kWide>>(code);
-        prev = valid ? code : prev;
-    };
-    // walk entries (v | a << 8 | b << 16 | c << 24), 16-byte aligned per meshlet
-    const uint4* wq = reinterpret_cast<const uint4*>(a.walk_scratch + L.wp_base);
-    // two quads in flight: the walk is read from L2
-    {
+    bool again = !kShared && n_walk;
+    if constexpr (kShared) {
+        constexpr uint32_t kSize = sizeof(PlaneT<kWide>);
+        const MeshParams* P = L.P;
+        const int32_t n0 = P->pred_n[3 * d], n1 = P->pred_n[3 * d + 1], n2 = P->pred_n[3 * d + 2];
+        const int32_t K = P->pred_k[d], half = P->pred_half[d];
+        // a codeword of z leading zeros has z * em + k1 bits, its value is
+        // z * zm + (its bits - pw)
+        const uint32_t kd = S.td & 0x3Fu, kp = S.tp & 0x3Fu;
+        const uint32_t emd = (S.td & 0x80u) ? 2u : 1u, emp = (S.tp & 0x80u) ? 2u : 1u;
+        const uint32_t pwd = 1u << kd, pwp = 1u << kp;
+        const uint32_t zmd = emd == 2u ? 0u : pwd, zmp = emp == 2u ? 0u : pwp;
+        const uint32_t base = smem_addr(w), pl = smem_addr(plane);
+        const uint32_t end = L.d.end_bit + rbase;
+        uint32_t cdd = S.cdd + rbase, cp = S.cp + rbase;
+        int32_t prev = S.anc;
+        uint32_t codes = 0u, longest = 0u, over = 0u;
+        auto ld = [](uint32_t at) -> int32_t {
+            int32_t c;
+            if constexpr (kWide) {
+                asm volatile("ld.shared.s32 %0, [%1];" : "=r"(c) : "r"(at) : "memory");
+            } else {
+                asm volatile("ld.shared.u16 %0, [%1];" : "=r"(c) : "r"(at) : "memory");
+            }
+            return c;
+        };
+        auto put = [](uint32_t at, int32_t code, uint32_t on) {
+            if constexpr (kWide) {
+                asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %2, 0;\n@p st.shared.u32 [%0], %1;\n}" ::"r"(at), "r"(code),
+                             "r"(on)
+                             : "memory");
+            } else {
+                asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %2, 0;\n@p st.shared.u16 [%0], %1;\n}" ::"r"(at),
+                             "h"(static_cast<short>(code)), "r"(on)
+                             : "memory");
+            }
+        };
+        auto step = [&](uint32_t e, uint32_t i) {
+            const uint32_t in = static_cast<uint32_t>(static_cast<int32_t>(i - n_walk) >> 31);  // ones inside
+            e &= in;  // a masked entry reads plane[0] and commits nothing
+            const uint32_t av = mad_u32(__byte_perm(e, 0u, 0x4440u), kSize, pl);
+            const uint32_t aa = mad_u32(__byte_perm(e, 0u, 0x4441u), kSize, pl);
+            const uint32_t ab = mad_u32(__byte_perm(e, 0u, 0x4442u), kSize, pl);
+            const uint32_t ac = mad_u32(e >> 24, kSize, pl);
+            const bool para = av != aa;  // roots are stored as (v, v, v, v)
+            const uint32_t x = peek_shared(base, para ? cp : cdd);
+            const int32_t ca = ld(aa), cb = ld(ab), cc = ld(ac);
+            const uint32_t z = __clz(x);
+            const uint32_t len = mad_u32(z, para ? emp : emd, (para ? kp : kd) + 1u);
+            // the value bits with the terminator as their leading one: 2^nb + value
+            const uint32_t u = mad_u32(z, para ? zmp : zmd, __funnelshift_rc(x, 0u, 32u - len) - (para ? pwp : pwd));
+            const int32_t code = (para ? (n0 * ca + n1 * cb + n2 * cc + half) >> K : prev) + unzigzag(u);
+            const uint32_t adv = len & in;
+            longest = max(longest, adv);
+            cp += para ? adv : 0u;
+            cdd += para ? 0u : adv;
+            codes |= static_cast<uint32_t>(code) & in;
+            put(av, code, in);
+            prev = code;
+        };
+        // walk entries (v | a << 8 | b << 16 | c << 24), 16-byte aligned per
+        // meshlet; two quads in flight: the walk is read from L2
+        const uint4* wq = reinterpret_cast<const uint4*>(a.walk_scratch + L.wp_base);
         uint4 qn = n_walk ? __ldcg(wq) : make_uint4(0u, 0u, 0u, 0u);
         uint4 qm = n_walk > 4u ? __ldcg(wq + 1) : qn;
+        if (n_walk) {  // the anchor
+            put(mad_u32(qn.x & 0xFFu, kSize, pl), S.anc, 1u);
+            codes = static_cast<uint32_t>(S.anc);
+        }
         for (uint32_t i = 0; i < n_walk; i += 4u) {
             const uint4 q = qn;
             qn = qm;
             if (i + 8u < n_walk) qm = __ldcg(wq + (i >> 2) + 2u);
-            step(q.x, true, i == 0u);
-            step(q.y, i + 1u < n_walk, false);
-            step(q.z, i + 2u < n_walk, false);
-            step(q.w, i + 3u < n_walk, false);
+            if (i) step(q.x, i);
+            step(q.y, i + 1u);
+            step(q.z, i + 2u);
+            step(q.w, i + 3u);
+            // a corrupt lane's cursor stays within four codewords of the meshlet
+            over |= static_cast<uint32_t>(max(cp, cdd) > end);
+            cp = min(cp, end);
+            cdd = min(cdd, end);
+        }
+        again = longest > 32u;
+        if (!again) {
+            S.cp = cp - rbase;
+            S.bad = S.bad || over || (codes & ~P->code_max[d]) != 0u;
         }
     }
-    if (longc) {  // rare: the lane's axis again, from its substream starts
-        fast = false;
-        cdd = S.cdd;
-        cp = S.cp;
-        prev = 0;
-        fail = false;
-        for (uint32_t i = 0; i < n_walk; i += 4u) {
-            const uint4 q = __ldcg(wq + (i >> 2));
-            step(q.x, true, i == 0u);
-            step(q.y, i + 1u < n_walk, false);
-            step(q.z, i + 2u < n_walk, false);
-            step(q.w, i + 3u < n_walk, false);
-        }
+    if (again) {  // rare: from its substream starts
+        const unsigned long long r = vert_axis_general<kShared, kWide>(a.walk_scratch + L.wp_base, n_walk, L.P, d, w, rbase,
+                                                                       L.d.end_bit, plane, S.cdd, S.cp, S.td, S.tp, S.anc);
+        S.cp = static_cast<uint32_t>(r);
+        S.bad = S.bad || (r >> 32) == 0ull;
     }
-    S.cp = cp;
-    S.bad = S.bad || fail;
 }
 
 // One round of warp d: its active lanes find where their axis' two
