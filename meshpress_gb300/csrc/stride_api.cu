@@ -419,6 +419,8 @@ int decode_to_host(HostLink& L, const DecodeArgs& a, LaunchCfg cfg, void* stream
         cudaStreamSynchronize(s);
         cudaStreamSynchronize(L.copy[0]);
         cudaStreamSynchronize(L.copy[1]);
+        // parts may have ended half-way: the next scan finds its counter at zero
+        if (cudaMemsetAsync(a.status, 0, sizeof(Status), s) == cudaSuccess) cudaStreamSynchronize(s);
     };
     auto bail = [&](cudaError_t err, const char* what) {
         drain();
@@ -745,6 +747,7 @@ int stride_info(const stride_handle* h, stride_info_t* info) {
 static DecodeArgs handle_args(stride_handle* h, uint32_t* d_idx, float* d_pos, int32_t* d_codes) {
     DecodeArgs a;
     a.wait_clocks = h->wait_clocks;
+    a.status_kept = true;
     a.arena = h->d_blob;
     a.meshes = &h->d_fixed->params;
     a.meshlet_mesh = nullptr;

@@ -117,6 +117,7 @@ static DecodeArgs batch_args(const stride_batch* b, uint32_t* d_idx, float* d_po
     a.walk_scratch = b->d_walk_scratch;
     a.walk_cap = b->walk_cap;
     a.status = b->d_status;
+    a.status_kept = true;
     a.idx = d_idx;
     a.pos = d_pos;
     a.codes = nullptr;

@@ -132,6 +132,7 @@ struct DecodeArgs {
     uint32_t* walk_scratch;          // walk entries, 4-aligned per meshlet
     unsigned long long walk_cap;     // words in walk_scratch
     Status* status;                  // device
+    bool status_kept = false;        // zero at first, then only decodes write it: no memset before the scan
     uint32_t* idx;                   // device outputs (idx 16-byte aligned)
     float* pos;
     int32_t* codes;                  // optional

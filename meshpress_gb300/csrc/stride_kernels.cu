@@ -168,19 +168,29 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(DecodeArgs a, uint32
     const uint32_t blk = b0 + blockIdx.x;
     const uint32_t m = blk * kScanThreads + tid;
     uint32_t nl = 0u, nt = 0u;
+    int e = 0;
     MeshletDesc d;
     memset(&d, 0, sizeof(d));
     if (m < a.total_meshlets) {
         const uint32_t mi = a.meshlet_mesh ? __ldcg(a.meshlet_mesh + m) : 0u;
         const MeshParams& P = a.meshes[mi];
-        const int e = scan_meshlet(a.arena, P, m - P.meshlet_begin, d);
+        e = scan_meshlet(a.arena, P, m - P.meshlet_begin, d);
         if (e) {
-            report(a.status, e, m);
             d.counts0 = 0u;  // keeps the prefixes finite; the decode is abandoned
         } else {
             nl = d.counts0 & 0xFFFFu;
             nt = d.counts0 >> 16;
         }
+    }
+    // the block's first error goes out with its sums
+    __shared__ uint32_t s_err;
+    if (__syncthreads_or(e != 0)) {
+        if (tid == 0) s_err = 0xFFFFFFFFu;
+        __syncthreads();
+        if (e) atomicMin(&s_err, tid << 8 | static_cast<uint32_t>(e));
+        __syncthreads();
+    } else if (tid == 0) {
+        s_err = 0u;
     }
     unsigned long long t1, t2;
     const unsigned long long e1 = block_scan((static_cast<unsigned long long>(nt) << 32) | nl, wsum, t1);
@@ -215,7 +225,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(DecodeArgs a, uint32
     }
     if (tid == 0)
         a.blk_sums[blk] = make_uint4(static_cast<uint32_t>(t1), static_cast<uint32_t>(t1 >> 32),
-                                     static_cast<uint32_t>(t2), 0u);
+                                     static_cast<uint32_t>(t2), s_err);
     // The last block to finish turns the block sums into block prefixes
     // (the ticket counts the blocks of this decode's scan launches so far).
     // Only the block sum, thread 0's own write, is read inside this grid,
@@ -225,11 +235,15 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(DecodeArgs a, uint32
     __syncthreads();
     if (tid == 0) {
         __threadfence();
-        is_last = atomicAdd(&a.status->ticket, 1u) == b0 + nb - 1u;
+        // (the decode's last ticket sets the counter back to zero)
+        is_last = atomicInc(&a.status->ticket, (a.total_meshlets + kScanThreads - 1u) / kScanThreads - 1u) == b0 + nb - 1u;
     }
     __syncthreads();
     if (!is_last) return;
     __threadfence();
+    __shared__ unsigned long long s_first;  // the first block with an error, and its error
+    if (tid == 0) s_first = ~0ull;
+    __syncthreads();
     unsigned long long cv = 0ull, ct = 0ull, cw = 0ull;
     if (b0) {  // the totals of the blocks before this launch's
         const BlockPrefix* pp = a.blk_prefix + b0 - 1u;
@@ -241,6 +255,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(DecodeArgs a, uint32
     for (uint32_t base = 0; base < nb; base += kScanThreads) {
         const uint32_t i = base + tid;
         const uint4 s = i < nb ? __ldcg(a.blk_sums + b0 + i) : make_uint4(0u, 0u, 0u, 0u);
+        if (s.w) atomicMin(&s_first, static_cast<unsigned long long>(b0 + i) << 16 | s.w);
         // per-chunk sums stay below 2^32 (256 blocks x 65536), so pack pairs
         unsigned long long ta, tb;
         const unsigned long long ea = block_scan((static_cast<unsigned long long>(s.y) << 32) | s.x, wsum, ta);
@@ -256,6 +271,20 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(DecodeArgs a, uint32
         cv += ta & 0xFFFFFFFFull;
         ct += ta >> 32;
         cw += tb;
+    }
+    // The status word starts here: what the last decode left in it goes with
+    // the scan's first error, so that no memset (2 us of a small decode) comes
+    // before the scan.
+    __syncthreads();
+    if (tid != 0) return;
+    const int code = static_cast<int>(s_first & 0xFFull);
+    const uint32_t bad = static_cast<uint32_t>(s_first >> 16) * kScanThreads + static_cast<uint32_t>((s_first >> 8) & 0xFFull);
+    const bool any = s_first != ~0ull;
+    if (b0 == 0u) {
+        a.status->err = any ? (static_cast<unsigned long long>(static_cast<unsigned>(code)) << 32) | bad : 0ull;
+        a.status->work_conn = a.status->work_vert = a.status->done_tail = 0u;
+    } else if (any) {
+        report(a.status, code, bad);
     }
 }
 
@@ -1351,7 +1380,9 @@ int launch_scan(const DecodeArgs& a, cudaStream_t s, uint32_t b0, uint32_t b1, b
 int enqueue_decode(const DecodeArgs& a, const LaunchCfg& cfg, void* stream, void* const* ev) {
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (check_config(cfg, a.wide_codes)) return STRIDE_ERR_ARG;
-    if (cudaMemsetAsync(a.status, 0, sizeof(Status), s) != cudaSuccess) return STRIDE_ERR_CUDA;
+    // the scan resets a status that earlier decodes have left whole
+    if ((!a.status_kept || a.total_meshlets == 0) && cudaMemsetAsync(a.status, 0, sizeof(Status), s) != cudaSuccess)
+        return STRIDE_ERR_CUDA;
     record(ev, 0, s);
     const int rc = launch_scan(a, s, 0u, scan_blocks(a.total_meshlets), true);
     if (rc) return rc;

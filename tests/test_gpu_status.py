@@ -1,0 +1,51 @@
+"""The status word, which the scan starts anew for each decode: an error in any
+of its blocks is reported with its meshlet, and neither the error nor the
+counters of a failed decode reach the next one, in every launch shape."""
+import numpy as np
+import pytest
+
+import oracle
+from meshpress_gb300 import _lib, encoder, synth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def good():
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from meshpress_gb300 import _build
+    _build.build_decoder()
+    oracle.build()
+    V, T = synth.noise_heightfield(257, seed=3)  # 650 meshlets: three scan blocks
+    data = encoder.encode(V, T, precision_error=synth.bbox_bits_error(12), precision_mode="bbox_frac").data
+    return data, oracle.decode(data)
+
+
+@pytest.mark.parametrize("shape", [(4, 1), (4, 2), (1, 3), (2, 4)])
+def test_errors_stay_with_their_decode(good, shape):
+    from meshpress_gb300 import ParaDeltaV5GpuDecoder
+    from meshpress_gb300._lib import StrideFormatError
+    data, (opos, oidx) = good
+    n = int(np.frombuffer(data, ">u4", 1, 82)[0])
+    dec = ParaDeltaV5GpuDecoder(data)
+    cfg = _lib.LaunchCfg()
+    cfg.warps_per_cta, cfg.persistent, cfg.stage_bytes, cfg.code_bytes = *shape, 16384, 16384
+    dec.set_launch_config(cfg)
+    for k in (0, 255, 256, 300, n - 1):
+        bad = bytearray(data)
+        at = 86 + 4 * k
+        bad[at:at + 4] = (8 * len(data) if k else 8 * (86 + 4 * n) + 1).to_bytes(4, "big")
+        dec.reload(bytes(bad))
+        for _ in range(2):
+            with pytest.raises(StrideFormatError, match=rf"meshlet {k}\)"):
+                dec.decode_to_device()
+            with pytest.raises(StrideFormatError, match=rf"meshlet {k}\)"):
+                dec.check()  # what stride_finish has read
+        dec.reload(data)
+        for _ in range(2):
+            tris, verts = dec.decode_to_device()
+            assert np.array_equal(verts.cpu().numpy().view(np.uint32), opos.view(np.uint32))
+            assert np.array_equal(tris.cpu().numpy().astype(np.int64), oidx)
+    dec.close()
