@@ -22,7 +22,7 @@ constexpr uint32_t kTeamParser = 2u, kTeamFifo = 3u;
 __device__ __forceinline__ uint32_t team_asm_index(uint32_t warp) {  // 0 1 4 5 8 9 6 7 -> 0..7
     return warp < 2u ? warp : (warp < 6u ? warp - 2u : (warp < 8u ? warp : warp - 4u));
 }
-constexpr uint32_t kTeamSteps = 16u;  // parser steps between hand-overs
+constexpr uint32_t kTeamSteps = 20u;  // parser steps between hand-overs
 constexpr uint32_t kTeamTokens = 768u;  // most tokens of a meshlet: n_tris + 2 n_strips
 // Token records: bits 0..8 the nine bits after the flag (a raw token's id on
 // top, or a FIFO index in bits 4..8, replaced by the field of the id it
