@@ -612,6 +612,8 @@ int stride_device_info(int* sm_count, int* arch) {
     return STRIDE_OK;
 }
 
+static bool wide_codes(const MeshParams& p) { return p.g_bits[0] > 16 || p.g_bits[1] > 16 || p.g_bits[2] > 16; }
+
 static void fill_info(const MeshParams& p, size_t len, int persistent, stride_info_t* info) {
     std::memset(info, 0, sizeof(*info));
     info->n_meshlets = p.n_meshlets;
@@ -637,7 +639,7 @@ int stride_inspect(const uint8_t* data, size_t len, stride_info_t* info) {
     char why[256] = {0};
     const int rc = parse_header(data, len, &p, why, sizeof(why));
     if (rc) return fail(rc, "%s", why);
-    fill_info(p, len, default_config(p.n_meshlets).persistent, info);
+    fill_info(p, len, default_config(p.n_meshlets, 1u, wide_codes(p)).persistent, info);
     return STRIDE_OK;
 }
 
@@ -654,7 +656,7 @@ int stride_open(const uint8_t* data, size_t len, stride_handle** out) {
     cudaError_t e;
     rc = ensure_capacity(h, len, p);
     h->params = p;
-    h->cfg = default_config(p.n_meshlets);
+    h->cfg = default_config(p.n_meshlets, 1u, wide_codes(p));
     if (rc != STRIDE_OK) {
         free_buffers(h);
         delete h;
@@ -686,7 +688,7 @@ int stride_reload(stride_handle* h, const uint8_t* data, size_t len, void* strea
     if ((rc = ensure_capacity(h, len, p)) != STRIDE_OK) return rc;
     h->params = p;
     h->len = len;
-    if (!h->cfg_set) h->cfg = default_config(p.n_meshlets);
+    if (!h->cfg_set) h->cfg = default_config(p.n_meshlets, 1u, wide_codes(p));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     cudaError_t e;
     const size_t pad = std::min<size_t>(h->cap_bytes - len, kBlobPad);
@@ -762,7 +764,7 @@ static DecodeArgs handle_args(stride_handle* h, uint32_t* d_idx, float* d_pos, i
     a.idx = d_idx;
     a.pos = d_pos;
     a.codes = d_codes;
-    a.wide_codes = h->params.g_bits[0] > 16 || h->params.g_bits[1] > 16 || h->params.g_bits[2] > 16;
+    a.wide_codes = wide_codes(h->params);
     a.lut = h->d_lut;
     a.lut_meshes = &h->d_fixed->lut_mesh;
     a.n_lut_meshes = h->n_lut;
@@ -981,7 +983,7 @@ int stride_set_config(stride_handle* h, const stride_launch_cfg* c) {
     cfg.ctas_per_sm = c->ctas_per_sm;
     cfg.stage_bytes = c->stage_bytes;
     cfg.code_bytes = c->code_bytes;
-    const bool wide = h->params.g_bits[0] > 16 || h->params.g_bits[1] > 16 || h->params.g_bits[2] > 16;
+    const bool wide = wide_codes(h->params);
     if (check_config(cfg, wide)) return fail(STRIDE_ERR_ARG, "launch configuration not launchable");
     h->cfg = cfg;
     h->cfg_set = true;

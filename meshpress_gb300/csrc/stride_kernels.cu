@@ -1342,11 +1342,21 @@ int check_config(const LaunchCfg& cfg, bool wide) {
 //   16 per CTA          44    46    46    46    54    58    93    99   106    138
 // (14-bit spheres of 103 and 1,738 meshlets: 220 -> 48, 196 -> 52 us; 20-bit
 // heightfield of 5,221: 245 -> 96 us.)
-constexpr uint32_t kTeam4 = 700u, kTeam8 = 2432u, kTeamMost = 9728u;
+// Codes above 16 bits (no tables; codewords longer than the windows of the
+// group kernels' lanes) and batches of many meshes (unequal meshlets side by
+// side in a group) keep it for three and a half waves:
+//   20-bit heightfields, 15,068 / 21,307 meshlets: team 180 / 238, two kernels 257 / 285
+//   18 bits: 178 / 236 and 209 / 229
+//   batches of 56 / 64 / 80 / 100 mixed meshes, 11,854 / 13,238 / 16,853 / 20,903
+//   meshlets: 154 / 168 / 205 / 244 and 199 / 209 / 213 / 238
+//   (one mesh of 15,068 meshlets, 12 bits: 170 and 139)
+constexpr uint32_t kTeam4 = 700u, kTeam8 = 2432u, kTeamMost = 9728u, kTeamMore = 17024u;
+constexpr uint32_t kSmallMesh = 512u;  // meshlets per mesh, on average
 
-LaunchCfg default_config(uint32_t total_meshlets) {
+LaunchCfg default_config(uint32_t total_meshlets, uint32_t n_meshes, bool wide) {
     LaunchCfg cfg;
-    if (total_meshlets <= kTeamMost) {
+    const bool more = wide || (n_meshes > 1u && total_meshlets / n_meshes < kSmallMesh);
+    if (total_meshlets <= (more ? kTeamMore : kTeamMost)) {
         cfg.persistent = 4;
         cfg.warps_per_cta = total_meshlets <= kTeam4 ? 1 : (total_meshlets <= kTeam8 ? 2 : 4);
         return cfg;
