@@ -69,7 +69,7 @@ typedef struct {
     float g_range[3];    /* value is g_min + q / (2^g_bits - 1) * g_range     */
     uint32_t shared_bytes;      /* stride_info only, after a decode: dynamic
                                    shared memory per CTA of the decode's main
-                                   kernel (fused, group or vertex kernel)     */
+                                   kernel (team, fused, group or vertex)      */
     uint32_t persistent_blocks; /* ... and its CTAs; the reference's
                                    _shared_bytes / _persistent_blocks
                                    (utils/paradelta_v5_cuda.py:656-683)      */
@@ -228,7 +228,7 @@ int stride_decode_timed(stride_handle* h, void* stream, uint32_t* d_idx, float* 
 
 /* Launch shape for this handle's decodes.  Until it is set the shape
  * follows the mesh's size: the team kernel (persistent 4) up to 9,728
- * meshlets, the two kernels (persistent 1) up to 1,023 groups of 32
+ * meshlets (17,024 for codes above 16 bits), the two kernels (persistent 1) up to 1,023 groups of 32
  * meshlets, the fused kernel (persistent 2) above; a reload keeps a shape
  * that was set. */
 int stride_set_config(stride_handle* h, const stride_launch_cfg* cfg);
