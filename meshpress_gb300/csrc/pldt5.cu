@@ -482,12 +482,20 @@ __global__ void __launch_bounds__(kP5Threads) p5_decode_kernel(P5Args a) {
 // one lane has all of it, tokens one by one, takes ten times as long: 361 x 361
 // terrain, 1,295 meshlets, 715 us against 90.
 //
-// The host knows every meshlet's size, so each one has the same room, that of
-// the stream's largest.
-struct P5Team {
-    uint32_t bits;                  // staged bytes of a meshlet (odd in units of 16)
-    uint32_t axis;                  // doubles of an axis (odd)
-    uint32_t walk, tok, asm_w, tab;  // words: walk, token records, assembly, row table
+// The host knows every meshlet's size: a CTA's shared memory is what the
+// stream's largest group of M needs, and each meshlet gets the room of its own
+// (the room of the largest kept CTAs of sixteen from sharing an SM: 9,921
+// meshlets 251 us, now 214).
+struct P5Room {
+    uint32_t bits = 0u;  // staged bytes (odd in units of 16)
+    uint32_t loc = 0u;   // words of the walk, of the row table, and doubles of an axis (odd)
+    uint32_t tok = 0u, asm_w = 0u;  // words of the token records and of the assembly
+    __host__ __device__ void add(uint32_t bytes, uint32_t n_local, uint32_t n_tris, uint32_t n_tok) {
+        bits += bytes | 16u;
+        loc += n_local | 1u;
+        tok += team_tok_words(n_tok);
+        asm_w += team_asm_words(n_tris);
+    }
 };
 
 constexpr int32_t kP5Zigzag = 1 << 30;  // in place of a minimum (16 bits): zigzag values
@@ -505,20 +513,22 @@ __host__ __device__ constexpr uint32_t p5_team_threads() {
 // Shared memory: staged bytes, then (also where a corrupt lane's reads end)
 // walks and row tables, then the token records (read up to 31 past the last)
 // and the assembly, whose place the planes take when the walk starts.
-__host__ __device__ inline uint32_t p5_tables(const P5Team& t, uint32_t m) {  // bytes before that
-    return (m * (t.bits + 4u * (t.walk + t.tab)) + 15u) & ~15u;
+__host__ __device__ inline uint32_t p5_tables(const P5Room& t) {  // bytes before that
+    return (t.bits + 8u * t.loc + 15u) & ~15u;
 }
-__host__ __device__ inline uint32_t p5_records(const P5Team& t, uint32_t m) {  // their words
-    return (m * t.tok + 3u) & ~3u;
+__host__ __device__ inline uint32_t p5_records(const P5Room& t) {  // their words
+    return (t.tok + 3u) & ~3u;
 }
-inline uint32_t p5_team_bytes(const P5Team& t, uint32_t m) {
-    const uint32_t both = std::max(24u * m * t.axis, 4u * (p5_records(t, m) + m * t.asm_w));
-    return (std::max(p5_tables(t, m) + both, m * t.bits + kTeamSlack) + 15u) & ~15u;
+inline uint32_t p5_team_bytes(const P5Room& t) {
+    const uint32_t both = std::max(24u * t.loc, 4u * (p5_records(t) + t.asm_w));
+    return (std::max(p5_tables(t) + both, t.bits + kTeamSlack) + 15u) & ~15u;
 }
 
 struct P5Facts : TeamSize {
     unsigned long long row0, tri0;
     uint32_t m, n_bnd, n_int, n_strips;
+    uint32_t loc_off, tok_off, asm_off;  // words (doubles of an axis)
+    uint32_t axis;       // doubles of an axis
     uint32_t at, end;    // bits of the staged words: after the header, the meshlet's end
     uint32_t conn;       // where the connectivity starts
     uint32_t anchor;     // ... and ends
@@ -666,7 +676,7 @@ __device__ __forceinline__ void p5_predict(uint32_t plane, const uint32_t* __res
 }
 
 template <uint32_t M>
-__global__ void __launch_bounds__(p5_team_threads<M>(), 2) p5_team_kernel(P5Args a, P5Team L) {
+__global__ void __launch_bounds__(p5_team_threads<M>(), 2) p5_team_kernel(P5Args a) {
     constexpr uint32_t kThreads = p5_team_threads<M>(), kPred = p5_pred_warps<M>();
     constexpr uint32_t kPer = (M + kTeamAsm - 1u) / kTeamAsm;  // meshlets of an assembler warp
     extern __shared__ __align__(128) uint8_t smem[];
@@ -678,21 +688,78 @@ __global__ void __launch_bounds__(p5_team_threads<M>(), 2) p5_team_kernel(P5Args
     const uint32_t aw0 = team_asm_index(warp);  // an assembler's first meshlet
     const uint32_t n_here = min(M, a.n_meshlets - blockIdx.x * M);
     const uint32_t* words = reinterpret_cast<const uint32_t*>(smem);
-    uint32_t* walks = reinterpret_cast<uint32_t*>(smem + M * L.bits);
-    uint32_t* tabs = walks + M * L.walk;
-    double* planes = reinterpret_cast<double*>(smem + p5_tables(L, M));
+    // 1. facts (lane j of every warp: meshlet j) and layout; stage.  The header
+    // (:350-353), inside the stream as the host has checked, may end past the
+    // meshlet.
+    const bool have = static_cast<uint32_t>(lane) < n_here;
+    const uint32_t lm = blockIdx.x * M + (have ? lane : 0);
+    const uint32_t ls0 = __ldcg(a.start + lm), ls1 = __ldcg(a.start + lm + 1u);
+    const uint32_t lrow = __ldcg(a.row_base + lm), ltri = __ldcg(a.tri_base + lm);
+    const uint32_t lfrom = (ls0 >> 3) & ~15u;  // the first byte staged
+    const uint32_t ln16 = ((ls1 - 8u * lfrom) + 127u) >> 7;
+    uint32_t lh0, lh1;
+    {
+        const uint32_t* g = reinterpret_cast<const uint32_t*>(a.blob) + (ls0 >> 5);
+        const uint32_t x = bswap32(__ldcg(g)), y = bswap32(__ldcg(g + 1)), z = bswap32(__ldcg(g + 2));
+        lh0 = __funnelshift_l(y, x, ls0 & 31u);
+        lh1 = __funnelshift_l(z, y, ls0 & 31u);
+    }
+    const uint32_t lloc = (lh0 >> 16) + (lh0 & 0xFFFFu), ltok = (lh1 >> 16) + 2u * (lh1 & 0xFFFFu);
+    P5Room mine, all;
+    if (have) mine.add(16u * ln16, lloc, lh1 >> 16, ltok);
+    all = mine;
+#pragma unroll
+    for (uint32_t o = 1; o < M; o <<= 1) {
+        const uint32_t b0 = __shfl_up_sync(kFull, all.bits, o), b1 = __shfl_up_sync(kFull, all.loc, o);
+        const uint32_t b2 = __shfl_up_sync(kFull, all.tok, o), b3 = __shfl_up_sync(kFull, all.asm_w, o);
+        if (static_cast<uint32_t>(lane) >= o) {
+            all.bits += b0;
+            all.loc += b1;
+            all.tok += b2;
+            all.asm_w += b3;
+        }
+    }
+    P5Room off;  // exclusive
+    off.bits = all.bits - mine.bits;
+    off.loc = all.loc - mine.loc;
+    off.tok = all.tok - mine.tok;
+    off.asm_w = all.asm_w - mine.asm_w;
+    all.bits = __shfl_sync(kFull, all.bits, M - 1u);
+    all.loc = __shfl_sync(kFull, all.loc, M - 1u);
+    all.tok = __shfl_sync(kFull, all.tok, M - 1u);
+    uint32_t* walks = reinterpret_cast<uint32_t*>(smem + all.bits);
+    uint32_t* tabs = walks + all.loc;
+    double* planes = reinterpret_cast<double*>(smem + p5_tables(all));
     uint32_t* toks = reinterpret_cast<uint32_t*>(planes);
-    uint32_t* asms = toks + p5_records(L, M);
-    // 1. stage; facts of the meshlets
+    uint32_t* asms = toks + p5_records(all);
     if (threadIdx.x < 17u) s.masks[threadIdx.x] = threadIdx.x < 16u ? mtf_mask_row(threadIdx.x) : make_uint4(0u, 0u, 0u, 0u);
+    if (warp == 0u && have) {
+        P5Facts& F = s.f[lane];
+        F.m = lm;
+        F.n_bnd = lh0 >> 16;
+        F.n_int = lh0 & 0xFFFFu;
+        F.n_local = lloc;
+        F.n_tris = lh1 >> 16;
+        F.n_strips = lh1 & 0xFFFFu;
+        F.n_tok = ltok;
+        F.idsh = 9u - max(1u, 32u - __clz(lloc));
+        F.loc_off = off.loc;
+        F.tok_off = off.tok;
+        F.asm_off = off.asm_w;
+        F.axis = lloc | 1u;
+        F.row0 = lrow;
+        F.tri0 = ltri;
+        F.end = ls1 - 8u * lfrom + 8u * off.bits;
+        F.at = ls0 + 64u - 8u * lfrom + 8u * off.bits;
+    }
     if (assembler) {
-        for (uint32_t j = aw0; j < n_here; j += kTeamAsm) {
-            const uint32_t m = blockIdx.x * M + j;
-            const uint32_t s0 = __ldcg(a.start + m), s1 = __ldcg(a.start + m + 1u);
-            const uint32_t from = (s0 >> 3) & ~15u;  // the first byte staged
-            const uint32_t n16 = (((s1 - 8u * from) + 127u) >> 7);
+        for (uint32_t j = aw0; j < M; j += kTeamAsm) {
+            const uint32_t from = __shfl_sync(kFull, lfrom, j), n16 = __shfl_sync(kFull, ln16, j);
+            const uint32_t boff = __shfl_sync(kFull, off.bits, j), loff = __shfl_sync(kFull, off.loc, j);
+            const uint32_t row0 = __shfl_sync(kFull, lrow, j), h0 = __shfl_sync(kFull, lh0, j);
+            if (j >= n_here) continue;  // warp-uniform
             const uint4* src = reinterpret_cast<const uint4*>(a.blob + from);
-            uint4* dst = reinterpret_cast<uint4*>(smem + j * L.bits);
+            uint4* dst = reinterpret_cast<uint4*>(smem + boff);
             for (uint32_t i = lane; i < n16; i += 32u) {
                 uint4 q = __ldcg(src + i);
                 q.x = bswap32(q.x);
@@ -701,29 +768,9 @@ __global__ void __launch_bounds__(p5_team_threads<M>(), 2) p5_team_kernel(P5Args
                 q.w = bswap32(q.w);
                 dst[i] = q;
             }
-            // the header (:350-353), inside the stream as the host has checked, may end past the meshlet
-            const uint32_t* g = reinterpret_cast<const uint32_t*>(a.blob) + (s0 >> 5);
-            const uint32_t x = bswap32(__ldcg(g)), y = bswap32(__ldcg(g + 1)), z = bswap32(__ldcg(g + 2));
-            const uint32_t h0 = __funnelshift_l(y, x, s0 & 31u), h1 = __funnelshift_l(z, y, s0 & 31u);
-            P5Facts& F = s.f[j];
-            const unsigned long long row0 = __ldcg(a.row_base + m), tri0 = __ldcg(a.tri_base + m);
             const uint32_t n_bnd = h0 >> 16, n_int = h0 & 0xFFFFu;
-            if (lane == 0) {
-                F.m = m;
-                F.n_bnd = n_bnd;
-                F.n_int = n_int;
-                F.n_local = n_bnd + n_int;
-                F.n_tris = h1 >> 16;
-                F.n_strips = h1 & 0xFFFFu;
-                F.n_tok = F.n_tris + 2u * F.n_strips;
-                F.idsh = 9u - max(1u, 32u - __clz(F.n_local));
-                F.row0 = row0;
-                F.tri0 = tri0;
-                F.end = s1 - 8u * from + 8u * j * L.bits;
-                F.at = s0 + 64u - 8u * from + 8u * j * L.bits;
-            }
             // rows of the interior vertices
-            for (uint32_t i = lane; i < n_int; i += 32u) tabs[j * L.tab + n_bnd + i] = static_cast<uint32_t>(row0) + i;
+            for (uint32_t i = lane; i < n_int; i += 32u) tabs[loff + n_bnd + i] = row0 + i;
         }
     }
     __syncthreads();
@@ -733,7 +780,7 @@ __global__ void __launch_bounds__(p5_team_threads<M>(), 2) p5_team_kernel(P5Args
         const bool act = static_cast<uint32_t>(lane) < n_here;
         P5Facts& F = s.f[act ? lane : 0];
         const uint32_t n = act ? F.n_bnd : 0u;
-        uint32_t* tab = tabs + (act ? lane : 0) * L.tab;
+        uint32_t* tab = tabs + (act ? F.loc_off : 0u);
         bool bad = act && (F.n_strips > F.n_tris || F.at > F.end);  // every strip emits a triangle
         const uint32_t limit = act ? F.end : 0u;
         const uint32_t base = smem_addr(words);
@@ -793,7 +840,7 @@ __global__ void __launch_bounds__(p5_team_threads<M>(), 2) p5_team_kernel(P5Args
     const uint32_t pid = (warp - kTeamAsm - 2u) * 32u + lane;
     const uint32_t pj = pid % M, pd = pid / M < 3u ? pid / M : 2u;
     const bool pon = predictor && pid < 3u * M && ((rmask >> pj) & 1u);
-    double* pplane = planes + (pon ? (pj * 3u + pd) * L.axis : 0u);
+    double* pplane = planes + (pon ? 3u * s.f[pj].loc_off + pd * s.f[pj].axis : 0u);
     // 2. connectivity, in step: chunk c with the parser, c - 1 with the FIFO
     // warp, c - 2 with the assemblers
     for (uint32_t pass = 0; pass < 2u; pass++) {  // the second one with the exact FIFO, rarely
@@ -806,7 +853,7 @@ __global__ void __launch_bounds__(p5_team_threads<M>(), 2) p5_team_kernel(P5Args
             // order (:362-365)
             const uint32_t n = pon && !exact ? s.f[pj].n_bnd : 0u;
             const uint32_t most = __reduce_max_sync(kFull, n);
-            const uint32_t* tab = tabs + (pon ? pj : 0u) * L.tab;
+            const uint32_t* tab = tabs + (pon ? s.f[pj].loc_off : 0u);
             double mean = 0.0;
             uint32_t at = 0u;
             auto sum = [&](uint32_t upto) {
@@ -840,7 +887,7 @@ __global__ void __launch_bounds__(p5_team_threads<M>(), 2) p5_team_kernel(P5Args
             const uint32_t n_tok = act ? F.n_tok : 0u;
             const uint32_t sl = act ? lane : 0u;  // an idle lane repeats the first one's steps
             const uint32_t ib = act ? 9u - F.idsh : 1u;
-            uint16_t* row = reinterpret_cast<uint16_t*>(toks + sl * L.tok) + 2;
+            uint16_t* row = reinterpret_cast<uint16_t*>(toks + (act ? F.tok_off : 0u)) + 2;
             TeamParse T;
             MtfFifo fifo;
             uint32_t t = 0u;
@@ -883,18 +930,18 @@ __global__ void __launch_bounds__(p5_team_threads<M>(), 2) p5_team_kernel(P5Args
             // the windows that the records fill (or end)
             auto windows = [&](TeamAsm& A, uint32_t j) {
                 const P5Facts& F = s.f[j];
-                uint32_t* last = asms + j * L.asm_w;
+                uint32_t* last = asms + F.asm_off;
                 const uint32_t have = A.t >= F.n_tok ? F.n_tok + 31u : A.t;
                 for (; A.t0 + 32u <= have; A.t0 += 32u)
-                    team_window<false>(A, F, F.n_bnd, exact, A.t0, reinterpret_cast<const uint16_t*>(toks + j * L.tok) + 2,
-                                       walks + j * L.walk, nullptr, last, last + 256, lane);
+                    team_window<false>(A, F, F.n_bnd, exact, A.t0, reinterpret_cast<const uint16_t*>(toks + F.tok_off) + 2,
+                                       walks + F.loc_off, nullptr, last, last + 256, lane);
             };
             auto chunk = [&](uint32_t c) {
 #pragma unroll
                 for (uint32_t q = 0; q < kPer; q++) {
                     const uint32_t j = aw0 + q * kTeamAsm;
                     if (!mine(q) || S[q].t >= s.f[j].n_tok) continue;  // warp-uniform, here and below
-                    team_records<M>(S[q], s.f[j], exact, reinterpret_cast<uint16_t*>(toks + j * L.tok) + 2,
+                    team_records<M>(S[q], s.f[j], exact, reinterpret_cast<uint16_t*>(toks + s.f[j].tok_off) + 2,
                                     s.x[c % 3u] + j, s.step[c % 3u] + j, lane);
                     if (!exact) windows(S[q], j);
                 }
@@ -903,7 +950,7 @@ __global__ void __launch_bounds__(p5_team_threads<M>(), 2) p5_team_kernel(P5Args
             for (uint32_t q = 0; q < kPer; q++) {
                 const uint32_t j = aw0 + q * kTeamAsm;
                 if (!mine(q)) continue;
-                uint4* last = reinterpret_cast<uint4*>(asms + j * L.asm_w);
+                uint4* last = reinterpret_cast<uint4*>(asms + s.f[j].asm_off);
                 last[lane] = last[lane + 32] = make_uint4(0u, 0u, 0u, 0u);
             }
             __syncwarp();
@@ -929,12 +976,12 @@ __global__ void __launch_bounds__(p5_team_threads<M>(), 2) p5_team_kernel(P5Args
                 const uint32_t j = aw0 + q * kTeamAsm;
                 if (!mine(q)) continue;
                 P5Facts& F = s.f[j];
-                const uint32_t* tab = tabs + j * L.tab;
+                const uint32_t* tab = tabs + F.loc_off;
                 // ids of a valid meshlet lie in the table; an invalid one's are cut to it
                 const uint32_t vmax = F.n_local ? F.n_local - 1u : 0u;
                 uint32_t* out = a.idx + 3ull * F.tri0;
                 const uint32_t ph = (0u - static_cast<uint32_t>(reinterpret_cast<uintptr_t>(out) >> 2)) & 3u;
-                team_triangles(out, asms + j * L.asm_w + 256, ph, min(S[q].tcnt, F.n_tris),
+                team_triangles(out, asms + F.asm_off + 256, ph, min(S[q].tcnt, F.n_tris),
                                [&](uint32_t v) { return tab[min(v, vmax)]; }, lane);
                 const bool bad = __any_sync(kFull, S[q].out) || S[q].tcnt != F.n_tris;
                 if (lane == 0) {
@@ -970,7 +1017,7 @@ __global__ void __launch_bounds__(p5_team_threads<M>(), 2) p5_team_kernel(P5Args
                 for (uint32_t i = 0; i < F.n_int; i++) pplane[F.n_bnd + i] = 0.0;
             __syncwarp();
             bar();
-            const uint32_t* walk = walks + (on ? pj : 0u) * L.walk;
+            const uint32_t* walk = walks + (on ? F.loc_off : 0u);
             const uint32_t plane_addr = smem_addr(pplane);
             const bool unit = a.w0 == 1.0 && a.w1 == 1.0 && a.w2 == -1.0;
             for (uint32_t g = 0; g < steps; g++) {
@@ -1005,10 +1052,10 @@ __global__ void __launch_bounds__(p5_team_threads<M>(), 2) p5_team_kernel(P5Args
                         const int32_t mn = s.f[j].mn[d];
                         const unsigned long long u = s.res[(g - 1u) & 1u][it];
                         r[q] = mn == kP5Zigzag ? unzig(u) : mn + static_cast<long long>(u);
-                        const uint32_t e = walks[j * L.walk + (in[q] ? i : 0u)], v = e & 0xFFu;
+                        const uint32_t e = walks[(in[q] ? s.f[j].loc_off + i : 0u)], v = e & 0xFFu;
                         // roots are (v, v, v, v); a residual that is added to nothing is added to -0
                         mean[q] = v == ((e >> 8) & 0xFFu) ? s.mean[d * M + j] : -0.0;
-                        slot[q] = planes + (3u * j + d) * L.axis + v;
+                        slot[q] = planes + (in[q] ? 3u * s.f[j].loc_off + d * s.f[j].axis : 0u) + v;
                         x[q] = p5_double(static_cast<uint32_t>(r[q]));
                         wide = wide | (r[q] != static_cast<int32_t>(r[q]));
                     }
@@ -1098,8 +1145,8 @@ __global__ void __launch_bounds__(p5_team_threads<M>(), 2) p5_team_kernel(P5Args
                 const uint32_t n3 = 3u * s.f[j].n_bnd;
                 for (uint32_t e = 32u * emitter + lane; e < n3; e += 32u * kEmitters) {
                     const uint32_t i = e / 3u, d = e - 3u * i;
-                    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(planes + (3u * j + d) * L.axis + i)),
-                                 "l"(a.rows + 3ull * tabs[j * L.tab + i] + d)
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(planes + 3u * s.f[j].loc_off + d * s.f[j].axis + i)),
+                                 "l"(a.rows + 3ull * tabs[s.f[j].loc_off + i] + d)
                                  : "memory");
                 }
             }
@@ -1113,8 +1160,8 @@ __global__ void __launch_bounds__(p5_team_threads<M>(), 2) p5_team_kernel(P5Args
                         const uint32_t d = it % 3u, j = it / (3u * kP5Res), i = c * kP5Res + it / 3u % kP5Res;
                         const P5Facts& F = s.f[j];
                         if (!((on_mask >> j) & 1u) || i >= F.n_walk) continue;
-                        const uint32_t v = walks[j * L.walk + i] & 0xFFu;
-                        a.pos[3ull * (F.row0 + (v - F.n_bnd)) + d] = p5_world(a, planes[(3u * j + d) * L.axis + v], d);
+                        const uint32_t v = walks[F.loc_off + i] & 0xFFu;
+                        a.pos[3ull * (F.row0 + (v - F.n_bnd)) + d] = p5_world(a, planes[3u * F.loc_off + d * F.axis + v], d);
                     }
                 }
                 __syncwarp();
@@ -1133,7 +1180,7 @@ __global__ void __launch_bounds__(p5_team_threads<M>(), 2) p5_team_kernel(P5Args
             } else if (F.n_walk < F.n_int) {
                 for (uint32_t e = lane; e < 3u * F.n_int; e += 32u) {
                     const uint32_t i = e / 3u, d = e - 3u * i;
-                    a.pos[3ull * F.row0 + e] = p5_world(a, planes[(3u * j + d) * L.axis + F.n_bnd + i], d);
+                    a.pos[3ull * F.row0 + e] = p5_world(a, planes[3u * F.loc_off + d * F.axis + F.n_bnd + i], d);
                 }
             }
         }
@@ -1145,8 +1192,8 @@ __global__ void p5_world_kernel(P5Args a, unsigned long long n) {
     if (i < 3ull * n) a.pos[i] = p5_world(a, a.rows[i], static_cast<uint32_t>(i % 3ull));
 }
 
-constexpr uint32_t kP5Eight = 8u * 2u * 152u;  // meshlets that CTAs of eight take at once
-constexpr uint32_t kP5Two = 103u << 10;        // two CTAs to an SM
+constexpr uint32_t kP5Eight = 8u * 2u * 152u * 9u / 8u;  // about as many as CTAs of eight take at once
+constexpr uint32_t kP5Two = 102u << 10;        // two CTAs to an SM
 // eight meshlets of the largest size that is accepted (197 KB) and the static part, in an SM's 227 KB
 constexpr uint32_t kP5MaxSmem = 200u << 10;
 
@@ -1161,8 +1208,8 @@ cudaError_t p5_team_prepare() {
 }
 
 template <uint32_t M>
-cudaError_t p5_team_launch(const P5Args& a, const P5Team& room, cudaStream_t s) {
-    p5_team_kernel<M><<<(a.n_meshlets + M - 1u) / M, p5_team_threads<M>(), p5_team_bytes(room, M), s>>>(a, room);
+cudaError_t p5_team_launch(const P5Args& a, uint32_t smem, cudaStream_t s) {
+    p5_team_kernel<M><<<(a.n_meshlets + M - 1u) / M, p5_team_threads<M>(), smem, s>>>(a);
     return cudaGetLastError();
 }
 
@@ -1222,7 +1269,7 @@ struct pldt5_handle {
     uint32_t* d_walk = nullptr;
     double* d_rows = nullptr;    // the boundary's, and for the general kernel all
     uint32_t team = 0;           // meshlets per CTA of the team kernel, 0: the general kernel
-    P5Team room;
+    uint32_t team_smem = 0;      // its dynamic shared memory
     Status* d_status = nullptr;
     Status* h_status = nullptr;
     cudaEvent_t done = nullptr;
@@ -1252,7 +1299,9 @@ struct P5Host {
     std::vector<uint32_t> meta;   // start (M + 1) | row_base (M) | tri_base (M) | ref_base (M)
     uint64_t refs = 0;
     // the largest meshlet's
-    uint32_t most_local = 0, most_tris = 0, most_tokens = 0, most_bytes = 0;
+    uint32_t most_tokens = 0, most_bytes = 0;
+    // shared memory of the largest group of eight and of sixteen meshlets
+    uint32_t smem8 = 0, smem16 = 0;
 };
 
 static int p5_host_parse_sized(const uint8_t* data, size_t len, P5Host& H);
@@ -1342,6 +1391,7 @@ static int p5_host_parse_sized(const uint8_t* data, size_t len, P5Host& H) {
     start[M] = static_cast<uint32_t>(std::min<uint64_t>(8ull * len, 0xFFFFFFFFull));
     if (8ull * len > 0xFFFFFFFFull) return fail(STRIDE_ERR_UNSUPPORTED, "stream above 512 MiB");
     uint64_t rows = nb, tris = 0, refs = 0;
+    P5Room r8, r16;  // of the group so far
     for (uint64_t m = 0; m < M; m++) {
         // the CPU decoder reads meshlets back to back from the end of the table
         if ((m == 0 && start[0] != body) || start[m] < body || start[m] + 64ull > 8ull * len ||
@@ -1352,12 +1402,19 @@ static int p5_host_parse_sized(const uint8_t* data, size_t len, P5Host& H) {
         const uint32_t n_int = static_cast<uint32_t>(hb.read(16));
         const uint32_t n_tris = static_cast<uint32_t>(hb.read(16));
         const uint32_t n_strips = static_cast<uint32_t>(hb.read(16));
-        H.most_local = std::max(H.most_local, n_bnd + n_int);
-        H.most_tris = std::max(H.most_tris, n_tris);
         H.most_tokens = std::max(H.most_tokens, n_tris + 2u * n_strips);
         // staged: from the 16 bytes of its first bit to those of its last
         const uint64_t first = (start[m] >> 3) & ~15ull, end = ((start[m + 1] + 127ull) >> 7) << 4;
-        H.most_bytes = std::max(H.most_bytes, static_cast<uint32_t>(std::min<uint64_t>(end - first, 0xFFFFFFF0u)));
+        const uint32_t staged = static_cast<uint32_t>(std::min<uint64_t>(end - first, 0xFFFFFFF0u));
+        H.most_bytes = std::max(H.most_bytes, staged);
+        if (m % 8 == 0) r8 = P5Room{};
+        if (m % 16 == 0) r16 = P5Room{};
+        if (H.most_tokens <= kTeamTokens && H.most_bytes <= kP5MaxStage) {  // else there is no team
+            r8.add(staged, n_bnd + n_int, n_tris, n_tris + 2u * n_strips);
+            r16.add(staged, n_bnd + n_int, n_tris, n_tris + 2u * n_strips);
+            H.smem8 = std::max(H.smem8, p5_team_bytes(r8));
+            H.smem16 = std::max(H.smem16, p5_team_bytes(r16));
+        }
         if (n_bnd + n_int > static_cast<uint32_t>(kP5MaxLocal))
             return fail(STRIDE_ERR_UNSUPPORTED, "meshlet %llu has %u local vertices (at most 256)",
                         (unsigned long long)m, n_bnd + n_int);
@@ -1380,23 +1437,18 @@ static int p5_host_parse_sized(const uint8_t* data, size_t len, P5Host& H) {
 // Room and launch shape for a stream: the team kernel takes meshlets of up to
 // kTeamTokens tokens and kP5MaxStage bytes (encoded meshlets of 256 vertices
 // have half as many and a tenth), the general kernel streams with larger ones.
-static cudaError_t p5_plan(const P5Host& H, uint32_t& team, P5Team& room) {
-    team = 0;
-    room = P5Team{};
+static cudaError_t p5_plan(const P5Host& H, uint32_t& team, uint32_t& smem) {
+    team = smem = 0;
     if (H.info.n_meshlets == 0 || H.most_tokens > kTeamTokens || H.most_bytes > kP5MaxStage) return cudaSuccess;
-    room.bits = H.most_bytes | 16u;
-    room.axis = H.most_local | 1u;
-    room.walk = H.most_local | 1u;
-    room.tok = team_tok_words(H.most_tokens);
-    room.asm_w = team_asm_words(H.most_tris);
-    room.tab = H.most_local | 1u;
     // Eight meshlets per CTA as long as the CTAs are on the chip at once, two
-    // to an SM; above, sixteen where two such CTAs fit an SM: a decode then
-    // takes the CTAs' waves, and a CTA's chains hardly depend on its number of
-    // meshlets (sixteen against eight: meshlets of up to 64 vertices, 3,072 of
-    // them, 64 us against 81, 23,843 211 against 298; of up to 189 vertices,
-    // 10 79 against 75, 1,295 90 against 90, 9,921 211 against 250).
-    team = H.info.n_meshlets > kP5Eight && p5_team_bytes(room, 16u) <= kP5Two ? 16u : 8u;
+    // to an SM (or all but a few); above, sixteen where two such CTAs fit an SM:
+    // a decode then takes the CTAs' waves, and a CTA's chains hardly depend on
+    // its number of meshlets (sixteen against eight: meshlets of up to 64
+    // vertices, 3,072 of them, 65 us against 87, 23,843 212 against 298; of up to
+    // 199 vertices, 10 79 against 75, 2,451 100 against 90, 4,913 141 against 151,
+    // 9,921 214 against 253).
+    team = H.info.n_meshlets > kP5Eight && H.smem16 <= kP5Two ? 16u : 8u;
+    smem = team == 8u ? H.smem8 : H.smem16;
     return team == 8u ? p5_team_prepare<8>() : p5_team_prepare<16>();
 }
 
@@ -1423,7 +1475,7 @@ int pldt5_open(const uint8_t* data, size_t len, pldt5_handle** out) {
     }
     h->scale = static_cast<double>(info.scale);
     h->delta = 2.0 * static_cast<double>(per_coord_err);
-    cudaError_t e = p5_plan(H, h->team, h->room);
+    cudaError_t e = p5_plan(H, h->team, h->team_smem);
     if (e != cudaSuccess) {
         pldt5_free(h);
         return cuda_fail(e, "pldt5_open");
@@ -1495,7 +1547,7 @@ int pldt5_decode(pldt5_handle* h, void* stream, uint32_t* d_idx, float* d_pos) {
     a.status = h->d_status;
     if ((e = cudaMemsetAsync(h->d_status, 0, sizeof(Status), s)) != cudaSuccess) return cuda_fail(e, "pldt5_decode");
     if (h->team) {
-        e = h->team == 8 ? p5_team_launch<8>(a, h->room, s) : p5_team_launch<16>(a, h->room, s);
+        e = h->team == 8 ? p5_team_launch<8>(a, h->team_smem, s) : p5_team_launch<16>(a, h->team_smem, s);
         if (e != cudaSuccess) return cuda_fail(e, "p5_team_kernel");
     } else {
         if (rows > nb && (e = cudaMemsetAsync(h->d_rows + 3 * nb, 0, 24 * (rows - nb), s)) != cudaSuccess)

@@ -128,7 +128,7 @@ CASES = {
     "all_boundary": {"n": 3, "bnd": 17, "int": 0, "tris": 40, "tags": ()},
     "unreached": {"n": 17, "bnd": 6, "int": 50, "tris": 40, "reach": 30, "tags": (2, 0, 1)},
     "nine_bit_ids": {"n": 5, "bnd": 120, "int": 136, "tris": 450, "tags": (1, 2, 1), "w": W},
-    "groups_of_16": {"n": 2433, "bnd": 4, "int": 5, "tris": 8, "tags": (1, 2, 0), "again": 0.02},
+    "groups_of_16": {"n": 2800, "bnd": 4, "int": 5, "tris": 8, "tags": (1, 2, 0), "again": 0.02},
     "most_bytes": {"n": 9, "bnd": 2, "int": 250, "tris": 300, "tags": (1, 1, 1), "long": 0.7, "ones": 300, "w": W},
     "most_tokens": {"n": 4, "bnd": 30, "int": 100, "tris": 728, "strip": 200, "tags": (1, 2, 0), "again": 0.05},
     "more_tokens": {"n": 4, "bnd": 30, "int": 100, "tris": 800, "strip": 200, "tags": (1, 2, 0), "again": 0.05},
