@@ -1193,6 +1193,7 @@ __global__ void p5_world_kernel(P5Args a, unsigned long long n) {
 }
 
 constexpr uint32_t kP5Eight = 8u * 2u * 152u * 9u / 8u;  // about as many as CTAs of eight take at once
+constexpr uint32_t kP5Most = 44u << 10;        // meshlets of a stream
 constexpr uint32_t kP5Two = 102u << 10;        // two CTAs to an SM
 // eight meshlets of the largest size that is accepted (197 KB) and the static part, in an SM's 227 KB
 constexpr uint32_t kP5MaxSmem = 200u << 10;
@@ -1436,10 +1437,16 @@ static int p5_host_parse_sized(const uint8_t* data, size_t len, P5Host& H) {
 
 // Room and launch shape for a stream: the team kernel takes meshlets of up to
 // kTeamTokens tokens and kP5MaxStage bytes (encoded meshlets of 256 vertices
-// have half as many and a tenth), the general kernel streams with larger ones.
+// have half as many and a tenth), in streams of up to kP5Most meshlets; the
+// general kernel the others.  Its time hardly grows with the meshlets, the
+// team's does: up to 256 vertices, 21,307 / 43,086 meshlets 785 / 912 us and 377
+// / 713; up to 64 vertices, 23,843 / 50,955 meshlets about 370 / 380 and 212 /
+// 440.
 static cudaError_t p5_plan(const P5Host& H, uint32_t& team, uint32_t& smem) {
     team = smem = 0;
-    if (H.info.n_meshlets == 0 || H.most_tokens > kTeamTokens || H.most_bytes > kP5MaxStage) return cudaSuccess;
+    if (H.info.n_meshlets == 0 || H.info.n_meshlets > kP5Most || H.most_tokens > kTeamTokens ||
+        H.most_bytes > kP5MaxStage)
+        return cudaSuccess;
     // Eight meshlets per CTA as long as the CTAs are on the chip at once, two
     // to an SM (or all but a few); above, sixteen where two such CTAs fit an SM:
     // a decode then takes the CTAs' waves, and a CTA's chains hardly depend on
