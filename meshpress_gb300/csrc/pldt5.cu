@@ -1139,20 +1139,21 @@ __global__ void __launch_bounds__(p5_team_threads<M>(), 2) p5_team_kernel(P5Args
         } else {
             // f32(row * scale + center)
             bar();
-            // first, the boundary rows into the planes
-            for (uint32_t j = 0; j < n_here; j++) {
-                if (!((on_mask >> j) & 1u)) continue;
-                const uint32_t n3 = 3u * s.f[j].n_bnd;
-                for (uint32_t e = 32u * emitter + lane; e < n3; e += 32u * kEmitters) {
-                    const uint32_t i = e / 3u, d = e - 3u * i;
-                    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(planes + 3u * s.f[j].loc_off + d * s.f[j].axis + i)),
-                                 "l"(a.rows + 3ull * tabs[s.f[j].loc_off + i] + d)
-                                 : "memory");
-                }
-            }
-            cp_async_commit();
+            uint32_t rows = 0u;  // meshlets whose boundary rows are in the planes
             for (uint32_t g = 0; g < steps; g++) {
-                if (g == 2u * chunks + 1u) cp_async_wait_all();
+                // first, before the predictors start, the boundary rows of a
+                // meshlet a step (through L2, as every global read: a handle
+                // may have another's memory)
+                const uint32_t upto = g < 2u * chunks ? min(rows + 1u, n_here) : n_here;
+                for (; g < 2u * chunks + 2u && rows < upto; rows++) {
+                    if (!((on_mask >> rows) & 1u)) continue;
+                    const P5Facts& F = s.f[rows];
+#pragma unroll 4
+                    for (uint32_t e = 32u * emitter + lane; e < 3u * F.n_bnd; e += 32u * kEmitters) {
+                        const uint32_t i = e / 3u, d = e - 3u * i;
+                        planes[3u * F.loc_off + d * F.axis + i] = __ldcg(a.rows + 3ull * tabs[F.loc_off + i] + d);
+                    }
+                }
                 if (g >= 2u * chunks + 3u) {
                     const uint32_t c = g - 3u - 2u * chunks;
 #pragma unroll 2
