@@ -522,27 +522,42 @@ __device__ __forceinline__ void team_round(const DecodeArgs& a, TeamShared<M>& s
     const bool assembler = warp != kTeamParser && warp != kTeamFifo;
     const uint32_t aw0 = team_asm_index(warp);  // an assembler's first meshlet
     const uint32_t* bit_words = reinterpret_cast<const uint32_t*>(bits);
-    // 1. stage
+    // 1. stage; the mesh records' loads on their way beside the bytes' (a trip to
+    // L2 less per meshlet of a warp: sixteen to a CTA, 55 -> 53 and 96 -> 94 us for
+    // 4,090 and 7,503 meshlets)
     if (assembler) {
-        for (uint32_t j = aw0; j < M; j += kTeamAsm) {
-            if (!((rmask >> j) & 1u)) continue;  // warp-uniform, here and below
+        constexpr uint32_t kWords = sizeof(MeshParams) / 4u, kP = (kWords + 31u) / 32u;
+        uint32_t pv[kPer][kP];
+#pragma unroll
+        for (uint32_t q = 0; q < kPer; q++) {
+            const uint32_t j = aw0 + q * kTeamAsm;
+            const bool in = j < M && ((rmask >> (j & 31u)) & 1u);  // warp-uniform
+            const uint32_t* ps = reinterpret_cast<const uint32_t*>(a.meshes + (in ? s.f[j].mi : 0u));
+#pragma unroll
+            for (uint32_t r = 0; r < kP; r++) pv[q][r] = __ldcg(ps + min(lane + 32u * r, kWords - 1u));
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < kPer; q++) {
+            const uint32_t j = aw0 + q * kTeamAsm;
+            if (j >= M || !((rmask >> j) & 1u)) continue;
             TeamFacts& F = s.f[j];
-            const uint32_t* ps = reinterpret_cast<const uint32_t*>(a.meshes + F.mi);
-            uint32_t* pd = reinterpret_cast<uint32_t*>(&F.P);
-            for (uint32_t i = lane; i < sizeof(MeshParams) / 4u; i += 32u) pd[i] = __ldcg(ps + i);
             if constexpr (kShared) {
                 const uint32_t n16 = F.ssz >> 4;
                 const uint4* src = reinterpret_cast<const uint4*>(a.arena + F.src16);
                 uint4* dst = reinterpret_cast<uint4*>(bits + F.bit_off);
                 for (uint32_t i = lane; i < n16; i += 32u) {
-                    uint4 q = __ldcg(src + i);
-                    q.x = bswap32(q.x);
-                    q.y = bswap32(q.y);
-                    q.z = bswap32(q.z);
-                    q.w = bswap32(q.w);
-                    dst[i] = q;
+                    uint4 v = __ldcg(src + i);
+                    v.x = bswap32(v.x);
+                    v.y = bswap32(v.y);
+                    v.z = bswap32(v.z);
+                    v.w = bswap32(v.w);
+                    dst[i] = v;
                 }
             }
+            uint32_t* pd = reinterpret_cast<uint32_t*>(&F.P);
+#pragma unroll
+            for (uint32_t r = 0; r < kP; r++)
+                if (lane + 32u * r < kWords) pd[lane + 32u * r] = pv[q][r];
         }
     }
     // bit p of the stream is bit p + rbase of w
