@@ -190,7 +190,10 @@ struct stride_handle {
     size_t cap_v = 0, cap_t = 0;
     cudaEvent_t done = nullptr;
     Status* h_status = nullptr;         // pinned: stride_finish's copy
+    cudaEvent_t used = nullptr;         // behind the last use of the buffers that `done` does not cover
     bool launched = false;
+    bool in_use = false;                // `used` is recorded
+    bool unseen = false;                // work that no event of the handle covers (a capture's replays, a failed call's)
     bool known = false;                 // last: the last decode's status
     Status last;
     LaunchCfg cfg;
@@ -264,8 +267,8 @@ namespace {
 // Device blocks of closed handles for the next ones: a cudaMalloc and its
 // cudaFree take 60 us.  At most kBlocks blocks and kBytes bytes per process;
 // the oldest go back to the driver beyond that, all of them when an allocation
-// fails.  A block comes in once its device is idle (as cudaFree would wait),
-// so whoever takes it, on whatever stream, finds it unused.
+// fails.  A block comes in once everything its handle has enqueued is over
+// (handle_idle), so whoever takes it, on whatever stream, finds it unused.
 struct DeviceBlocks {
     static constexpr size_t kBlocks = 16, kBytes = size_t(32) << 20;
     struct Block {
@@ -332,7 +335,8 @@ static cudaError_t block_take(size_t bytes, void** out) {
     }
 }
 
-// `idle`: the caller has waited for the device the block is on.
+// `idle`: the caller has waited for whatever was to use the block; else cudaFree
+// does.
 static void block_give(void* p, bool idle) {
     if (!p) return;
     DeviceBlocks& B = device_blocks();
@@ -357,15 +361,6 @@ static void block_give(void* p, bool idle) {
         }
     }
     if (!kept) cudaFree(p);
-}
-
-// Whether device `dev` has nothing left to do.
-static bool device_idle(int dev) {
-    int now = -1;
-    if (cudaGetDevice(&now) != cudaSuccess || now != dev) return false;
-    if (cudaDeviceSynchronize() == cudaSuccess) return true;
-    cudaGetLastError();
-    return false;
 }
 
 static void for_link_events(HostLink& L, void (*f)(cudaEvent_t*, cudaError_t*), cudaError_t* e) {
@@ -530,8 +525,40 @@ int decode_to_host(HostLink& L, const DecodeArgs& a, LaunchCfg cfg, void* stream
 
 }  // namespace stride
 
-static void free_buffers(stride_handle* h) {
-    const bool idle = device_idle(h->device);
+// Waits for everything the handle has enqueued; false when that cannot be
+// told.  (Not by a device synchronisation, which would end another thread's
+// stream capture.)
+static bool handle_idle(stride_handle* h) {
+    bool ok = !h->unseen;
+    if (h->launched) ok = cudaEventSynchronize(h->done) == cudaSuccess && ok;
+    if (h->in_use) ok = cudaEventSynchronize(h->used) == cudaSuccess && ok;
+    if (h->up_parts) ok = cudaEventSynchronize(h->link.bytes_in[kHostParts - 1]) == cudaSuccess && ok;
+    if (!ok) cudaGetLastError();
+    return ok;
+}
+
+// Behind work on `stream` that reads or writes the handle's buffers and that
+// stride_decode's event does not cover.
+static cudaError_t mark_use(stride_handle* h, cudaStream_t s) {
+    const cudaError_t e = cudaEventRecord(h->used, s);
+    if (e == cudaSuccess) h->in_use = true;
+    if (e != cudaSuccess) h->unseen = true;
+    return e;
+}
+
+static bool capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cap) == cudaSuccess) return cap != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return true;  // the legacy stream while a stream captures
+}
+
+// Before such work: behind the one before it, so that one event covers both.
+static cudaError_t chain_use(stride_handle* h, cudaStream_t s) {
+    return h->in_use ? cudaStreamWaitEvent(s, h->used, 0) : cudaSuccess;
+}
+
+static void free_buffers(stride_handle* h, bool idle) {
     block_give(h->d_fixed, idle);
     block_give(h->d_mem, idle);
     block_give(h->d_out, idle);
@@ -658,7 +685,7 @@ int stride_open(const uint8_t* data, size_t len, stride_handle** out) {
     h->params = p;
     h->cfg = default_config(p.n_meshlets, 1u, wide_codes(p));
     if (rc != STRIDE_OK) {
-        free_buffers(h);
+        free_buffers(h, false);
         delete h;
         return rc;
     }
@@ -670,8 +697,10 @@ int stride_open(const uint8_t* data, size_t len, stride_handle** out) {
         (e = cudaMemcpy(h->d_blob, data, len, cudaMemcpyHostToDevice)) != cudaSuccess ||
         (e = cudaMemset(h->d_blob + len, 0, h->cap_bytes - len)) != cudaSuccess ||
         (e = cudaMemcpy(h->d_fixed, &fixed, sizeof(HandleFixed), cudaMemcpyHostToDevice)) != cudaSuccess ||
-        (e = cudaEventCreateWithFlags(&h->done, cudaEventDisableTiming)) != cudaSuccess) {
-        free_buffers(h);
+        (e = cudaEventCreateWithFlags(&h->done, cudaEventDisableTiming)) != cudaSuccess ||
+        (e = cudaEventCreateWithFlags(&h->used, cudaEventDisableTiming)) != cudaSuccess) {
+        if (h->done) cudaEventDestroy(h->done);
+        free_buffers(h, false);
         delete h;
         return cuda_fail(e, "stride_open");
     }
@@ -692,6 +721,8 @@ int stride_reload(stride_handle* h, const uint8_t* data, size_t len, void* strea
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     cudaError_t e;
     const size_t pad = std::min<size_t>(h->cap_bytes - len, kBlobPad);
+    const bool cap = capturing(s), unseen = h->unseen;
+    h->unseen = true;  // until all of it is enqueued
     // an earlier upload by parts may still be writing the arena
     if ((e = wait_upload(h, s)) != cudaSuccess) return cuda_fail(e, "stride_reload");
     h->up_parts = false;
@@ -732,9 +763,11 @@ int stride_reload(stride_handle* h, const uint8_t* data, size_t len, void* strea
     } else if ((e = cudaMemcpyAsync(h->d_blob, data, len, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
                (e = cudaMemsetAsync(h->d_blob + len, 0, pad, s)) != cudaSuccess ||
                (e = cudaMemcpyAsync(&h->d_fixed->params, &h->params, sizeof(MeshParams), cudaMemcpyHostToDevice, s)) !=
-                   cudaSuccess) {
+                   cudaSuccess ||
+               (!cap && ((e = chain_use(h, s)) != cudaSuccess || (e = mark_use(h, s)) != cudaSuccess))) {
         return cuda_fail(e, "stride_reload");
     }
+    h->unseen = unseen || cap;
     return STRIDE_OK;
 }
 
@@ -817,6 +850,7 @@ int stride_decode(stride_handle* h, void* stream, uint32_t* d_idx, float* d_pos,
     if (wait_upload(h, static_cast<cudaStream_t>(stream)) != cudaSuccess)
         return fail(STRIDE_ERR_CUDA, "decode launch failed: %s", cudaGetErrorString(cudaGetLastError()));
     h->known = false;
+    h->unseen = h->unseen || capturing(static_cast<cudaStream_t>(stream));
     const int rc = enqueue_decode(handle_args(h, d_idx, d_pos, d_codes), h->cfg, stream);
     if (rc) return fail(rc, "decode launch failed: %s", cudaGetErrorString(cudaGetLastError()));
     last_launch(&h->launch_smem, &h->launch_grid);
@@ -870,8 +904,10 @@ int stride_side_table(stride_handle* h, void* stream, uint64_t* d_resid_bit, uin
     if (!h->launched) return fail(STRIDE_ERR_ARG, "no decode yet");
     const int rc = stride_status(h, 1, nullptr);
     if (rc) return rc;
+    if (chain_use(h, static_cast<cudaStream_t>(stream)) != cudaSuccess) return fail(STRIDE_ERR_CUDA, "side table launch failed");
     const int r2 = enqueue_side_table(h->d_descs, n, reinterpret_cast<unsigned long long*>(d_resid_bit), d_sub_offs,
                                       stream);
+    mark_use(h, static_cast<cudaStream_t>(stream));
     return r2 ? fail(r2, "side table launch failed") : STRIDE_OK;
 }
 
@@ -890,9 +926,12 @@ int stride_meshlet_ranges(stride_handle* h, void* stream, uint64_t* d_v_first, u
             return cuda_fail(cudaGetLastError(), "meshlet ranges");
         return STRIDE_OK;
     }
+    if (chain_use(h, static_cast<cudaStream_t>(stream)) != cudaSuccess)
+        return fail(STRIDE_ERR_CUDA, "meshlet ranges launch failed");
     const int r2 = enqueue_meshlet_ranges(h->d_descs, h->d_blk_prefix, n,
                                           reinterpret_cast<unsigned long long*>(d_v_first),
                                           reinterpret_cast<unsigned long long*>(d_t_first), stream);
+    mark_use(h, static_cast<cudaStream_t>(stream));
     return r2 ? fail(r2, "meshlet ranges launch failed") : STRIDE_OK;
 }
 
@@ -903,7 +942,10 @@ int stride_meshlet_bounds(stride_handle* h, void* stream, const float* d_pos, fl
     if (!h->launched) return fail(STRIDE_ERR_ARG, "no decode yet");
     const int rc = stride_status(h, 1, nullptr);
     if (rc) return rc;
+    if (chain_use(h, static_cast<cudaStream_t>(stream)) != cudaSuccess)
+        return fail(STRIDE_ERR_CUDA, "meshlet bounds launch failed");
     const int r2 = enqueue_meshlet_bounds(h->d_descs, h->d_blk_prefix, h->params.n_meshlets, d_pos, d_bounds, stream);
+    mark_use(h, static_cast<cudaStream_t>(stream));
     return r2 ? fail(r2, "meshlet bounds launch failed") : STRIDE_OK;
 }
 
@@ -992,10 +1034,11 @@ int stride_set_config(stride_handle* h, const stride_launch_cfg* c) {
 
 void stride_close(stride_handle* h) {
     if (!h) return;
-    if (h->launched) cudaEventSynchronize(h->done);
-    if (h->done) cudaEventDestroy(h->done);
+    const bool idle = handle_idle(h);
+    cudaEventDestroy(h->done);
+    cudaEventDestroy(h->used);
     host_link_free(h->link);
-    free_buffers(h);
+    free_buffers(h, idle);
     delete h;
 }
 

@@ -49,3 +49,35 @@ def test_errors_stay_with_their_decode(good, shape):
             assert np.array_equal(verts.cpu().numpy().view(np.uint32), opos.view(np.uint32))
             assert np.array_equal(tris.cpu().numpy().astype(np.int64), oidx)
     dec.close()
+
+
+def test_memory_of_closed_handles(good):
+    """Handles closed with work still queued on two streams hand their memory to
+    the next ones, larger and smaller: every output is its own stream's."""
+    import torch
+    from meshpress_gb300 import ParaDeltaV5GpuDecoder
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    blobs = [good[0]] + [encoder.encode(*synth.noise_heightfield(n, seed=n), precision_error=synth.bbox_bits_error(12),
+                                        precision_mode="bbox_frac").data for n in (33, 129, 200)]
+    want = [oracle.decode(b) for b in blobs]
+    got = []
+    for r in range(24):
+        k = (r * 7) % len(blobs)
+        dec = ParaDeltaV5GpuDecoder(blobs[(k + 1) % len(blobs)])
+        dec.reload(blobs[k], stream=streams[r % 2])  # may grow
+        with torch.cuda.stream(streams[r % 2]):
+            tris, verts = dec.decode_to_device(check=False)
+            bounds = dec.meshlet_bounds(verts, stream=streams[r % 2])
+        streams[1 - r % 2].wait_stream(streams[r % 2])
+        with torch.cuda.stream(streams[1 - r % 2]):
+            again = dec.meshlet_bounds(verts, stream=streams[1 - r % 2])
+        dec.close()
+        got.append((k, tris, verts, bounds, again))
+    torch.cuda.synchronize()
+    for k, tris, verts, bounds, again in got:
+        opos, oidx = want[k]
+        assert np.array_equal(verts.cpu().numpy().view(np.uint32), opos.view(np.uint32))
+        assert np.array_equal(tris.cpu().numpy().astype(np.int64), oidx)
+        assert torch.equal(bounds, again)
+        b = bounds.cpu().numpy()
+        assert np.array_equal(b[:, :3].min(0), opos.min(0)) and np.array_equal(b[:, 3:].max(0), opos.max(0))
