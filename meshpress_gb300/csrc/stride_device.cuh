@@ -12,6 +12,7 @@
 
 #include <cstdint>
 #include <cstring>
+#include <mutex>
 #include <type_traits>
 
 #include "stride_common.cuh"
@@ -717,12 +718,16 @@ __device__ __forceinline__ int scan_meshlet(const uint8_t* __restrict__ arena, c
 }
 
 // Host: lets `kernel` use `smem` bytes of dynamic shared memory on the
-// current device (once per device and size; `configured` is the caller's).
+// current device (once per device and size; `configured` is the caller's).  The
+// limit only grows: sizes follow the meshes, and a thread that set a smaller one
+// last would fail the others' launches.
 template <class K>
 cudaError_t opt_in_smem(K kernel, size_t smem, size_t* configured) {
     int dev = 0;
     cudaGetDevice(&dev);
     dev = dev < 0 || dev >= 64 ? 0 : dev;
+    static std::mutex mu;
+    std::lock_guard<std::mutex> guard(mu);
     if (configured[dev] < smem) {
         cudaError_t e =
             cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));

@@ -81,3 +81,42 @@ def test_memory_of_closed_handles(good):
         assert torch.equal(bounds, again)
         b = bounds.cpu().numpy()
         assert np.array_equal(b[:, :3].min(0), opos.min(0)) and np.array_equal(b[:, 3:].max(0), opos.max(0))
+
+
+def test_threads_with_meshes_of_different_sizes(good):
+    """Launch attributes, pinned words and closed handles' memory are shared by
+    the process: eight threads open, decode and close their own meshes at once."""
+    import threading
+    import torch
+    from meshpress_gb300 import ParaDeltaV5GpuDecoder
+    blobs = [encoder.encode(*synth.noise_heightfield(n, seed=n), precision_error=synth.bbox_bits_error(b),
+                            precision_mode="bbox_frac", max_verts=v, max_tris=t).data
+             for n, b, v, t in ((33, 12, 64, 124), (65, 16, 256, 256), (97, 10, 128, 256), (129, 12, 256, 256))]
+    want = [oracle.decode(b) for b in blobs]
+    bad = []
+
+    def work(k):
+        try:
+            s = torch.cuda.Stream()
+            for r in range(12):
+                i = (k + r) % len(blobs)
+                dec = ParaDeltaV5GpuDecoder(blobs[i])
+                if r % 2:
+                    pos, idx = dec.decode_to_host(stream=s)
+                else:
+                    with torch.cuda.stream(s):
+                        tris, verts = dec.decode_to_device(stream=s)
+                        pos, idx = verts.cpu().numpy(), tris.cpu().numpy()
+                dec.close()
+                if not (np.array_equal(pos.view(np.uint32), want[i][0].view(np.uint32)) and
+                        np.array_equal(idx.astype(np.int64), want[i][1])):
+                    bad.append((k, r))
+        except Exception as e:  # noqa: BLE001 -- reported below
+            bad.append((k, repr(e)))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(8)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
