@@ -666,7 +666,7 @@ int stride_inspect(const uint8_t* data, size_t len, stride_info_t* info) {
     char why[256] = {0};
     const int rc = parse_header(data, len, &p, why, sizeof(why));
     if (rc) return fail(rc, "%s", why);
-    fill_info(p, len, default_config(p.n_meshlets, 1u, wide_codes(p)).persistent, info);
+    fill_info(p, len, default_config(p.n_meshlets, p.n_t, 1u, wide_codes(p)).persistent, info);
     return STRIDE_OK;
 }
 
@@ -683,7 +683,7 @@ int stride_open(const uint8_t* data, size_t len, stride_handle** out) {
     cudaError_t e;
     rc = ensure_capacity(h, len, p);
     h->params = p;
-    h->cfg = default_config(p.n_meshlets, 1u, wide_codes(p));
+    h->cfg = default_config(p.n_meshlets, p.n_t, 1u, wide_codes(p));
     if (rc != STRIDE_OK) {
         free_buffers(h, false);
         delete h;
@@ -717,7 +717,7 @@ int stride_reload(stride_handle* h, const uint8_t* data, size_t len, void* strea
     if ((rc = ensure_capacity(h, len, p)) != STRIDE_OK) return rc;
     h->params = p;
     h->len = len;
-    if (!h->cfg_set) h->cfg = default_config(p.n_meshlets, 1u, wide_codes(p));
+    if (!h->cfg_set) h->cfg = default_config(p.n_meshlets, p.n_t, 1u, wide_codes(p));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     cudaError_t e;
     const size_t pad = std::min<size_t>(h->cap_bytes - len, kBlobPad);

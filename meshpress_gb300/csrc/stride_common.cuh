@@ -190,7 +190,7 @@ int enqueue_part(const DecodeArgs& a, const LaunchCfg& cfg, void* stream, uint32
                  void* bytes_in, void* scan_done, void* conn_done);
 int enqueue_parts_end(const DecodeArgs& a, const LaunchCfg& cfg, void* stream, void* vert_done);
 // The launch shape a decode of this many meshlets takes unless one is set.
-LaunchCfg default_config(uint32_t total_meshlets, uint32_t n_meshes, bool wide);
+LaunchCfg default_config(uint32_t total_meshlets, uint64_t total_tris, uint32_t n_meshes, bool wide);
 
 // Meshlet-native outputs of a finished decode: each meshlet's first vertex
 // and triangle row (n + 1 entries, the last the totals); the bounds (min

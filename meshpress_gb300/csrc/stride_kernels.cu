@@ -1331,7 +1331,7 @@ int check_config(const LaunchCfg& cfg, bool wide) {
 
 // Meshlets up to which the default launch shape is the team kernel, and with
 // 4, 8 and 16 meshlets per CTA: as many CTAs as the 152 SMs hold at once (two
-// per SM; four meshlets while there is one CTA per SM), and 16 for up to two
+// per SM; four small meshlets while there is one CTA per SM), and 16 for up to two
 // such waves.  Step in us, L2 flushed, 12-bit heightfields, every output
 // bit-identical; before: the fused kernel up to 128 groups, then the two
 // kernels:
@@ -1350,15 +1350,20 @@ int check_config(const LaunchCfg& cfg, bool wide) {
 //   batches of 56 / 64 / 80 / 100 mixed meshes, 11,854 / 13,238 / 16,853 / 20,903
 //   meshlets: 154 / 168 / 205 / 244 and 199 / 209 / 213 / 238
 //   (one mesh of 15,068 meshlets, 12 bits: 170 and 139)
-constexpr uint32_t kTeam4 = 700u, kTeam8 = 2432u, kTeamMost = 9728u, kTeamMore = 17024u;
+// Four to a CTA stay ahead of eight for a whole wave of them when the meshlets
+// are large (923 / 1,190 of 195 triangles 35 / 35 us, by eight 39 / 39; 962 of 84
+// triangles 28.6 and 26.6).
+constexpr uint32_t kTeam4 = 700u, kTeam4Full = 1216u, kTeam8 = 2432u, kTeamMost = 9728u, kTeamMore = 17024u;
+constexpr uint32_t kFullMeshlet = 128u;  // triangles, on average
 constexpr uint32_t kSmallMesh = 512u;  // meshlets per mesh, on average
 
-LaunchCfg default_config(uint32_t total_meshlets, uint32_t n_meshes, bool wide) {
+LaunchCfg default_config(uint32_t total_meshlets, uint64_t total_tris, uint32_t n_meshes, bool wide) {
     LaunchCfg cfg;
     const bool more = wide || (n_meshes > 1u && total_meshlets / n_meshes < kSmallMesh);
     if (total_meshlets <= (more ? kTeamMore : kTeamMost)) {
         cfg.persistent = 4;
-        cfg.warps_per_cta = total_meshlets <= kTeam4 ? 1 : (total_meshlets <= kTeam8 ? 2 : 4);
+        const uint32_t four = total_tris / kFullMeshlet < total_meshlets ? kTeam4 : kTeam4Full;
+        cfg.warps_per_cta = total_meshlets <= four ? 1 : (total_meshlets <= kTeam8 ? 2 : 4);
         return cfg;
     }
     const uint32_t groups = (total_meshlets + 31u) / 32u;

@@ -505,7 +505,7 @@ bool dispatch(stride_server* s, int slot_i) {
         a.wide_codes = false;
         for (const MeshParams& p : params)
             a.wide_codes = a.wide_codes || p.g_bits[0] > 16 || p.g_bits[1] > 16 || p.g_bits[2] > 16;
-        LaunchCfg cfg = default_config(tm, a.n_meshes, a.wide_codes);  // the launch's shape by its size
+        LaunchCfg cfg = default_config(tm, tt, a.n_meshes, a.wide_codes);  // the launch's shape by its size
         if (a.wide_codes) cfg.code_bytes = std::max<uint32_t>(cfg.code_bytes, kMaxLocal * 4u);
         rc = enqueue_decode(a, cfg, st);
         if (rc == STRIDE_OK &&
