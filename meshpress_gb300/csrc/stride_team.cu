@@ -794,7 +794,8 @@ __device__ __forceinline__ void team_round(const DecodeArgs& a, TeamShared<M>& s
             team_dec_bar(k);  // the predictor has left the planes
             if (on && X.slow) {
                 TeamAxis Y = X;  // a copy: only this path keeps it in memory
-                X.bad = !team_walk_slow<kShared, kWide>(Y, &P, d, w, limit, walk, n_walk, plane);
+                // (what the header's checks refused stays refused: the walk knows only the low bits of k)
+                X.bad = X.bad || !team_walk_slow<kShared, kWide>(Y, &P, d, w, limit, walk, n_walk, plane);
                 cend = Y.pos0;
                 X.cp = Y.cp;
                 X.cdd = Y.cdd;
