@@ -867,10 +867,14 @@ static int say_status(const Status& st, uint32_t* bad_meshlet) {
     return rc ? fail(rc, "%s (meshlet %u)", status_message(rc), bad) : STRIDE_OK;
 }
 
+// Whether `last` is the last decode's status: a captured one's replays run
+// without a call.
+static bool seen(const stride_handle* h) { return h->known && !h->unseen; }
+
 int stride_status(stride_handle* h, int wait, uint32_t* bad_meshlet) {
     if (!h) return fail(STRIDE_ERR_ARG, "null handle");
     if (!h->launched) return STRIDE_OK;
-    if (h->known) return say_status(h->last, bad_meshlet);
+    if (seen(h)) return say_status(h->last, bad_meshlet);
     cudaError_t e = wait ? cudaEventSynchronize(h->done) : cudaEventQuery(h->done);
     if (e == cudaErrorNotReady) return STRIDE_ERR_BUSY;
     if (e != cudaSuccess) return cuda_fail(e, "decode");
@@ -885,7 +889,7 @@ int stride_status(stride_handle* h, int wait, uint32_t* bad_meshlet) {
 int stride_finish(stride_handle* h, void* stream, uint32_t* bad_meshlet) {
     if (!h) return fail(STRIDE_ERR_ARG, "null handle");
     if (!h->launched) return STRIDE_OK;
-    if (h->known) return say_status(h->last, bad_meshlet);
+    if (seen(h)) return say_status(h->last, bad_meshlet);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     cudaError_t e = cudaStreamWaitEvent(s, h->done, 0);  // another stream's decode
     if (e == cudaSuccess) e = cudaMemcpyAsync(h->h_status, &h->d_fixed->status, sizeof(Status), cudaMemcpyDeviceToHost, s);
