@@ -154,6 +154,15 @@ struct DecodeArgs {
     unsigned long long hint_bytes = 0ull, hint_v = 0ull, hint_t = 0ull;
 };
 
+// Bytes of a meshlet, arena offsets [src16, end16), as the sums by which the
+// kernels form rounds of staged meshlets count them.  A last meshlet may be padded
+// to 512 MiB, eight of which wrap a 32-bit sum; above kStageMost it fits no stage
+// (an SM has 227 KB) and counts as that, so that a warp's 32 stay far below.
+constexpr uint32_t kStageMost = 1u << 20;
+constexpr uint32_t staged_bytes(unsigned long long src16, unsigned long long end16) {
+    return end16 - src16 < kStageMost ? static_cast<uint32_t>(end16 - src16) : kStageMost;
+}
+
 // Host: assigns table offsets (has_lut, lut_off) to the meshes that get
 // tables (`alone`: see lut_entries); returns the floats needed, fills `meshes` (at most max_meshes
 // indices) and the largest per-mesh size.

@@ -652,7 +652,7 @@ __device__ void group_decode(const DecodeArgs& a, uint32_t g, int lane, uint8_t*
     const uint32_t csz = 4u * (((n_local * static_cast<uint32_t>(sizeof(PlaneT<kWide>)) + 3u) >> 2) | 1u);
     const unsigned long long src16 = (L.blob_off + (G.anchor >> 3)) & ~15ull;
     const unsigned long long end16 = (L.blob_off + ((L.d.end_bit + 7u) >> 3) + 12ull + 15ull) & ~15ull;
-    const uint32_t ssz = ok ? static_cast<uint32_t>(end16 - src16) : 0u;
+    const uint32_t ssz = ok ? staged_bytes(src16, end16) : 0u;
     const uint32_t sbase = static_cast<uint32_t>((src16 - L.blob_off) * 8ull);
     uint32_t todo = __ballot_sync(kFull, ok);
     while (todo) {

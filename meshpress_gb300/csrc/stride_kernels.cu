@@ -922,7 +922,7 @@ __device__ __forceinline__ bool vert_group(const DecodeArgs& a, uint32_t g, uint
     // this lane's residual bits: anchor .. end, 16-byte aligned
     const unsigned long long src16 = (L.blob_off + (L.d.anchor_bit >> 3)) & ~15ull;
     const unsigned long long end16 = (L.blob_off + ((L.d.end_bit + 7u) >> 3) + 15ull) & ~15ull;
-    const uint32_t ssz = ok ? static_cast<uint32_t>(end16 - src16) : 0u;
+    const uint32_t ssz = ok ? staged_bytes(src16, end16) : 0u;
     // its stage region: an odd number of 16-byte units, for the reason
     // the code planes have odd word counts (lanes read at about the same
     // offsets at the same time)

@@ -891,7 +891,7 @@ __global__ void __launch_bounds__(kTeamThreads, 2) team_kernel(DecodeArgs a, uin
                 const unsigned long long blob = P.blob_off;
                 F.src16 = (blob + (D.start_bit >> 3)) & ~15ull;
                 const unsigned long long end16 = (blob + ((D.end_bit + 7u) >> 3) + 15ull) & ~15ull;
-                F.ssz = ok ? static_cast<uint32_t>(end16 - F.src16) : 0u;
+                F.ssz = ok ? staged_bytes(F.src16, end16) : 0u;
             }
             F.n_local = ok ? D.counts0 & 0xFFFFu : 0u;
             F.n_tris = ok ? D.counts0 >> 16 : 0u;
