@@ -820,12 +820,14 @@ int stride_decode_timed(stride_handle* h, void* stream, uint32_t* d_idx, float* 
     for (auto& e : ev) cudaEventCreate(&e);
     void* evp[4] = {ev[0], ev[1], ev[2], ev[3]};
     h->known = false;
+    const bool unseen = h->unseen || capturing(static_cast<cudaStream_t>(stream));
+    h->unseen = true;  // as in stride_decode
     int rc = wait_upload(h, static_cast<cudaStream_t>(stream)) == cudaSuccess
                  ? enqueue_decode(handle_args(h, d_idx, d_pos, nullptr), h->cfg, stream, evp)
                  : STRIDE_ERR_CUDA;
     if (rc == STRIDE_OK) {
         last_launch(&h->launch_smem, &h->launch_grid);
-        cudaEventRecord(h->done, static_cast<cudaStream_t>(stream));
+        if (cudaEventRecord(h->done, static_cast<cudaStream_t>(stream)) == cudaSuccess) h->unseen = unseen;
         h->launched = true;
         cudaError_t e = cudaEventSynchronize(ev[3]);
         if (e != cudaSuccess) {
@@ -850,13 +852,15 @@ int stride_decode(stride_handle* h, void* stream, uint32_t* d_idx, float* d_pos,
     if (wait_upload(h, static_cast<cudaStream_t>(stream)) != cudaSuccess)
         return fail(STRIDE_ERR_CUDA, "decode launch failed: %s", cudaGetErrorString(cudaGetLastError()));
     h->known = false;
-    h->unseen = h->unseen || capturing(static_cast<cudaStream_t>(stream));
+    const bool unseen = h->unseen || capturing(static_cast<cudaStream_t>(stream));
+    h->unseen = true;  // until all of it is enqueued, and the event behind it
     const int rc = enqueue_decode(handle_args(h, d_idx, d_pos, d_codes), h->cfg, stream);
     if (rc) return fail(rc, "decode launch failed: %s", cudaGetErrorString(cudaGetLastError()));
     last_launch(&h->launch_smem, &h->launch_grid);
     cudaError_t e = cudaEventRecord(h->done, static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return cuda_fail(e, "cudaEventRecord");
     h->launched = true;
+    h->unseen = unseen;
     return STRIDE_OK;
 }
 
@@ -1004,8 +1008,9 @@ int stride_decode_host(stride_handle* h, void* stream, uint32_t* h_idx, float* h
     const cudaEvent_t* bytes_in = h->up_parts ? h->link.bytes_in : nullptr;
     const int rc = decode_to_host(h->link, handle_args(h, d_idx, d_pos, nullptr), h->cfg, stream,
                                   h->params.n_t, h->params.n_v, h_idx, h_pos, bytes_in, &bad, &ran);
-    if (!ran) {
+    if (!ran) {  // what was enqueued before the failure may still run
         h->known = false;
+        h->unseen = true;
         return rc;
     }
     h->last = *h->link.h_status;

@@ -60,6 +60,29 @@ def _open(lib, data=SMALL):
     return h
 
 
+CALLS = {
+    "decode": lambda lib, h: lib.stride_decode(h, S, AT, AT, None),
+    "timed": lambda lib, h: lib.stride_decode_timed(h, S, AT, AT, None),
+    "host": lambda lib, h: lib.stride_decode_host(h, S, AT, AT),
+}
+
+
+@pytest.mark.parametrize("call", CALLS)
+def test_memory_of_a_failed_decode_is_not_handed_on(lib, call):
+    """A launch that fails leaves the scan before it on the stream: the handle's
+    memory goes back to the driver, whose cudaFree waits, and not to the next handle."""
+    h = _open(lib)
+    assert CALLS[call](lib, h) == 0
+    lib.stride_close(h)
+    assert not lib.fake_returned()  # kept for the next handle
+    h = _open(lib)
+    lib.fake_decode(_lib.STRIDE_ERR_CUDA, 0)
+    assert CALLS[call](lib, h) == _lib.STRIDE_ERR_CUDA
+    lib.fake_decode(0, 0)
+    lib.stride_close(h)
+    assert lib.fake_returned()
+
+
 OUTPUTS = {
     "ranges": lambda lib, h, s=S: lib.stride_meshlet_ranges(h, s, AT, AT),
     "bounds": lambda lib, h, s=S: lib.stride_meshlet_bounds(h, s, AT, AT),
