@@ -589,7 +589,12 @@ static int ensure_capacity(stride_handle* h, size_t len, MeshParams& p) {
                  o_prefix = place(sizeof(BlockPrefix) * static_cast<unsigned long long>(nb)), o_walk = place(4ull * c_ww),
                  o_lut = place(4ull * c_lut);
     block_give(h->d_mem, false);  // cudaFree: after the work queued on it
-    h->d_mem = nullptr;
+    h->d_mem = h->d_blob = nullptr;
+    h->d_descs = nullptr;
+    h->d_blk_sums = nullptr;
+    h->d_blk_prefix = nullptr;
+    h->d_walk_scratch = nullptr;
+    h->d_lut = nullptr;
     h->cap_bytes = 0;
     h->cap_meshlets = 0;
     h->walk_cap = h->lut_cap = 0;
@@ -910,6 +915,7 @@ int stride_side_table(stride_handle* h, void* stream, uint64_t* d_resid_bit, uin
     const uint32_t n = h->params.n_meshlets;
     if (n && (!d_resid_bit || !d_sub_offs)) return fail(STRIDE_ERR_ARG, "null output pointer");
     if (!h->launched) return fail(STRIDE_ERR_ARG, "no decode yet");
+    if (!h->d_mem) return no_buffers();
     const int rc = stride_status(h, 1, nullptr);
     if (rc) return rc;
     if (chain_use(h, static_cast<cudaStream_t>(stream)) != cudaSuccess) return fail(STRIDE_ERR_CUDA, "side table launch failed");
@@ -922,6 +928,7 @@ int stride_side_table(stride_handle* h, void* stream, uint64_t* d_resid_bit, uin
 int stride_meshlet_ranges(stride_handle* h, void* stream, uint64_t* d_v_first, uint64_t* d_t_first) {
     if (!h || !d_v_first || !d_t_first) return fail(STRIDE_ERR_ARG, "null argument");
     if (!h->launched) return fail(STRIDE_ERR_ARG, "no decode yet");
+    if (!h->d_mem) return no_buffers();
     const int rc = stride_status(h, 1, nullptr);
     if (rc) return rc;
     const uint32_t n = h->params.n_meshlets;
@@ -948,6 +955,7 @@ int stride_meshlet_bounds(stride_handle* h, void* stream, const float* d_pos, fl
     if ((reinterpret_cast<uintptr_t>(d_pos) & 3u) || (reinterpret_cast<uintptr_t>(d_bounds) & 3u))
         return fail(STRIDE_ERR_ARG, "positions and bounds must be 4-byte aligned");
     if (!h->launched) return fail(STRIDE_ERR_ARG, "no decode yet");
+    if (!h->d_mem) return no_buffers();
     const int rc = stride_status(h, 1, nullptr);
     if (rc) return rc;
     if (chain_use(h, static_cast<cudaStream_t>(stream)) != cudaSuccess)

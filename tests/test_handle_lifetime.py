@@ -90,6 +90,24 @@ OUTPUTS = {
 }
 
 
+@pytest.mark.parametrize("call", OUTPUTS)
+def test_outputs_after_a_reload_that_could_not_allocate(lib, call):
+    h = _open(lib)
+    assert lib.stride_decode(h, S, AT, AT, None) == 0
+    assert lib.stride_finish(h, S, None) == 0
+    assert OUTPUTS[call](lib, h) == 0
+    lib.fake_most(len(SMALL))
+    assert lib.stride_reload(h, LARGE, len(LARGE), S) == _lib.STRIDE_ERR_CUDA
+    n = lib.fake_outputs()
+    assert OUTPUTS[call](lib, h) != 0
+    assert lib.fake_outputs() == n and not lib.fake_freed_used()  # nothing launched on the memory given back
+    lib.fake_most(1 << 40)
+    assert lib.stride_reload(h, LARGE, len(LARGE), S) == 0
+    assert lib.stride_decode(h, S, AT, AT, None) == 0
+    assert OUTPUTS[call](lib, h) == 0
+    lib.stride_close(h)
+
+
 def test_status_of_a_replayed_decode(lib):
     """A decode captured, then one run eagerly and checked, then the captured one
     replayed: the status is the replay's."""
