@@ -4,6 +4,7 @@
 // handles, which a failing launch or allocation tests without a GPU.
 #include "../meshpress_gb300/csrc/stride_api.cu"
 
+#include <map>
 #include <set>
 
 namespace {
@@ -11,7 +12,8 @@ namespace {
 struct Ev {
     bool recorded = false, captured = false;
 };
-std::set<void*> g_live, g_freed;
+std::map<void*, size_t> g_bytes;  // of every block ever
+std::set<void*> g_freed;
 size_t g_most = ~size_t(0);  // cudaMalloc fails above
 void* g_capturing = nullptr; // the stream in capture
 int g_decode_rc = 0;
@@ -23,11 +25,14 @@ uint8_t* g_arena = nullptr;
 
 Ev* ev(cudaEvent_t e) { return reinterpret_cast<Ev*>(e); }
 
+bool freed(const void* p) {
+    for (void* q : g_freed)
+        if (p >= q && p < static_cast<uint8_t*>(q) + g_bytes[q]) return true;
+    return false;
+}
+
 void records(const void* p) {
-    for (void* q : g_freed) {  // blocks are far apart: below 1 MB each here
-        const uint8_t* b = static_cast<const uint8_t*>(q);
-        if (p >= b && p < b + 4096) g_freed_used = true;
-    }
+    g_freed_used = g_freed_used || freed(p);
     g_outputs++;
 }
 
@@ -40,12 +45,12 @@ cudaError_t cudaGetLastError() { return cudaSuccess; }
 const char* cudaGetErrorString(cudaError_t) { return "fake"; }
 cudaError_t cudaMalloc(void** p, size_t n) {
     if (n > g_most) return *p = nullptr, cudaErrorMemoryAllocation;
-    *p = std::calloc(1, n + 256);
-    g_live.insert(*p);
+    *p = std::calloc(1, n);
+    g_bytes[*p] = n;
     return cudaSuccess;
 }
 cudaError_t cudaFree(void* p) {
-    if (p) g_live.erase(p), g_freed.insert(p);
+    if (p) g_freed.insert(p);
     return cudaSuccess;
 }
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { return *p = std::calloc(1, n), cudaSuccess; }
@@ -100,15 +105,7 @@ void fake_replay(unsigned long long err) { g_status->err = err; }  // of the las
 uint32_t fake_outputs() { return g_outputs; }
 int fake_freed_used() { return g_freed_used ? 1 : 0; }
 // whether the last decode's status word and bytes have gone back to the driver
-int fake_returned() {
-    bool st = false, by = false;
-    for (void* p : g_freed) {
-        const uint8_t* b = static_cast<const uint8_t*>(p);
-        st = st || (reinterpret_cast<uint8_t*>(g_status) >= b && reinterpret_cast<uint8_t*>(g_status) < b + 4096);
-        by = by || g_arena == b;
-    }
-    return st && by ? 1 : 0;
-}
+int fake_returned() { return freed(g_status) && freed(g_arena) ? 1 : 0; }
 
 }  // extern "C"
 
