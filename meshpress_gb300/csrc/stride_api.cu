@@ -880,10 +880,9 @@ static int say_status(const Status& st, uint32_t* bad_meshlet) {
 // without a call.
 static bool seen(const stride_handle* h) { return h->known && !h->unseen; }
 
-int stride_status(stride_handle* h, int wait, uint32_t* bad_meshlet) {
-    if (!h) return fail(STRIDE_ERR_ARG, "null handle");
+static int read_status(stride_handle* h, int wait, uint32_t* bad_meshlet, bool kept) {
     if (!h->launched) return STRIDE_OK;
-    if (seen(h)) return say_status(h->last, bad_meshlet);
+    if (kept && seen(h)) return say_status(h->last, bad_meshlet);
     cudaError_t e = wait ? cudaEventSynchronize(h->done) : cudaEventQuery(h->done);
     if (e == cudaErrorNotReady) return STRIDE_ERR_BUSY;
     if (e != cudaSuccess) return cuda_fail(e, "decode");
@@ -891,6 +890,11 @@ int stride_status(stride_handle* h, int wait, uint32_t* bad_meshlet) {
     if ((e = cudaMemcpy(&st, &h->d_fixed->status, sizeof(st), cudaMemcpyDeviceToHost)) != cudaSuccess)
         return cuda_fail(e, "cudaMemcpy(status)");
     return say_status(st, bad_meshlet);
+}
+
+int stride_status(stride_handle* h, int wait, uint32_t* bad_meshlet) {
+    if (!h) return fail(STRIDE_ERR_ARG, "null handle");
+    return read_status(h, wait, bad_meshlet, true);
 }
 
 // The status comes back on the decode's stream, queued behind it: a copy
@@ -910,18 +914,32 @@ int stride_finish(stride_handle* h, void* stream, uint32_t* bad_meshlet) {
     return say_status(h->last, bad_meshlet);
 }
 
+// Before work on `stream` that reads the last decode's records: its status, and
+// the order behind the work before it, so that one event covers both.  No event
+// covers a captured call's replays (an event recorded in a capture cannot be
+// waited for outside it, nor the handle's eager ones inside), and its status is
+// read, not taken from an earlier call.
+static int begin_use(stride_handle* h, cudaStream_t s, bool* cap, const char* what) {
+    *cap = capturing(s);
+    const int rc = read_status(h, 1, nullptr, !*cap);
+    if (rc) return rc;
+    if (*cap) h->unseen = true;
+    if (!*cap && chain_use(h, s) != cudaSuccess) return fail(STRIDE_ERR_CUDA, "%s launch failed", what);
+    return STRIDE_OK;
+}
+
 int stride_side_table(stride_handle* h, void* stream, uint64_t* d_resid_bit, uint16_t* d_sub_offs) {
     if (!h) return fail(STRIDE_ERR_ARG, "null handle");
     const uint32_t n = h->params.n_meshlets;
     if (n && (!d_resid_bit || !d_sub_offs)) return fail(STRIDE_ERR_ARG, "null output pointer");
     if (!h->launched) return fail(STRIDE_ERR_ARG, "no decode yet");
     if (!h->d_mem) return no_buffers();
-    const int rc = stride_status(h, 1, nullptr);
+    bool cap = false;
+    const int rc = begin_use(h, static_cast<cudaStream_t>(stream), &cap, "side table");
     if (rc) return rc;
-    if (chain_use(h, static_cast<cudaStream_t>(stream)) != cudaSuccess) return fail(STRIDE_ERR_CUDA, "side table launch failed");
     const int r2 = enqueue_side_table(h->d_descs, n, reinterpret_cast<unsigned long long*>(d_resid_bit), d_sub_offs,
                                       stream);
-    mark_use(h, static_cast<cudaStream_t>(stream));
+    if (!cap) mark_use(h, static_cast<cudaStream_t>(stream));
     return r2 ? fail(r2, "side table launch failed") : STRIDE_OK;
 }
 
@@ -929,7 +947,8 @@ int stride_meshlet_ranges(stride_handle* h, void* stream, uint64_t* d_v_first, u
     if (!h || !d_v_first || !d_t_first) return fail(STRIDE_ERR_ARG, "null argument");
     if (!h->launched) return fail(STRIDE_ERR_ARG, "no decode yet");
     if (!h->d_mem) return no_buffers();
-    const int rc = stride_status(h, 1, nullptr);
+    bool cap = false;
+    const int rc = begin_use(h, static_cast<cudaStream_t>(stream), &cap, "meshlet ranges");
     if (rc) return rc;
     const uint32_t n = h->params.n_meshlets;
     if (n == 0u) {
@@ -941,12 +960,10 @@ int stride_meshlet_ranges(stride_handle* h, void* stream, uint64_t* d_v_first, u
             return cuda_fail(cudaGetLastError(), "meshlet ranges");
         return STRIDE_OK;
     }
-    if (chain_use(h, static_cast<cudaStream_t>(stream)) != cudaSuccess)
-        return fail(STRIDE_ERR_CUDA, "meshlet ranges launch failed");
     const int r2 = enqueue_meshlet_ranges(h->d_descs, h->d_blk_prefix, n,
                                           reinterpret_cast<unsigned long long*>(d_v_first),
                                           reinterpret_cast<unsigned long long*>(d_t_first), stream);
-    mark_use(h, static_cast<cudaStream_t>(stream));
+    if (!cap) mark_use(h, static_cast<cudaStream_t>(stream));
     return r2 ? fail(r2, "meshlet ranges launch failed") : STRIDE_OK;
 }
 
@@ -956,12 +973,11 @@ int stride_meshlet_bounds(stride_handle* h, void* stream, const float* d_pos, fl
         return fail(STRIDE_ERR_ARG, "positions and bounds must be 4-byte aligned");
     if (!h->launched) return fail(STRIDE_ERR_ARG, "no decode yet");
     if (!h->d_mem) return no_buffers();
-    const int rc = stride_status(h, 1, nullptr);
+    bool cap = false;
+    const int rc = begin_use(h, static_cast<cudaStream_t>(stream), &cap, "meshlet bounds");
     if (rc) return rc;
-    if (chain_use(h, static_cast<cudaStream_t>(stream)) != cudaSuccess)
-        return fail(STRIDE_ERR_CUDA, "meshlet bounds launch failed");
     const int r2 = enqueue_meshlet_bounds(h->d_descs, h->d_blk_prefix, h->params.n_meshlets, d_pos, d_bounds, stream);
-    mark_use(h, static_cast<cudaStream_t>(stream));
+    if (!cap) mark_use(h, static_cast<cudaStream_t>(stream));
     return r2 ? fail(r2, "meshlet bounds launch failed") : STRIDE_OK;
 }
 

@@ -47,9 +47,31 @@ def test_status_of_a_replayed_decode(data):
     with pytest.raises(StrideFormatError):
         dec.meshlet_bounds(verts)
     dec.reload(data)
-    tris.zero_(), verts.zero_()
+    tris.view(torch.int32).zero_(), verts.zero_()
     graph.replay()
     torch.cuda.synchronize()
     dec.check()
     _same(data, tris, verts)
+    dec.close()
+
+
+def test_calls_after_captured_ones(data):
+    import torch
+    from meshpress_gb300 import ParaDeltaV5GpuDecoder
+    dec = ParaDeltaV5GpuDecoder(data)
+    tris, verts = dec.decode_to_device()
+    ranges, bounds, side = dec.meshlet_ranges(), dec.meshlet_bounds(verts), dec.side_table()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, capture_error_mode="relaxed"):
+        c_ranges, c_bounds, c_side = dec.meshlet_ranges(), dec.meshlet_bounds(verts), dec.side_table()
+    graph.replay()
+    for _ in range(2):
+        again = (*dec.meshlet_ranges(), dec.meshlet_bounds(verts), *dec.side_table())
+        for got in ((*c_ranges, c_bounds, *c_side), again):
+            for x, y in zip(got, (*ranges, bounds, *side)):
+                assert torch.equal(x, y)
+        dec.reload(data)
+        tris, verts = dec.decode_to_device()
+        _same(data, tris, verts)
     dec.close()

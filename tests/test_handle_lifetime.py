@@ -126,3 +126,21 @@ def test_status_of_a_replayed_decode(lib):
         for call in OUTPUTS.values():
             assert call(lib, h) == rc
     lib.stride_close(h)
+
+
+@pytest.mark.parametrize("call", OUTPUTS)
+def test_calls_after_a_captured_one(lib, call):
+    """A call captured after an eager one, and eager calls after it."""
+    h = _open(lib)
+    assert lib.stride_decode(h, S, AT, AT, None) == 0
+    assert lib.stride_finish(h, S, None) == 0
+    assert OUTPUTS[call](lib, h) == 0
+    lib.fake_capture(S)
+    assert OUTPUTS[call](lib, h) == 0
+    lib.fake_capture(None)
+    assert OUTPUTS[call](lib, h) == 0
+    assert lib.stride_reload(h, SMALL, len(SMALL), S) == 0
+    assert lib.stride_decode(h, S, AT, AT, None) == 0
+    assert lib.stride_finish(h, S, None) == 0
+    lib.stride_close(h)
+    assert lib.fake_returned()  # the capture's replays may still use it
