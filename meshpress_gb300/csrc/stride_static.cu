@@ -73,7 +73,8 @@ struct StaticLayout {
     size_t blob, params, lut_list, descs, sums, prefix, walk, lut, status, total;
 };
 
-StaticLayout plan(size_t len, const MeshParams& p) {
+// `alone`: with the tables that only a mesh decoded alone gets (lut_entries).
+StaticLayout plan(size_t len, const MeshParams& p, bool alone) {
     StaticLayout L;
     size_t o = 0;
     L.blob = o;
@@ -91,7 +92,7 @@ StaticLayout plan(size_t len, const MeshParams& p) {
     L.walk = o;
     o += up256(4ull * walk_scratch_words(p.n_v, p.n_meshlets));
     L.lut = o;
-    o += up256(4ull * lut_entries(p, true));
+    o += up256(4ull * lut_entries(p, alone));
     L.status = o;
     o += up256(sizeof(Status));
     L.total = o;
@@ -108,9 +109,10 @@ extern "C" int stride_decode_static(const uint8_t* data, size_t len, void* strea
     char why[256] = {0};
     int rc = parse_header(data, len, &p, why, sizeof(why));
     if (rc) return fail(rc, "%s", why);
+    const bool alone = plan(len, p, true).total <= kStaticScratchBytes;  // no stream is refused for these tables
     uint32_t n_lut = 0, lut_max = 0;
-    plan_luts(&p, 1, nullptr, 1, &n_lut, &lut_max, true);
-    const StaticLayout L = plan(len, p);
+    plan_luts(&p, 1, nullptr, 1, &n_lut, &lut_max, alone);
+    const StaticLayout L = plan(len, p, alone);
     if (L.total > kStaticScratchBytes)
         return fail(STRIDE_ERR_NOMEM,
                     "stream needs %zu bytes of decode scratch; the allocation-free entry point has a fixed "
