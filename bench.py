@@ -516,8 +516,7 @@ def run_single(args):
     peak, peak_src = measured_peak()
     k = np.array(kern_ms).mean(axis=0)
     names, dom, dom_bytes = kernel_split(k, int(dec.info.kernels) == 2, len(data), n_v, n_t,
-                                         int(launch["persistent"]) if launch
-                                         else (4 if dec.n_meshlets <= 9728 else 2))  # the default shapes
+                                         int(dec.launch_config().persistent))
     achieved = dom_bytes / (k[dom] / 1e3) / 1e9
     roofline = {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                 "frac": round(achieved / peak, 4), "traffic": ncu_traffic(names[dom], cfg["workload"]),

@@ -228,10 +228,12 @@ int stride_decode_timed(stride_handle* h, void* stream, uint32_t* d_idx, float* 
 
 /* Launch shape for this handle's decodes.  Until it is set the shape
  * follows the mesh's size: the team kernel (persistent 4) up to 9,728
- * meshlets (17,024 for codes above 16 bits), the two kernels (persistent 1) up to 1,023 groups of 32
- * meshlets, the fused kernel (persistent 2) above; a reload keeps a shape
- * that was set. */
+ * meshlets (17,024 for codes above 16 bits), the two kernels (persistent 1)
+ * up to 1,023 groups of 32 meshlets, the fused kernel (persistent 2) above; a
+ * reload keeps a shape that was set. */
 int stride_set_config(stride_handle* h, const stride_launch_cfg* cfg);
+/* The launch shape that this handle's decodes take. */
+int stride_get_config(const stride_handle* h, stride_launch_cfg* cfg);
 
 /* No counterpart in the reference.  SM clocks each device wait of this
  * handle's decodes may spin -- a bulk copy's mbarrier, the fused kernel's

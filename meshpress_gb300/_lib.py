@@ -109,6 +109,7 @@ SIGNATURES = [
     ("stride_meshlet_bounds", _I, [_P, _P, _P, _P]),
     ("stride_cull_meshlets", _I, [_P, ctypes.c_uint32, _P, _P, _P, _P]),
     ("stride_set_config", _I, [_P, ctypes.POINTER(LaunchCfg)]),
+    ("stride_get_config", _I, [_P, ctypes.POINTER(LaunchCfg)]),
     ("stride_set_wait_limit", _I, [_P, _U64]),
     ("stride_close", None, [_P]),
     ("stride_decode_static", _I, [_P, _SZ, _P, _P, _P]),

@@ -1065,6 +1065,16 @@ int stride_set_config(stride_handle* h, const stride_launch_cfg* c) {
     return STRIDE_OK;
 }
 
+int stride_get_config(const stride_handle* h, stride_launch_cfg* c) {
+    if (!h || !c) return fail(STRIDE_ERR_ARG, "null argument");
+    c->warps_per_cta = h->cfg.warps_per_cta;
+    c->persistent = h->cfg.persistent;
+    c->ctas_per_sm = h->cfg.ctas_per_sm;
+    c->stage_bytes = h->cfg.stage_bytes;
+    c->code_bytes = h->cfg.code_bytes;
+    return STRIDE_OK;
+}
+
 void stride_close(stride_handle* h) {
     if (!h) return;
     const bool idle = handle_idle(h);

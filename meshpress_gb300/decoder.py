@@ -109,6 +109,12 @@ class ParaDeltaV5GpuDecoder:
         _lib.check(self._lib.stride_set_config(self._h, ctypes.byref(cfg)), "stride_set_config")
         _lib.check(self._lib.stride_info(self._h, ctypes.byref(self.info)), "stride_info")  # kernels per decode
 
+    def launch_config(self) -> _lib.LaunchCfg:
+        """The shape that decodes take: what was set, or by the mesh's size."""
+        cfg = _lib.LaunchCfg()
+        _lib.check(self._lib.stride_get_config(self._h, ctypes.byref(cfg)), "stride_get_config")
+        return cfg
+
     # -- decoding --------------------------------------------------------------
     def _outputs(self):
         torch = _torch()
