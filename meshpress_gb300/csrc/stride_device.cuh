@@ -148,6 +148,22 @@ __device__ __forceinline__ uint32_t smem_addr(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// a * b + c on the multiplier, which leaves the integer ALU to the rest.
+__device__ __forceinline__ uint32_t mad_u32(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t d;
+    asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
+
+// 32 bits at bit `pos` of the words at shared address `base`.
+__device__ __forceinline__ uint32_t peek_shared(uint32_t base, uint32_t pos) {
+    const uint32_t a = mad_u32(pos >> 5, 4u, base);
+    uint32_t hi, lo;
+    asm("ld.shared.u32 %0, [%1];" : "=r"(hi) : "r"(a));
+    asm("ld.shared.u32 %0, [%1+4];" : "=r"(lo) : "r"(a));
+    return __funnelshift_l(lo, hi, pos & 31u);
+}
+
 __device__ __forceinline__ void mbar_init(uint64_t* bar) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(bar)) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -344,9 +360,10 @@ __device__ __forceinline__ uint32_t group_at(uint32_t f, uint32_t n_groups) {
     return kPer * w + l;
 }
 
-// The meshlet of a slot (of none when !in).
-__device__ __forceinline__ void load_slot_lane(const DecodeArgs& a, uint32_t slot, bool in, GroupLane& L) {
-    L.valid = in && slot < a.total_meshlets;
+// Lane's meshlet of a group of 32 slots.
+__device__ __forceinline__ void load_group_lane(const DecodeArgs& a, uint32_t g, int lane, GroupLane& L) {
+    const uint32_t slot = g * 32u + lane;
+    L.valid = slot < a.total_meshlets;
     L.m = L.valid ? __ldcg(&a.descs[slot].slot_meshlet) : slot;
     if (L.valid) {
         const uint4* src = reinterpret_cast<const uint4*>(a.descs + L.m);
@@ -367,11 +384,6 @@ __device__ __forceinline__ void load_slot_lane(const DecodeArgs& a, uint32_t slo
     L.mi = (L.valid && a.meshlet_mesh) ? __ldcg(a.meshlet_mesh + L.m) : 0u;
     L.P = a.meshes + L.mi;
     L.blob_off = L.valid ? L.P->blob_off : 0ull;
-}
-
-// Lane's meshlet of a group of 32 slots.
-__device__ __forceinline__ void load_group_lane(const DecodeArgs& a, uint32_t g, int lane, GroupLane& L) {
-    load_slot_lane(a, g * 32u + lane, true, L);
 }
 
 // The meshlet's output ranges lie inside its mesh's (header n_v_total, n_t)

@@ -40,7 +40,6 @@
 #include "stride_common.cuh"
 #include "stride_device.cuh"
 #include "stride_gb300.h"
-#include "stride_team.cuh"
 
 namespace stride {
 namespace {

@@ -41,22 +41,6 @@ __device__ __forceinline__ void team_all_bar() {  // every warp, from its own lo
     asm volatile("bar.sync 4, %0;" ::"n"(kThreads) : "memory");
 }
 
-// a * b + c on the multiplier, which leaves the integer ALU to the rest.
-__device__ __forceinline__ uint32_t mad_u32(uint32_t a, uint32_t b, uint32_t c) {
-    uint32_t d;
-    asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-    return d;
-}
-
-// 32 bits at bit `pos` of the words at shared address `base`.
-__device__ __forceinline__ uint32_t peek_shared(uint32_t base, uint32_t pos) {
-    const uint32_t a = mad_u32(pos >> 5, 4u, base);
-    uint32_t hi, lo;
-    asm("ld.shared.u32 %0, [%1];" : "=r"(hi) : "r"(a));
-    asm("ld.shared.u32 %0, [%1+4];" : "=r"(lo) : "r"(a));
-    return __funnelshift_l(lo, hi, pos & 31u);
-}
-
 // A parser step: what it read (32 bits from its first token's edge code or
 // flag) and, for the FIFO warp and the assembler, bits 0..1 the raw tokens,
 // bit 2 a FIFO token after them, bit 3 strip-body tokens (each with its edge
