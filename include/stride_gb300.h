@@ -399,6 +399,9 @@ int pldt5_open(const uint8_t* data, size_t len, pldt5_handle** out);
  * outputs, header fields); like stride_inspect. */
 int pldt5_inspect(const uint8_t* data, size_t len, pldt5_info_t* info);
 int pldt5_info(const pldt5_handle* h, pldt5_info_t* info);
+/* Meshlets that a CTA of this handle's decodes takes: 8 or 16 (the team
+ * kernel), or 0 (the general kernel, one lane per meshlet). */
+int pldt5_meshlets_per_cta(const pldt5_handle* h);
 /* Enqueue the decode on `stream`: triangles (n_t x 3 uint32, global rows)
  * and world-space positions (n_v x 3 float32) into device buffers.
  * Replaces ParaDeltaV5GpuDecoder.decode (:686-712) plus the world transform

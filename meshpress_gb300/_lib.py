@@ -140,6 +140,7 @@ SIGNATURES = [
     ("pldt5_open", _I, [_P, _SZ, ctypes.POINTER(_P)]),
     ("pldt5_inspect", _I, [_P, _SZ, ctypes.POINTER(Pldt5Info)]),
     ("pldt5_info", _I, [_P, ctypes.POINTER(Pldt5Info)]),
+    ("pldt5_meshlets_per_cta", _I, [_P]),
     ("pldt5_decode", _I, [_P, _P, _P, _P]),
     ("pldt5_status", _I, [_P, _I]),
     ("pldt5_close", None, [_P]),

@@ -1527,6 +1527,8 @@ int pldt5_info(const pldt5_handle* h, pldt5_info_t* info) {
     return STRIDE_OK;
 }
 
+int pldt5_meshlets_per_cta(const pldt5_handle* h) { return h ? static_cast<int>(h->team) : 0; }
+
 int pldt5_decode(pldt5_handle* h, void* stream, uint32_t* d_idx, float* d_pos) {
     if (!h || (!d_idx && h->info.n_t) || (!d_pos && h->info.n_v)) return fail(STRIDE_ERR_ARG, "null argument");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
