@@ -602,10 +602,10 @@ __device__ __forceinline__ bool p5_four(uint32_t base, uint32_t& pos, uint32_t t
     const uint32_t zmul = tag == 1u ? pow : 0u, most = tag ? 32u : 30u;
     const uint32_t a = mad_u32(pos >> 5, 4u, base), o = pos & 31u;
     uint32_t w0, w1, w2, w3;
-    asm("ld.shared.u32 %0, [%1];" : "=r"(w0) : "r"(a));
-    asm("ld.shared.u32 %0, [%1+4];" : "=r"(w1) : "r"(a));
-    asm("ld.shared.u32 %0, [%1+8];" : "=r"(w2) : "r"(a));
-    asm("ld.shared.u32 %0, [%1+12];" : "=r"(w3) : "r"(a));
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w0) : "r"(a));
+    asm volatile("ld.shared.u32 %0, [%1+4];" : "=r"(w1) : "r"(a));
+    asm volatile("ld.shared.u32 %0, [%1+8];" : "=r"(w2) : "r"(a));
+    asm volatile("ld.shared.u32 %0, [%1+12];" : "=r"(w3) : "r"(a));
     uint32_t hi = __funnelshift_l(w1, w0, o), mid = __funnelshift_l(w2, w1, o), lo = __funnelshift_l(w3, w2, o);
     uint32_t used = 0u, longest = 0u, before = 0u;
 #pragma unroll

@@ -155,12 +155,14 @@ __device__ __forceinline__ uint32_t mad_u32(uint32_t a, uint32_t b, uint32_t c) 
     return d;
 }
 
-// 32 bits at bit `pos` of the words at shared address `base`.
+// 32 bits at bit `pos` of the words at shared address `base`.  (Volatile, as the
+// other loads of this kind: the compiler may move plain assembly across the barrier
+// behind which the words are there.)
 __device__ __forceinline__ uint32_t peek_shared(uint32_t base, uint32_t pos) {
     const uint32_t a = mad_u32(pos >> 5, 4u, base);
     uint32_t hi, lo;
-    asm("ld.shared.u32 %0, [%1];" : "=r"(hi) : "r"(a));
-    asm("ld.shared.u32 %0, [%1+4];" : "=r"(lo) : "r"(a));
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(hi) : "r"(a));
+    asm volatile("ld.shared.u32 %0, [%1+4];" : "=r"(lo) : "r"(a));
     return __funnelshift_l(lo, hi, pos & 31u);
 }
 
