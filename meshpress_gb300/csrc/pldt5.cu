@@ -479,13 +479,13 @@ __global__ void __launch_bounds__(kP5Threads) p5_decode_kernel(P5Args a) {
 // What bounds it are the chains: 2.5K cycles to stage, 4.5K for the references,
 // 31K for 280 tokens, 21K for the first two substreams of 120 residuals, 39K
 // for 120 float64 predictions (a 33 x 33 terrain).  The general kernel, whose
-// one lane has all of it, tokens one by one, takes ten times as long: 361 x 361
-// terrain, 1,295 meshlets, 715 us against 90.
+// one lane has all of it, tokens one by one, takes eight times as long: 361 x 361
+// terrain, 1,295 meshlets, 714 us against 90.
 //
 // The host knows every meshlet's size: a CTA's shared memory is what the
 // stream's largest group of M needs, and each meshlet gets the room of its own
 // (the room of the largest kept CTAs of sixteen from sharing an SM: 9,921
-// meshlets 251 us, now 214).
+// meshlets 251 us, now 217).
 struct P5Room {
     uint32_t bits = 0u;  // staged bytes (odd in units of 16)
     uint32_t loc = 0u;   // words of the walk, of the row table, and doubles of an axis (odd)
@@ -1193,7 +1193,7 @@ __global__ void p5_world_kernel(P5Args a, unsigned long long n) {
     if (i < 3ull * n) a.pos[i] = p5_world(a, a.rows[i], static_cast<uint32_t>(i % 3ull));
 }
 
-constexpr uint32_t kP5Eight = 8u * 2u * 152u * 9u / 8u;  // about as many as CTAs of eight take at once
+constexpr uint32_t kP5Eight = 8u * 2u * 152u * 9u / 8u;  // about as many as CTAs of eight take at once on a GB300
 constexpr uint32_t kP5Most = 44u << 10;        // meshlets of a stream
 constexpr uint32_t kP5Two = 102u << 10;        // two CTAs to an SM
 // eight meshlets of the largest size that is accepted (197 KB) and the static part, in an SM's 227 KB
@@ -1440,9 +1440,8 @@ static int p5_host_parse_sized(const uint8_t* data, size_t len, P5Host& H) {
 // kTeamTokens tokens and kP5MaxStage bytes (encoded meshlets of 256 vertices
 // have half as many and a tenth), in streams of up to kP5Most meshlets; the
 // general kernel the others.  Its time hardly grows with the meshlets, the
-// team's does: up to 256 vertices, 21,307 / 43,086 meshlets 785 / 912 us and 377
-// / 713; up to 64 vertices, 23,843 / 50,955 meshlets about 370 / 380 and 212 /
-// 440.
+// team's does: up to 256 vertices, 21,307 / 43,086 meshlets 778 / 895 us and 383
+// / 721; up to 64 vertices, 23,843 / 50,955 meshlets 302 / 376 and 228 / 445.
 static cudaError_t p5_plan(const P5Host& H, uint32_t& team, uint32_t& smem) {
     team = smem = 0;
     if (H.info.n_meshlets == 0 || H.info.n_meshlets > kP5Most || H.most_tokens > kTeamTokens ||
@@ -1452,9 +1451,9 @@ static cudaError_t p5_plan(const P5Host& H, uint32_t& team, uint32_t& smem) {
     // to an SM (or all but a few); above, sixteen where two such CTAs fit an SM:
     // a decode then takes the CTAs' waves, and a CTA's chains hardly depend on
     // its number of meshlets (sixteen against eight: meshlets of up to 64
-    // vertices, 3,072 of them, 65 us against 87, 23,843 212 against 298; of up to
-    // 199 vertices, 10 79 against 75, 2,451 100 against 90, 4,913 141 against 151,
-    // 9,921 214 against 253).
+    // vertices, 3,072 of them, 65 us against 79, 23,843 228 against 289; of up to
+    // 199 vertices, 10 78 against 76, 2,451 102 against 90, 4,913 141 against 149,
+    // 9,921 217 against 252).
     team = H.info.n_meshlets > kP5Eight && H.smem16 <= kP5Two ? 16u : 8u;
     smem = team == 8u ? H.smem8 : H.smem16;
     return team == 8u ? p5_team_prepare<8>() : p5_team_prepare<16>();

@@ -36,9 +36,11 @@ constexpr uint64_t kHostPartTris = 3ull << 20;
 
 // Meshlets up to which such a decode keeps the team kernel, which ends before
 // the two kernels' triangles are out; above, their copy beside the vertex
-// kernel gains more (a call with pinned buffers, 14-bit heightfields of 45 /
-// 1,295 / 2,631 / 4,090 / 5,221 meshlets: two kernels 161 / 203 / 187 / 208 /
-// 234 us, team 85 / 121 / 165 / 204 / 268).
+// kernel gains more.  A call with pinned buffers, 14-bit heightfields of 45 / 1,295 /
+// 2,631 / 4,090 / 4,635 / 5,174 / 5,732 / 7,384 / 9,580 meshlets: two kernels 149 /
+// 167 / 153 / 174 / 186 / 196 / 209 / 240 / 286 us, team 63 / 89 / 128 / 159 / 170 /
+// 215 / 229 / 265 / 319.  The sides change with the second wave of team CTAs, at
+// 4,864; the line lies below it.
 constexpr uint32_t kHostTeam = 4096;
 
 // The end of a part's windows: the last window's block prefix and sums

@@ -1329,29 +1329,30 @@ int check_config(const LaunchCfg& cfg, bool wide) {
 }
 
 // Meshlets up to which the default launch shape is the team kernel, and with
-// 4, 8 and 16 meshlets per CTA: as many CTAs as the 152 SMs hold at once (two
-// per SM; four small meshlets while there is one CTA per SM), and 16 for up to two
-// such waves.  Step in us, L2 flushed, 12-bit heightfields, every output
-// bit-identical; before: the fused kernel up to 128 groups, then the two
-// kernels:
-//   meshlets            10   158   650  1295  2631  4090  5221  7503  9101  10584
-//   before              97   110   112   112   110   114   116   118   120    124
-//   4 per CTA           32    34    36    57    87   118   142   189   228    259
-//   8 per CTA           34    36    36    42    65    73    97   122   136    163
-//   16 per CTA          44    46    46    46    54    58    93    99   106    138
-// (14-bit spheres of 103 and 1,738 meshlets: 220 -> 48, 196 -> 52 us; 20-bit
-// heightfield of 5,221: 245 -> 96 us.)
+// 4, 8 and 16 meshlets per CTA: as many CTAs as the 152 SMs of a GB300 hold at
+// once (two per SM; four small meshlets while there is one CTA per SM), and 16 for
+// up to two such waves.  Step in us (to 2 us), L2 flushed, 12-bit heightfields,
+// every output bit-identical:
+//   meshlets            10   158   650  1295  2631  4090  5221  7503  9229  10584
+//   two kernels         94   109   109   109   109   109   111   111   113    117
+//   fused kernel        94   105   107   104   107   109   111   129   131    137
+//   4 per CTA           31    33    35    55    86   115   139   186   227    257
+//   8 per CTA           33    33    33    39    64    72    94   119   137    160
+//   16 per CTA          41    43    43    43    51    53    88    94   100    131
+// (14-bit spheres of 103 and 1,738 meshlets: two kernels 215 and 145, team 47 and
+// 51 us; 20-bit heightfield of 5,221: 242 and 93 us.)
 // Codes above 16 bits (no tables; codewords longer than the windows of the
 // group kernels' lanes) and batches of many meshes (unequal meshlets side by
 // side in a group) keep it for three and a half waves:
-//   20-bit heightfields, 15,068 / 21,307 meshlets: team 180 / 238, two kernels 257 / 285
-//   18 bits: 178 / 236 and 209 / 229
+//   20-bit heightfields, 15,068 / 21,307 meshlets: team 178 / 234, two kernels 256 / 330
+//   18 bits: 174 / 233 and 205 / 305
 //   batches of 56 / 64 / 80 / 100 mixed meshes, 11,854 / 13,238 / 16,853 / 20,903
-//   meshlets: 154 / 168 / 205 / 244 and 199 / 209 / 213 / 238
-//   (one mesh of 15,068 meshlets, 12 bits: 170 and 139)
+//   meshlets: 152 / 164 / 203 / 238 and 201 / 207 / 211 / 234
+//   (one mesh of 15,068 meshlets, 12 bits: 166 and 133)
+// (A wide mesh above the bound would still gain; the bound is the batches'.)
 // Four to a CTA stay ahead of eight for a whole wave of them when the meshlets
-// are large (923 / 1,190 of 195 triangles 35 / 35 us, by eight 39 / 39; 962 of 84
-// triangles 28.6 and 26.6).
+// are large (923 / 1,190 of 200 triangles 35 / 37 us, by eight 39 / 39; 934 of 85
+// triangles 22.5 by either).
 constexpr uint32_t kTeam4 = 700u, kTeam4Full = 1216u, kTeam8 = 2432u, kTeamMost = 9728u, kTeamMore = 17024u;
 constexpr uint32_t kFullMeshlet = 128u;  // triangles, on average
 constexpr uint32_t kSmallMesh = 512u;  // meshlets per mesh, on average
