@@ -1334,21 +1334,21 @@ int check_config(const LaunchCfg& cfg, bool wide) {
 // up to two such waves.  Step in us (to 2 us), L2 flushed, 12-bit heightfields,
 // every output bit-identical:
 //   meshlets            10   158   650  1295  2631  4090  5221  7503  9229  10584
-//   two kernels         94   109   109   109   109   109   111   111   113    117
-//   fused kernel        94   105   107   104   107   109   111   129   131    137
+//   two kernels         96   109   109   109   109   109   111   111   113    117
+//   fused kernel        96   107   109   104   107   109   109   129   135    141
 //   4 per CTA           31    33    35    55    86   115   139   186   227    257
 //   8 per CTA           33    33    33    39    64    72    94   119   137    160
-//   16 per CTA          41    43    43    43    51    53    88    94   100    131
-// (14-bit spheres of 103 and 1,738 meshlets: two kernels 215 and 145, team 47 and
+//   16 per CTA          41    43    43    43    51    54    88    94   100    130
+// (14-bit spheres of 103 and 1,738 meshlets: two kernels 217 and 145, team 47 and
 // 51 us; 20-bit heightfield of 5,221: 242 and 93 us.)
 // Codes above 16 bits (no tables; codewords longer than the windows of the
 // group kernels' lanes) and batches of many meshes (unequal meshlets side by
 // side in a group) keep it for three and a half waves:
-//   20-bit heightfields, 15,068 / 21,307 meshlets: team 178 / 234, two kernels 256 / 330
-//   18 bits: 174 / 233 and 205 / 305
+//   20-bit heightfields, 15,068 / 21,307 meshlets: team 178 / 234, two kernels 258 / 283
+//   18 bits: 174 / 231 and 203 / 235
 //   batches of 56 / 64 / 80 / 100 mixed meshes, 11,854 / 13,238 / 16,853 / 20,903
-//   meshlets: 152 / 164 / 203 / 238 and 201 / 207 / 211 / 234
-//   (one mesh of 15,068 meshlets, 12 bits: 166 and 133)
+//   meshlets: 152 / 166 / 203 / 240 and 199 / 207 / 211 / 240
+//   (one mesh of 15,068 meshlets, 12 bits: 168 and 139)
 // (A wide mesh above the bound would still gain; the bound is the batches'.)
 // Four to a CTA stay ahead of eight for a whole wave of them when the meshlets
 // are large (923 / 1,190 of 200 triangles 35 / 37 us, by eight 39 / 39; 934 of 85
@@ -1369,9 +1369,9 @@ LaunchCfg default_config(uint32_t total_meshlets, uint64_t total_tris, uint32_t 
     const uint32_t groups = (total_meshlets + 31u) / 32u;
     // Above: the two kernels below kFlowFiveGroups, where the fused kernel's
     // completion list runs short of finished groups and its vertex phase
-    // waits (1449^2, 666 groups: 0.177 against 0.173 ms), then the fused
+    // waits (1449^2, 666 groups: 0.171 against 0.168 ms), then the fused
     // kernel, whose overlap of the two phases wins (2049^2, 1,347 groups:
-    // 0.222 against 0.278).
+    // 0.215 against 0.274).
     cfg.persistent = groups < kFlowFiveGroups ? 1 : 2;
     return cfg;
 }
