@@ -412,14 +412,19 @@ int decode_to_host(HostLink& L, const DecodeArgs& a, LaunchCfg cfg, void* stream
     // or write the host outputs when this returns
     auto drain = [&]() {
         cudaStreamSynchronize(s);
-        cudaStreamSynchronize(L.copy[0]);
-        cudaStreamSynchronize(L.copy[1]);
+        for (cudaStream_t c : L.copy)
+            if (c) cudaStreamSynchronize(c);
         // parts may have ended half-way: the next scan finds its counter at zero
         if (cudaMemsetAsync(a.status, 0, sizeof(Status), s) == cudaSuccess) cudaStreamSynchronize(s);
     };
     auto bail = [&](cudaError_t err, const char* what) {
         drain();
         return cuda_fail(err, what);
+    };
+    auto not_launched = [&](int rc) {  // the scan may be queued
+        const char* why = cudaGetErrorString(cudaGetLastError());
+        drain();
+        return fail(rc, "decode launch failed: %s", why);
     };
     if (cfg.persistent == 2) cfg.persistent = 1;
     if (cfg.persistent == 4 && a.total_meshlets > kHostTeam) {
@@ -437,7 +442,7 @@ int decode_to_host(HostLink& L, const DecodeArgs& a, LaunchCfg cfg, void* stream
         if (bytes_in && (e = cudaStreamWaitEvent(s, bytes_in[kHostParts - 1], 0)) != cudaSuccess)
             return cuda_fail(e, "decode to host: upload");
         const int rc = enqueue_decode(a, cfg, stream);
-        if (rc) return fail(rc, "decode launch failed: %s", cudaGetErrorString(cudaGetLastError()));
+        if (rc) return not_launched(rc);
         e = cudaMemcpyAsync(L.h_status, a.status, sizeof(Status), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess && ib) e = cudaMemcpyAsync(h_idx, a.idx, ib, cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess && pb) e = cudaMemcpyAsync(h_pos, a.pos, pb, cudaMemcpyDeviceToHost, s);
@@ -484,16 +489,13 @@ int decode_to_host(HostLink& L, const DecodeArgs& a, LaunchCfg cfg, void* stream
         }
         if (rc == STRIDE_OK && e == cudaSuccess) rc = enqueue_parts_end(a, cfg, stream, L.vert_done);
         if (e != cudaSuccess) return bail(e, "decode to host: parts");
-        if (rc) {
-            drain();
-            return fail(rc, "decode launch failed: %s", cudaGetErrorString(cudaGetLastError()));
-        }
+        if (rc) return not_launched(rc);
     } else {
         if (bytes_in && (e = cudaStreamWaitEvent(s, bytes_in[kHostParts - 1], 0)) != cudaSuccess)
             return cuda_fail(e, "decode to host: upload");
         void* ev[4] = {nullptr, nullptr, L.conn_done, L.vert_done};
         const int rc = enqueue_decode(a, cfg, stream, ev);
-        if (rc) return fail(rc, "decode launch failed: %s", cudaGetErrorString(cudaGetLastError()));
+        if (rc) return not_launched(rc);
     }
     // each output (the triangles unless they went by parts) in two halves,
     // one per copy stream

@@ -20,6 +20,7 @@ int g_decode_rc = 0;
 unsigned long long g_decode_err = 0;
 uint32_t g_scans = 0, g_outputs = 0;  // launches that read or wrote a handle's records
 bool g_freed_used = false;            // ... of memory that had been given back
+std::set<void*> g_pending;            // streams with work that no one has waited for
 Status* g_status = nullptr;
 uint8_t* g_arena = nullptr;
 
@@ -78,7 +79,7 @@ cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) {
     return *s = reinterpret_cast<cudaStream_t>(new int), cudaSuccess;
 }
 cudaError_t cudaStreamDestroy(cudaStream_t s) { return delete reinterpret_cast<int*>(s), cudaSuccess; }
-cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t s) { return g_pending.erase(s), cudaSuccess; }
 cudaError_t cudaStreamIsCapturing(cudaStream_t s, cudaStreamCaptureStatus* c) {
     *c = s != nullptr && s == g_capturing ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
     return cudaSuccess;
@@ -97,12 +98,14 @@ void fake_reset() {
     g_decode_err = 0;
     g_scans = g_outputs = 0;
     g_freed_used = false;
+    g_pending.clear();
 }
 void fake_most(size_t n) { g_most = n; }
 void fake_capture(void* s) { g_capturing = s; }
 void fake_decode(int rc, unsigned long long err) { g_decode_rc = rc, g_decode_err = err; }
 void fake_replay(unsigned long long err) { g_status->err = err; }  // of the last decode that was enqueued
 uint32_t fake_outputs() { return g_outputs; }
+int fake_pending(void* s) { return static_cast<int>(g_pending.count(s)); }
 int fake_freed_used() { return g_freed_used ? 1 : 0; }
 // whether the last decode's status word and bytes have gone back to the driver
 int fake_returned() { return freed(g_status) && freed(g_arena) ? 1 : 0; }
@@ -119,8 +122,9 @@ LaunchCfg default_config(uint32_t, uint64_t, uint32_t, bool) {
     return c;
 }
 void last_launch(uint32_t* smem, uint32_t* grid) { *smem = *grid = 0; }
-int enqueue_decode(const DecodeArgs& a, const LaunchCfg&, void*, void* const*) {
+int enqueue_decode(const DecodeArgs& a, const LaunchCfg&, void* s, void* const*) {
     g_scans++;  // queued, whatever becomes of the kernel behind it
+    g_pending.insert(s);
     g_status = a.status;
     g_arena = const_cast<uint8_t*>(a.arena);
     a.status->err = g_decode_err;

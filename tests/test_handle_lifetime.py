@@ -32,7 +32,7 @@ def built(tmp_path_factory):
         if hasattr(lib, name):
             getattr(lib, name).restype, getattr(lib, name).argtypes = res, args
     lib.fake_most.argtypes = [_SZ]
-    lib.fake_capture.argtypes = [_P]
+    lib.fake_capture.argtypes = lib.fake_pending.argtypes = [_P]
     lib.fake_decode.argtypes = [ctypes.c_int, _ULL]
     lib.fake_replay.argtypes = [_ULL]
     return lib
@@ -81,6 +81,21 @@ def test_memory_of_a_failed_decode_is_not_handed_on(lib, call):
     lib.fake_decode(0, 0)
     lib.stride_close(h)
     assert lib.fake_returned()
+
+
+@pytest.mark.parametrize("shape", [4, 1])
+def test_failed_host_decode_leaves_nothing_running(lib, shape):
+    """In the one-kernel and the two-kernel shape."""
+    h = _open(lib)
+    cfg = _lib.LaunchCfg()
+    cfg.warps_per_cta, cfg.persistent, cfg.stage_bytes, cfg.code_bytes = 4, shape, 16384, 16384
+    assert lib.stride_set_config(h, ctypes.byref(cfg)) == 0
+    lib.fake_decode(_lib.STRIDE_ERR_CUDA, 0)
+    assert lib.stride_decode(h, S, AT, AT, None) == _lib.STRIDE_ERR_CUDA
+    assert lib.fake_pending(S)  # a device decode does not wait
+    assert lib.stride_decode_host(h, S, AT, AT) == _lib.STRIDE_ERR_CUDA
+    assert not lib.fake_pending(S)
+    lib.stride_close(h)
 
 
 OUTPUTS = {
